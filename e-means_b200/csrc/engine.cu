@@ -69,6 +69,62 @@ struct DevBuf {
     }
 };
 
+// Scratch of one call, stream-ordered, from a pool that the handles of a device
+// share: allocating and freeing costs microseconds and a new handle's first call
+// finds the memory of the last one, where cudaMalloc takes 0.3 ms (and tens of ms
+// beside other processes' allocations). The pool keeps at most kScratchKeep bytes
+// beyond what calls hold, and none once the device's last handle is destroyed.
+constexpr uint64_t kScratchKeep = (uint64_t)64 << 20;
+struct ScratchPools {
+    std::mutex mu;
+    std::map<int, cudaMemPool_t> pool;
+    std::map<int, int> users;
+};
+ScratchPools& scratch_pools() {
+    static ScratchPools* p = new ScratchPools();  // handles may outlive static destructors
+    return *p;
+}
+void scratch_users(int device, int change) {
+    ScratchPools& s = scratch_pools();
+    std::lock_guard<std::mutex> lock(s.mu);
+    auto it = s.pool.find(device);
+    if ((s.users[device] += change) == 0 && it != s.pool.end()) cudaMemPoolTrimTo(it->second, 0);
+}
+
+struct Scratch {
+    int device;
+    cudaStream_t st;
+    uint8_t* p = nullptr;
+    Scratch(int device_, cudaStream_t st_) : device(device_), st(st_) {}
+    Scratch(const Scratch&) = delete;
+    Scratch& operator=(const Scratch&) = delete;
+    ~Scratch() {
+        if (p) cudaFreeAsync(p, st);
+    }
+    cudaError_t alloc(size_t bytes) {
+        cudaMemPool_t pool = nullptr;
+        {
+            ScratchPools& s = scratch_pools();
+            std::lock_guard<std::mutex> lock(s.mu);
+            auto it = s.pool.find(device);
+            if (it == s.pool.end()) {
+                cudaMemPoolProps props{};
+                props.allocType = cudaMemAllocationTypePinned;
+                props.location.type = cudaMemLocationTypeDevice;
+                props.location.id = device;
+                cudaError_t e = cudaMemPoolCreate(&pool, &props);
+                if (e != cudaSuccess) return e;
+                uint64_t keep = kScratchKeep;
+                cudaMemPoolSetAttribute(pool, cudaMemPoolAttrReleaseThreshold, &keep);
+                s.pool[device] = pool;
+            } else {
+                pool = it->second;
+            }
+        }
+        return cudaMallocFromPoolAsync((void**)&p, std::max(bytes, (size_t)16), pool, st);
+    }
+};
+
 // Device state of a training run (filled by emb200_train).
 struct TrainState {
     DevBuf<float> usage, sums, pass_sums, batch_dist, alphas, xbatch;
@@ -947,6 +1003,19 @@ int check_ready(emb200_handle* h, int dtype) {
     return EMB200_OK;
 }
 
+// The handle's second stream and the events between it and the first.
+int ensure_copy_stream(emb200_handle* h) {
+    if (!h->copy_stream) CK(cudaStreamCreateWithFlags(&h->copy_stream, cudaStreamNonBlocking));
+    if (!h->ev_copied[0]) {
+        for (int b = 0; b < 2; b++) {
+            CK(cudaEventCreateWithFlags(&h->ev_copied[b], cudaEventDisableTiming));
+            CK(cudaEventCreateWithFlags(&h->ev_done[b], cudaEventDisableTiming));
+            CK(cudaEventRecord(h->ev_done[b], h->stream));
+        }
+    }
+    return EMB200_OK;
+}
+
 // Host-memory assign (the trait call). Rows go through two staging buffers in
 // chunks: the copy of chunk i+1 (its own stream) overlaps the search of chunk i,
 // and each chunk's labels and distances are copied back as soon as they are final.
@@ -958,14 +1027,8 @@ int assign_host(emb200_handle* h, int dtype, const void* x, size_t m, uint32_t* 
     if (m > 0xFFFFFFFFull) return fail(h, EMB200_EINVAL, "more than 2^32 - 1 rows in one call");
     h->stats = emb200_stats{};
     cudaStream_t st = h->stream;
-    if (!h->copy_stream) CK(cudaStreamCreateWithFlags(&h->copy_stream, cudaStreamNonBlocking));
-    if (!h->ev_copied[0]) {
-        for (int b = 0; b < 2; b++) {
-            CK(cudaEventCreateWithFlags(&h->ev_copied[b], cudaEventDisableTiming));
-            CK(cudaEventCreateWithFlags(&h->ev_done[b], cudaEventDisableTiming));
-            CK(cudaEventRecord(h->ev_done[b], st));
-        }
-    }
+    rc = ensure_copy_stream(h);
+    if (rc) return rc;
     CK(cudaEventRecord(h->ev0, st));
     const size_t esz = elt_size(dtype);
     const size_t row_bytes = h->d * esz;
@@ -1041,6 +1104,7 @@ int emb200_create(int ordinal, const emb200_opts* opts, emb200_handle** out) {
         delete h;
         return EMB200_ECUDA;
     }
+    scratch_users(ordinal, 1);
     *out = h;
     return EMB200_OK;
 }
@@ -1074,6 +1138,7 @@ int emb200_destroy(emb200_handle* h) {
         if (h->ev_done[b]) cudaEventDestroy(h->ev_done[b]);
     }
     if (h->stream) cudaStreamDestroy(h->stream);
+    scratch_users(h->device, -1);
     delete h;
     return EMB200_OK;
 }

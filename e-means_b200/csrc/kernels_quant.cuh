@@ -5,9 +5,9 @@
 // Exactness notes, per step of Int8Quantizer::fit (src/quantize.rs:45-62):
 //  * mean: the reference adds the rows in order into one f64 accumulator per
 //    dimension (`:48-51`). f64 addition is not associative, so a tree reduction
-//    could differ in the last bit; k_quant_colsum keeps the row order, one
-//    accumulator per dimension, and streams rows into shared memory by cp.async
-//    several stages ahead so that the chain of dependent adds sets its pace.
+//    could differ in the last bit; k_quant_colpart / k_quant_colscan add whole
+//    blocks of rows where that provably rounds nowhere and replay the rest in
+//    row order.
 //  * peak: `select_nth_unstable_by(idx, f32::total_cmp)` over |x - shift|
 //    (`:53-56`). Every magnitude has a clear sign bit, so total_cmp is the
 //    unsigned order of the bit patterns (NaNs above +inf); the select is a
@@ -23,9 +23,6 @@
 
 namespace emb {
 
-constexpr int kQsumRows = 256;     // rows per shared-memory stage of the column sums
-constexpr int kQsumStages = 4;     // stages in flight (cp.async groups)
-constexpr int kQsumThreads = 256;  // all threads copy; warp 0 sums
 constexpr int kQThreads = 512;     // element-wise passes
 constexpr int kQBins0 = 2048;      // bits 30..20 of a magnitude (bit 31 is always clear)
 constexpr int kQBins = 1024;       // bits 19..10, then bits 9..0
@@ -50,62 +47,330 @@ template <int N>
 __device__ __forceinline__ void qs_cp_wait() { asm volatile("cp.async.wait_group %0;\n" ::"n"(N) : "memory"); }
 
 // Per-dimension f64 sums in row order, then shift = (f32)(sum / n)
-// (src/quantize.rs:48-52). One CTA per 32 consecutive dimensions; lane t of
-// warp 0 owns dimension c0 + t and adds its values in row order. Rows arrive
-// in 256-row stages by cp.async, kQsumStages - 1 stages ahead of the sums (16-
-// byte copies when d % 4 == 0, else 4-byte copies). Dynamic shared memory:
-// kQsumStages x kQsumRows x 32 floats.
-__global__ void __launch_bounds__(kQsumThreads) k_quant_colsum(const float* __restrict__ x, size_t n, size_t d,
-                                                               float* __restrict__ shift) {
-    extern __shared__ __align__(16) float qs_stage[];
-    const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
-    const size_t c0 = (size_t)blockIdx.x * 32;
-    const size_t nchunks = (n + kQsumRows - 1) / kQsumRows;
-    const bool vec = (d & 3) == 0;
-    auto issue = [&](size_t chunk) {
-        if (chunk < nchunks) {
-            const size_t r0 = chunk * kQsumRows;
-            float* dst = qs_stage + (chunk % kQsumStages) * (kQsumRows * 32);
-            if (vec) {  // 8 x 16 bytes per row slice
-                for (int e = tid; e < kQsumRows * 8; e += kQsumThreads) {
-                    const int r = e >> 3, q = e & 7;
-                    const size_t row = r0 + r, col = c0 + 4 * q;
-                    if (row < n && col < d) qs_cp_async16(dst + r * 32 + 4 * q, x + row * d + col);
-                }
-            } else {
-                for (int e = tid; e < kQsumRows * 32; e += kQsumThreads) {
-                    const int r = e >> 5, t = e & 31;
-                    const size_t row = r0 + r, col = c0 + t;
-                    if (row < n && col < d) qs_cp_async4(dst + r * 32 + t, x + row * d + col);
-                }
-            }
+// (src/quantize.rs:48-52), without walking the n dependent adds one by one.
+//
+// A chain acc <- RN(acc + x_i) rounds only where a partial sum needs more than 53
+// bits: with every x_i and acc multiples of 2^q, all partial sums of magnitude at
+// most 2^(53 + q) are exact, and then any order of adding gives the chain's bits.
+//   k_quant_colpart  per block of kQsubRows rows and dimension: the sum, the
+//                    range of its prefix sums and its smallest non-zero magnitude
+//                    (which bounds q). One pass over the rows: HBM bounds it.
+//   k_quant_colscan  one warp per dimension walks the blocks 32 at a time: a lane's
+//                    block is accepted as a whole when the range above shows that
+//                    no partial sum inside it rounds; the first block that is not
+//                    is replayed from its rows (quant_replay64), which finds the
+//                    adds that do round by their exact error and redoes the rest
+//                    from there.
+// On 500,000 x 512 unit-norm rows: 0.175 ms (5.9 TB/s of rows, 0.90 of the copy
+// bandwidth) and 0.068 ms, against 4.25 ms for the chain itself (16.7 cycles an
+// add). Blocks of 256 rows: with 64 the scan of four times the entries took
+// 0.20 ms, and the rows it replays are few (none for most dimensions here).
+constexpr int kQsubRows = 256;
+constexpr int kQpartRows = 64;  // rows per thread of k_quant_colpart
+constexpr int kQscanDepth = 7;  // batches of 32 blocks in flight per warp (cp.async)
+constexpr int kQscanWarps = 8;  // neighbouring dimensions per CTA: they share the entries' sectors
+constexpr size_t kQsubBytes = (size_t)24 << 20;  // entries held at once; longer samples go in slabs of rows
+
+struct __align__(16) QuantSub {
+    double sum;
+    float lo, hi;  // range of the prefix sums, rounded outwards
+};
+
+// Smallest non-zero magnitude in a form that one unsigned minimum keeps: the bits
+// without the sign, doubled, less one (zero wraps to the largest value).
+__device__ __forceinline__ uint32_t quant_tiny(float v) { return (__float_as_uint(v) << 1) - 1u; }
+// The exponent of the lowest bit a value of at least that magnitude can have.
+__device__ __forceinline__ int quant_tiny_lsb(uint32_t tiny) {
+    if (tiny == 0xffffffffu) return 900;  // nothing but zeros
+    return max((int)(((tiny + 1u) >> 1) >> 23), 1) - 150;
+}
+__device__ __forceinline__ double quant_pow2(int e) { return __hiloint2double((min(e, 1000) + 1023) << 20, 0); }
+// The exponent of the lowest set bit of a finite double.
+__device__ __forceinline__ int quant_lsb(double v) {
+    const unsigned long long b = (unsigned long long)__double_as_longlong(v) & 0x7fffffffffffffffull;
+    if (b == 0) return 900;
+    const int e = (int)(b >> 52);
+    const unsigned long long m = (b & 0xfffffffffffffull) | (e ? 1ull << 52 : 0ull);
+    return max(e, 1) - 1075 + (__ffsll((long long)m) - 1);
+}
+
+// V consecutive dimensions per thread (V = 4: d % 4 == 0, 16-byte loads). 64 threads
+// side by side take the (block, dimensions) pairs, the four groups of 64 a quarter
+// of the block's rows each; their results are joined in row order through shared
+// memory.
+template <int V>
+__global__ void __launch_bounds__(256) k_quant_colpart(const float* __restrict__ x, size_t n, size_t d, size_t nsub,
+                                                       QuantSub* __restrict__ sub, uint32_t* __restrict__ tiny) {
+    constexpr int kParts = kQsubRows / kQpartRows;
+    static_assert(kParts == 4, "256 threads: four parts of 64");
+    __shared__ double sum_s[kParts - 1][V][64];
+    __shared__ float rng_s[kParts - 1][4][V][64];
+    __shared__ uint32_t tiny_s[kParts - 1][V][64];
+    const size_t dq = d / V;
+    const int lt = threadIdx.x & 63, part = threadIdx.x >> 6;
+    const size_t e = (size_t)blockIdx.x * 64 + lt;
+    const bool live = e < nsub * dq;
+    const size_t s = live ? e / dq : 0, q = live ? e - s * dq : 0;
+    const size_t r0 = s * kQsubRows + (size_t)part * kQpartRows;
+    const float* p = x + r0 * d + q * V;
+    const int rows = live && r0 < n ? (int)min((size_t)kQpartRows, n - r0) : 0;
+    // The prefix sums' range comes from two f32 chains rounded up and down: the f64
+    // conversions it would take otherwise cost more issue time than the loads.
+    double acc[V];
+    float up[V], dn[V], lo[V], hi[V];
+    uint32_t tn[V];
+#pragma unroll
+    for (int i = 0; i < V; i++) {
+        acc[i] = 0.0;
+        up[i] = dn[i] = lo[i] = hi[i] = 0.0f;
+        tn[i] = 0xffffffffu;
+    }
+    auto take = [&](const float (&v)[V]) {
+#pragma unroll
+        for (int i = 0; i < V; i++) {
+            acc[i] = __dadd_rn(acc[i], (double)v[i]);
+            dn[i] = __fadd_rd(dn[i], v[i]);
+            up[i] = __fadd_ru(up[i], v[i]);
+            lo[i] = fminf(lo[i], dn[i]);
+            hi[i] = fmaxf(hi[i], up[i]);
+            tn[i] = min(tn[i], quant_tiny(v[i]));
         }
-        qs_cp_commit();  // an empty group past the end keeps the group count uniform
     };
-#pragma unroll
-    for (int s = 0; s < kQsumStages - 1; s++) issue(s);
-    double acc = 0.0;
-    for (size_t c = 0; c < nchunks; c++) {
-        issue(c + kQsumStages - 1);
-        qs_cp_wait<kQsumStages - 1>();  // this thread's copies of chunk c have landed
-        __syncthreads();                  // everyone's have
-        if (warp == 0) {
-            const float* src = qs_stage + (c % kQsumStages) * (kQsumRows * 32);
-            const int rows = (int)min((size_t)kQsumRows, n - c * kQsumRows);
-            int r = 0;
-            for (; r + 16 <= rows; r += 16) {  // loads ahead of the dependent adds
-                float v[16];
-#pragma unroll
-                for (int i = 0; i < 16; i++) v[i] = src[(r + i) * 32 + lane];
-#pragma unroll
-                for (int i = 0; i < 16; i++) acc = __dadd_rn(acc, (double)v[i]);
-            }
-            for (; r < rows; r++) acc = __dadd_rn(acc, (double)src[r * 32 + lane]);
+    auto load = [&](int r, float (&v)[V]) {
+        if constexpr (V == 4) {
+            const float4 f = __ldg(reinterpret_cast<const float4*>(p + (size_t)r * d));
+            v[0] = f.x; v[1] = f.y; v[2] = f.z; v[3] = f.w;
+        } else {
+            v[0] = __ldg(p + (size_t)r * d);
         }
-        __syncthreads();  // the stage is free before it is refilled
+    };
+    int r = 0;
+    for (; r + 8 <= rows; r += 8) {
+        float v[8][V];
+#pragma unroll
+        for (int u = 0; u < 8; u++) load(r + u, v[u]);
+#pragma unroll
+        for (int u = 0; u < 8; u++) take(v[u]);
+    }
+    for (; r < rows; r++) {
+        float v[V];
+        load(r, v);
+        take(v);
+    }
+    if (part > 0) {
+#pragma unroll
+        for (int i = 0; i < V; i++) {
+            sum_s[part - 1][i][lt] = acc[i];
+            rng_s[part - 1][0][i][lt] = dn[i];
+            rng_s[part - 1][1][i][lt] = up[i];
+            rng_s[part - 1][2][i][lt] = lo[i];
+            rng_s[part - 1][3][i][lt] = hi[i];
+            tiny_s[part - 1][i][lt] = tn[i];
+        }
+    }
+    __syncthreads();
+    if (part > 0 || !live) return;
+#pragma unroll
+    for (int i = 0; i < V; i++) {
+#pragma unroll
+        for (int o = 0; o < kParts - 1; o++) {
+            lo[i] = fminf(lo[i], __fadd_rd(dn[i], rng_s[o][2][i][lt]));
+            hi[i] = fmaxf(hi[i], __fadd_ru(up[i], rng_s[o][3][i][lt]));
+            dn[i] = __fadd_rd(dn[i], rng_s[o][0][i][lt]);
+            up[i] = __fadd_ru(up[i], rng_s[o][1][i][lt]);
+            acc[i] = __dadd_rn(acc[i], sum_s[o][i][lt]);
+            tn[i] = min(tn[i], tiny_s[o][i][lt]);
+        }
+        QuantSub o;
+        o.sum = acc[i];
+        o.lo = lo[i];
+        o.hi = hi[i];
+        sub[s * d + q * V + i] = o;
+        tiny[s * d + q * V + i] = tn[i];
+    }
+}
+
+__device__ __forceinline__ double quant_scan32(double v, int lane) {
+#pragma unroll
+    for (int o = 1; o < 32; o <<= 1) {
+        const double u = __shfl_up_sync(0xffffffffu, v, o);
+        if (lane >= o) v = __dadd_rn(v, u);
+    }
+    return v;
+}
+
+__device__ __forceinline__ double quant_two_sum_err(double a, double b, double s) {
+    const double bb = __dsub_rn(s, a);
+    return __dadd_rn(__dsub_rn(a, __dsub_rn(s, bb)), __dsub_rn(b, bb));
+}
+
+// acc after 64 rows (lane i holds rows i and 32 + i), every rounding of the chain
+// kept. Mostly no add rounds after all: one look at all 64 partial sums shows that
+// (acc + the values' prefix sum is the chain's partial sum up to and including the
+// first add that rounds, and its two-sum error shows which that is). The rest is
+// then added one by one, from the warp's shared memory. The look needs the prefix
+// sums to be exact: 64 times the largest value within 53 bits of the lowest bit.
+// chain: straight to the adds. rough counts the groups that needed most of them.
+__device__ __forceinline__ double quant_replay64(double acc, float x0, float x1, int lane, bool chain, double* buf,
+                                                 int& rough) {
+    int s0 = 0;
+    if (!chain) {
+        const uint32_t tn = __reduce_min_sync(0xffffffffu, min(quant_tiny(x0), quant_tiny(x1)));
+        if (tn == 0xffffffffu) return acc;  // zeros change nothing
+        const uint32_t mx = __reduce_max_sync(
+            0xffffffffu, max(__float_as_uint(x0) & 0x7fffffffu, __float_as_uint(x1) & 0x7fffffffu));
+        if (mx < 0x7f800000u && isfinite(acc) &&
+            64.0 * (double)__uint_as_float(mx) <= quant_pow2(53 + quant_tiny_lsb(tn))) {
+            const double i0 = quant_scan32((double)x0, lane), i1r = quant_scan32((double)x1, lane);
+            const double i1 = __dadd_rn(__shfl_sync(0xffffffffu, i0, 31), i1r);
+            const double p0 = __dadd_rn(acc, i0), p1 = __dadd_rn(acc, i1);
+            const unsigned b0 = __ballot_sync(0xffffffffu, quant_two_sum_err(acc, i0, p0) != 0.0);
+            const unsigned b1 = __ballot_sync(0xffffffffu, quant_two_sum_err(acc, i1, p1) != 0.0);
+            if (!(b0 | b1)) return __shfl_sync(0xffffffffu, p1, 31);
+            const int f = b0 ? __ffs((int)b0) - 1 : __ffs((int)b1) - 1;
+            acc = __shfl_sync(0xffffffffu, b0 ? p0 : p1, f);
+            s0 = f + (b0 ? 1 : 33);
+        }
+        rough += s0 == 0 || s0 < 33;
+    }
+    buf[lane] = (double)x0;
+    buf[32 + lane] = (double)x1;
+    __syncwarp();
+#pragma unroll
+    for (int i = 0; i < 64; i += 16) {
+        if (i + 16 > s0) {
+            double u[16];
+#pragma unroll
+            for (int j = 0; j < 16; j++) u[j] = buf[i + j];
+#pragma unroll
+            for (int j = 0; j < 16; j++)
+                if (i + j >= s0) acc = __dadd_rn(acc, u[j]);
+        }
+    }
+    __syncwarp();
+    return acc;
+}
+
+// One warp per dimension; first / last: the sample's first / last slab of rows
+// (carry holds the sums in between). sub = nullptr: no entries, every block is
+// replayed (short samples: n <= kQscanShort, where the entries' launch costs more
+// than they save).
+// Where the adds round often (magnitudes spread over many binades), looking first is
+// slower than the chain: a block with two or more groups of 64 rows that needed
+// most of it sends the next kQscanChain blocks straight there, the rows of each on
+// their way while the one before is added. Magnitudes over 60 binades, 200,000 x 64:
+// 2.1 ms (1.77 ms for the bare chain); squares of normals 1.9 ms; normals 0.11 ms.
+constexpr size_t kQscanShort = 2048;
+constexpr int kQscanChain = 32;
+__global__ void __launch_bounds__(32 * kQscanWarps) k_quant_colscan(const float* __restrict__ x, size_t n, size_t d,
+                                                                    size_t nsub, const QuantSub* __restrict__ sub,
+                                                                    const uint32_t* __restrict__ tiny,
+                                                                    double* __restrict__ carry, bool first, bool last,
+                                                                    size_t n_all, float* __restrict__ shift) {
+    __shared__ QuantSub ring_s[kQscanWarps][kQscanDepth][32];
+    __shared__ uint32_t ring_t[kQscanWarps][kQscanDepth][32];
+    __shared__ __align__(16) double chain_s[kQscanWarps][64];
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    const size_t t = (size_t)blockIdx.x * kQscanWarps + warp;
+    if (t >= d) return;
+    const size_t nb = (nsub + 31) / 32;
+    auto issue = [&](size_t b) {  // each lane copies, and later reads, its own entries only
+        const size_t s = b * 32 + lane;
+        if (s < nsub) {
+            qs_cp_async16(reinterpret_cast<float*>(&ring_s[warp][b % kQscanDepth][lane]),
+                          reinterpret_cast<const float*>(sub + s * d + t));
+            qs_cp_async4(reinterpret_cast<float*>(&ring_t[warp][b % kQscanDepth][lane]),
+                         reinterpret_cast<const float*>(tiny + s * d + t));
+        }
+        qs_cp_commit();
+    };
+    double acc = first ? 0.0 : carry[t];
+    constexpr int kPer = kQsubRows / 32;
+    float ahead[kPer];  // rows of block ahead_s, loaded before they are needed
+    size_t ahead_s = ~(size_t)0;
+    int chain = 0;
+    auto rows_of = [&](size_t s, float (&v)[kPer]) {
+#pragma unroll
+        for (int u = 0; u < kPer; u++) {
+            const size_t r = s * kQsubRows + u * 32 + lane;
+            v[u] = r < n ? __ldg(x + r * d + t) : 0.0f;
+        }
+    };
+    auto replay = [&](size_t s) {
+        float v[kPer];
+        if (s == ahead_s) {
+#pragma unroll
+            for (int u = 0; u < kPer; u++) v[u] = ahead[u];
+        } else {
+            rows_of(s, v);
+        }
+        if (chain > 0 || !sub) {
+            ahead_s = s + 1;
+            rows_of(ahead_s, ahead);
+        }
+        int rough = 0;
+#pragma unroll
+        for (int u = 0; u < kPer; u += 2) acc = quant_replay64(acc, v[u], v[u + 1], lane, chain > 0, chain_s[warp], rough);
+        chain = rough >= 2 ? kQscanChain : max(chain - 1, 0);
+    };
+    if (!sub) {
+        for (size_t s = 0; s < nsub; s++) replay(s);
+    } else {
+        for (int b = 0; b < kQscanDepth - 1; b++) issue(b);
+    }
+    for (size_t b = 0; sub && b < nb; b++) {
+        issue(b + kQscanDepth - 1);
+        qs_cp_wait<kQscanDepth - 1>();
+        QuantSub e{0.0, 0.0f, 0.0f};
+        uint32_t tn = 0xffffffffu;
+        if (b * 32 + lane < nsub) {
+            e = ring_s[warp][b % kQscanDepth][lane];
+            tn = ring_t[warp][b % kQscanDepth][lane];
+        }
+        const int qx = quant_tiny_lsb(tn);
+        const int qmin = __reduce_min_sync(0xffffffffu, qx);
+        if (qmin == 900) continue;  // nothing but zeros
+        const float mag = fmaxf(fabsf(e.lo), fabsf(e.hi));
+        const float magmax = __uint_as_float(__reduce_max_sync(0xffffffffu, __float_as_uint(mag)));
+        // Sums of any of these blocks are exact; otherwise one block at a time.
+        const bool wide = 32.0 * (double)magmax < quant_pow2(53 + qmin);
+        const bool fin = isfinite(e.sum);
+        for (int s0 = 0; s0 < 32;) {
+            if (chain > 0) {
+                if (b * 32 + s0 < nsub) replay(b * 32 + s0);
+                s0++;
+                continue;
+            }
+            const int lim = wide ? 32 : s0 + 1;
+            double before = 0.0;  // of the blocks s0 .. lane - 1
+            if (wide) {
+                before = __shfl_up_sync(0xffffffffu, quant_scan32(lane >= s0 ? e.sum : 0.0, lane), 1);
+                if (lane == 0) before = 0.0;
+            }
+            const double p = __dadd_rn(acc, before);
+            bool ok = tn == 0xffffffffu || isnan(p) || (isinf(p) && fin);
+            if (!ok) {
+                const double top = quant_pow2(53 + min(qx, quant_lsb(p)));
+                ok = fin && (double)mag < quant_pow2(53 + qx) && __dadd_ru(p, (double)e.hi) <= top &&
+                     __dadd_rd(p, (double)e.lo) >= -top;
+            }
+            const unsigned bad = __ballot_sync(0xffffffffu, lane >= s0 && lane < lim && !ok);
+            if (!bad) {
+                acc = __shfl_sync(0xffffffffu, __dadd_rn(p, e.sum), lim - 1);
+                s0 = lim;
+                continue;
+            }
+            const int f = __ffs((int)bad) - 1;
+            acc = __shfl_sync(0xffffffffu, p, f);
+            replay(b * 32 + f);
+            s0 = f + 1;
+        }
     }
     qs_cp_wait<0>();
-    if (warp == 0 && c0 + lane < d) shift[c0 + lane] = __double2float_rn(__ddiv_rn(acc, (double)n));
+    if (lane == 0) {
+        if (last) shift[t] = __double2float_rn(__ddiv_rn(acc, (double)n_all));
+        else carry[t] = acc;
+    }
 }
 
 // The element-wise passes visit elements e = 4 * t + j * S (t the global thread
@@ -216,13 +481,22 @@ __global__ void __launch_bounds__(kQThreads) k_quant_extreme(const float* __rest
 #pragma unroll
         for (int i = 0; i < 4; i++) s[i] = shift[(4 * t + i) % d];
         const float4* x4 = reinterpret_cast<const float4*>(x);
-        for (size_t g = t; g < N4; g += nthr) {
-            const float4 v = __ldg(x4 + g);
+        auto take4 = [&](const float4& v) {
             take(quant_mag_bits(v.x, s[0]));
             take(quant_mag_bits(v.y, s[1]));
             take(quant_mag_bits(v.z, s[2]));
             take(quant_mag_bits(v.w, s[3]));
+        };
+        size_t g = t;
+        for (; g + 3 * nthr < N4; g += 4 * nthr) {  // four loads in flight
+            const float4 a = __ldg(x4 + g), b = __ldg(x4 + g + nthr), c = __ldg(x4 + g + 2 * nthr),
+                         e = __ldg(x4 + g + 3 * nthr);
+            take4(a);
+            take4(b);
+            take4(c);
+            take4(e);
         }
+        for (; g < N4; g += nthr) take4(__ldg(x4 + g));
     }
     if (t < N - 4 * N4) {
         const size_t e = 4 * N4 + t;

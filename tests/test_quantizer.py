@@ -157,3 +157,51 @@ def test_quantizer_errors(emb, qa):
     with pytest.raises(emb.EngineError):
         emb.Int8Quantizer(4, shift, 1.0).quantize_resident(a)
     a.close()
+
+
+def _chain_rows(kind, n, d, rng):
+    """Rows whose f64 column chains stress the block sums: where partial sums round, and where they do not."""
+    x = rng.standard_normal((n, d))
+    if kind == "wide":  # every add rounds: exponents over 60 binades
+        x *= np.exp2(rng.integers(-40, 20, (n, d)).astype(np.float64))
+    elif kind == "offset":  # a large mean: the sums climb through many binades
+        x = x + 1000.0
+    elif kind == "near_zero":  # squares: many magnitudes near zero under a growing sum
+        x = x * x
+    elif kind == "cancel":  # huge terms that cancel to what is left of small ones
+        x[1::2] = -x[:n - n % 2:2]
+        x *= 2.0 ** 100
+        x[::7] = 2.0 ** -30
+    elif kind == "zeros":
+        x[rng.random((n, d)) < 0.9] = 0.0
+        x[rng.random((n, d)) < 0.3] *= -0.0
+    elif kind == "subnormal":
+        x *= 2.0 ** -140
+    elif kind == "largest":  # the block sums leave the f32 range
+        x = np.copysign(3.4e38, x)
+    elif kind == "nonfinite":
+        x[n // 2, 0] = np.inf
+        x[n // 3, d // 2] = np.nan
+        x[n - 1, d - 1] = -np.inf
+    return x.astype(np.float32)
+
+
+@pytest.mark.parametrize("kind", ["plain", "wide", "offset", "near_zero", "cancel", "zeros", "subnormal", "largest",
+                                  "nonfinite"])
+@pytest.mark.parametrize("n,d", [(63, 4), (255, 3), (256, 4), (257, 8), (256 * 32, 5), (2048, 6), (2049, 7), (256 * 32 + 1, 36), (70001, 12)])
+def test_row_order_sums_bit_exact(emb, orc, qa, kind, n, d):
+    x = _chain_rows(kind, n, d, np.random.default_rng(n + d))
+    q = emb.Int8Quantizer.fit(x, d, emb.Calibration.faiss(), assigner=qa)
+    shift, _ = orc.quantizer_fit(x)
+    assert np.array_equal(np.isnan(q.shift), np.isnan(shift))
+    ok = ~np.isnan(shift)
+    assert np.array_equal(q.shift[ok].view(np.uint32), shift[ok].view(np.uint32))
+
+
+def test_row_order_sums_over_several_slabs(emb, orc, qa):
+    # wide enough that the block entries of all rows do not fit at once
+    n, d = 8200, 40001
+    x = (np.random.default_rng(5).standard_normal((n, d), dtype=np.float32) + np.float32(0.7))
+    q = emb.Int8Quantizer.fit(x, d, emb.Calibration.faiss(), assigner=qa)
+    shift, scale = orc.quantizer_fit(x)
+    assert np.array_equal(q.shift.view(np.uint32), shift.view(np.uint32)) and q.scale == np.float32(scale)
