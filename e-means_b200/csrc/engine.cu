@@ -37,6 +37,7 @@
 #include "kernels_batched.cuh"
 
 constexpr int kRefineCap = 32;  // candidates kept per refined row
+constexpr size_t kBlindMin = 2048, kBlindMax = 65536;  // rows of a search without a host read in its middle
 constexpr size_t kMaxSearchRows = (size_t)1 << 26;  // rows per search pass (32-bit row indexing inside)
 
 using namespace emb;
@@ -631,10 +632,13 @@ bool tc_supported(const emb200_handle* h, int nterms, bool fp8 = false) {
     return L.stages >= 2 && L.total + 1024 <= (uint32_t)kTcSmemLimit;
 }
 
-// Column splits of the tensor-core search: the one with the fewest waves of CTAs
-// times the tiles a CTA takes (plus half a tile of per-CTA setup), a larger
-// split only when it saves 3%. 394 row tiles on 148 SMs: 3 splits, 8 waves of 22
-// tiles, against 3 waves of 64 unsplit.
+// Column splits of the tensor-core search: the one with the fewest waves of items
+// times the tiles an item takes plus two tiles' time for its rows and the drain of
+// its accumulators, a larger split only when it saves 3%. 394 row tiles on 148 SMs:
+// 3 splits, 8 waves of 22 tiles, against 3 waves of 64 unsplit. Half a tile for an
+// item split too much: 20,011 x 100 rows against 1031 centroids 55 -> 38 us (three
+// terms) and 91 -> 38 us (single term), 19,000 x 4096 single term 81 -> 57 us; 3 or
+// 5 tiles measured the same as 2 or slower.
 //
 // Splits with the same tiles per CTA form runs of consecutive counts, and within
 // a run the waves never decrease with the count, so only the first count of each
@@ -649,7 +653,7 @@ int tc_nsplit(const emb200_handle* h, size_t m) {
     for (int ns = 1; ns <= ntiles;) {
         const int per_cta = (ntiles + ns - 1) / ns;
         const double waves = (double)((row_tiles * ns + sms - 1) / sms);
-        const double cost = waves * ((double)per_cta + 0.5);
+        const double cost = waves * ((double)per_cta + 2.0);
         if (ns == 1 || cost < 0.97 * best_cost) {
             best = ns;
             best_cost = cost;
@@ -736,15 +740,22 @@ int launch_tc(emb200_handle* h, const T* x, const uint32_t* gather, const uint32
     return launch_tc_kernel<T, COLLECT, false>(h, x, p, nsplit, st);
 }
 
-// Fold the device counters of one pipeline run into the handle's stats.
-int finish_counters(emb200_handle* h, cudaStream_t st, bool refined) {
-    uint32_t c[5];
+// The device counters of one pipeline run, and the fast kernel's time (waits for the stream).
+int read_counters(emb200_handle* h, cudaStream_t st, uint32_t (&c)[5]) {
     CK(cudaMemcpyAsync(c, h->counters.p, sizeof c, cudaMemcpyDeviceToHost, st));
     CK(cudaStreamSynchronize(st));
+    float kms = 0.0f;
+    CK(cudaEventElapsedTime(&kms, h->evk0, h->evk1));
+    h->stats.fast_ms += kms;
+    h->stats.fast_launches += 1;
+    return EMB200_OK;
+}
+
+// Fold them into the handle's stats.
+void fold_counters(emb200_handle* h, const uint32_t (&c)[5], bool refined) {
     h->stats.rows_certified += c[1];
     h->stats.rows_researched += refined ? c[3] : c[0];
     if (c[2] || c[4]) h->stats.fast_aborted = 1;
-    return EMB200_OK;
 }
 
 // Full pipeline of one assign over m rows already on the device (x, or
@@ -928,38 +939,63 @@ int settle_rows(emb200_handle* h, const T* x, const uint32_t* gather, size_t m, 
                                                                ka2, kb2, row_bounds, kr);
     }
     CKL();
-    if (graph) {
+    // Batches of some size: the host does not wait for the uncertified rows' count
+    // either. The read costs 12 us, the launches whose rows it would have spared 2 us
+    // each; a few rows are usually all certified, many rows need the exact grids.
+    const bool blind = !graph && m > kBlindMin && m <= kBlindMax;
+    if (graph || blind) {
         // No host reads: every later launch takes its row count from the device
         // counters (grids sized for all m rows, surplus CTAs leave at once).
         const uint32_t* exhaustive = h->redo_rows.p;
         const uint32_t* exhaustive_count = ctr;
+        const int ntiles = (int)((h->k + kTcBN - 1) / kTcBN);
+        Scratch scratch(h->device, st);
         if (tc_supported(h, refine_terms)) {
             const int cap = kRefineCap;
-            if (h->cand.ensure(m * cap) || h->cand_count.ensure(m) || h->redo2_rows.ensure(m))
-                return fail(h, EMB200_ENOMEM, "refine allocation failed for %zu rows", m);
-            CK(cudaMemsetAsync(h->cand_count.p, 0, m * sizeof(uint32_t), st));
-            const int ntl = (int)((h->k + kTcBN - 1) / kTcBN);
-            int rc = launch_tc<T, true>(h, x, gather, h->redo_rows.p, m, refine_terms, h->redo_theta.p, h->cand.p,
-                                        h->cand_count.p, cap, (int*)(ctr + 4), st, ctr, std::min(ntl, 4));
+            uint32_t *cand = nullptr, *cand_count = nullptr, *redo2 = nullptr;
+            if (blind) {  // room for all m rows, most of it untouched: from the shared pool
+                if (scratch.alloc(m * (cap + 2) * sizeof(uint32_t)))
+                    return fail(h, EMB200_ENOMEM, "refine allocation failed for %zu rows", m);
+                cand = (uint32_t*)scratch.p;
+                cand_count = cand + m * cap;
+                redo2 = cand_count + m;
+            } else {
+                if (h->cand.ensure(m * cap) || h->cand_count.ensure(m) || h->redo2_rows.ensure(m))
+                    return fail(h, EMB200_ENOMEM, "refine allocation failed for %zu rows", m);
+                cand = h->cand.p;
+                cand_count = h->cand_count.p;
+                redo2 = h->redo2_rows.p;
+            }
+            CK(cudaMemsetAsync(cand_count, 0, m * sizeof(uint32_t), st));
+            // (nsplit: the kernel picks its own from the rows there are)
+            int rc = launch_tc<T, true>(h, x, gather, h->redo_rows.p, m, refine_terms, h->redo_theta.p, cand,
+                                        cand_count, cap, (int*)(ctr + 4), st, ctr, ntiles);
             if (rc) return rc;
             k_rescore_cands<T><<<(unsigned)((m + 7) / 8), 256, 0, st>>>(
-                x, gather, d, h->c.p, h->norms.p, match, h->redo_rows.p, ctr, h->cand.p, h->cand_count.p, cap,
-                (const int*)(ctr + 4), labels, dist, h->redo2_rows.p, ctr + 3);
+                x, gather, d, h->c.p, h->norms.p, match, h->redo_rows.p, ctr, cand, cand_count, cap,
+                (const int*)(ctr + 4), labels, dist, redo2, ctr + 3);
             CKL();
-            exhaustive = h->redo2_rows.p;
+            exhaustive = redo2;
             exhaustive_count = ctr + 3;
         }
-        return launch_research(h, x, gather, m, exhaustive, exhaustive_count, labels, dist, st);
+        const int rc = launch_research(h, x, gather, m, exhaustive, exhaustive_count, labels, dist, st);
+        if (rc || graph) return rc;
+        uint32_t c[5];
+        const int rc2 = read_counters(h, st, c);
+        if (rc2) return rc2;
+        h->stats.rows_refined += c[0];
+        fold_counters(h, c, exhaustive_count == ctr + 3);
+        return EMB200_OK;
     }
-    uint32_t nredo = 0;
-    CK(cudaMemcpyAsync(&nredo, ctr, sizeof nredo, cudaMemcpyDeviceToHost, st));
-    CK(cudaStreamSynchronize(st));
-    float kms = 0.0f;
-    CK(cudaEventElapsedTime(&kms, h->evk0, h->evk1));
-    h->stats.fast_ms += kms;
-    h->stats.fast_launches += 1;
+    uint32_t c0[5];
+    const int rc0 = read_counters(h, st, c0);
+    if (rc0) return rc0;
+    const uint32_t nredo = c0[0];
     h->stats.rows_refined += nredo;
-    if (nredo == 0) return finish_counters(h, st, false);
+    if (nredo == 0) {
+        fold_counters(h, c0, false);
+        return EMB200_OK;
+    }
     const uint32_t* exhaustive = h->redo_rows.p;
     const uint32_t* exhaustive_count = ctr;
     if (tc_supported(h, refine_terms)) {
@@ -981,7 +1017,10 @@ int settle_rows(emb200_handle* h, const T* x, const uint32_t* gather, size_t m, 
     // at most nredo rows reach the exhaustive list: grids sized by it, not by m
     const int rc = launch_research(h, x, gather, nredo, exhaustive, exhaustive_count, labels, dist, st);
     if (rc) return rc;
-    return finish_counters(h, st, exhaustive_count == ctr + 3);
+    CK(cudaMemcpyAsync(c0, ctr, sizeof c0, cudaMemcpyDeviceToHost, st));
+    CK(cudaStreamSynchronize(st));
+    fold_counters(h, c0, exhaustive_count == ctr + 3);
+    return EMB200_OK;
 }
 
 int assign_dispatch(emb200_handle* h, int dtype, const void* x, const uint32_t* gather, size_t m, uint32_t* labels,

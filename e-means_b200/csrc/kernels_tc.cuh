@@ -773,25 +773,28 @@ struct TcBest {
 //   warp 0      TMA producer of the centroid stages (and each tile's norms)
 //   warp 1      TMEM allocation; tcgen05.mma issue (one thread)
 //   warps 2-3   row loaders: the next work item's row tile into the other buffer
-//               (BF16 hi/lo split or e4m3 with a per-row scale)
+//               (BF16 hi/lo split or e4m3 with a per-row scale); the first item's
+//               rows, and all of them with a single buffer, are loaded by the
+//               epilogue warps
 //   warps 4-19  epilogue, four warps per TMEM lane quarter, 64 columns of each
 //               256-column tile per warp: all 64 loaded (four 16-column loads,
 //               one wait), the accumulator released, then the 64 scored
 // COLLECT = false: per-row (best key, column, lower bound of the rest) to part_s/part_i.
 // COLLECT = true : every centroid with approximate score <= theta[row] is appended
 //                  to cand[row][*] (cand_count[row] counts all, capped storage).
-// Certification of one work item's 128 rows by the two row-loader warps, 16 rows
-// at a time with four threads per row (k_certify16v's decisions, so every value
-// has the same bits). fin[r]: the row's merged (best key, column, bound of the
-// rest) as scores. valid = false (the item's results never completed: the CTA
-// gave up): every row is listed for the exhaustive search instead. valid must
-// be the same across each warp.
+// Certification of one work item's 128 rows with four threads per row (k_certify16v's
+// decisions, so every value has the same bits): by the two row-loader warps, 16 rows
+// at a time, while the next item is searched, and for a CTA's last item, which
+// nothing follows, by the 16 epilogue warps at once (in the loaders it took 10 of the
+// 50 us of a 16384 x 4096 search). Threads lt = 0 .. nthr - 1. fin[r]: the row's
+// merged (best key, column, bound of the rest) as scores. valid = false (the item's
+// results never completed: the CTA gave up): every row is listed for the exhaustive
+// search instead. valid must be the same across each warp.
 EMB_DEV void tc_fused_certify(const TcParams& p, const float* __restrict__ x, const uint32_t* __restrict__ fin,
-                              int row0, int m, bool valid) {
-    const int lt = (int)threadIdx.x - 32 * (kTcEpi0 - kTcLoadWarps);  // 0 .. 63
+                              int row0, int m, bool valid, int lt, int nthr) {
     const int q = lt & 3, lane = (int)threadIdx.x & 31;
     const int d = p.d, k = p.k;
-    for (int r0 = 0; r0 < kTcBM; r0 += 8 * kTcLoadWarps) {
+    for (int r0 = 0; r0 < kTcBM; r0 += nthr / 4) {
         const int r = r0 + (lt >> 2);
         const int row = row0 + r;
         const bool live = row < m;
@@ -887,7 +890,14 @@ k_assign_tc(const T* __restrict__ x, const __grid_constant__ CUtensorMap map_hi,
         const int md = (int)*p.m_dev;
         m = md < m ? md : m;
     }
-    const int nsplit = p.nsplit;
+    int nsplit = p.nsplit;
+    if (COLLECT && p.m_dev) {
+        // The rows are usually few (the uncertified ones): their columns are split so
+        // that the grid's CTAs get one item each (4096 centroids, 7 row tiles, three
+        // terms: 36 -> 17 us a launch against a fixed split of 4).
+        const int rt = (m + kTcBM - 1) / kTcBM, nt = (p.k + kTcBN - 1) / kTcBN;
+        nsplit = max(1, min(nt, (int)gridDim.x / max(rt, 1)));
+    }
     const int nitems = ((m + kTcBM - 1) / kTcBM) * nsplit;
     if ((int)blockIdx.x >= nitems) return;  // no work: the whole CTA leaves before any setup
     const int my_items = (nitems - (int)blockIdx.x + (int)gridDim.x - 1) / (int)gridDim.x;
@@ -1070,9 +1080,9 @@ k_assign_tc(const T* __restrict__ x, const __grid_constant__ CUtensorMap map_hi,
         const int ltid = threadIdx.x - 64;
         // Fused certification (NM, TcParams::fuse): after loading item i's rows the
         // loaders certify item i - 1 (its merged top-2 is complete once the
-        // epilogue finishes that item, while item i is searched), and the last item
-        // after the loop. After an abort they load nothing more, but still list the
-        // rows of every item whose results never completed for the exact search.
+        // epilogue finishes that item, while item i is searched); the epilogue warps
+        // certify the last item. After an abort they load nothing more, but still list
+        // the rows of every item whose results never completed for the exact search.
         // Once a wait has failed, no later item counts as complete either (its
         // barrier phases no longer line up with the items).
         const bool fuse = NM && p.fuse;
@@ -1082,16 +1092,20 @@ k_assign_tc(const T* __restrict__ x, const __grid_constant__ CUtensorMap map_hi,
             valid = __all_sync(0xffffffffu, valid);
             fin_ok = valid;
             if constexpr (std::is_same<T, float>::value)
-                tc_fused_certify(p, x, fin, (item_of(j) / nsplit) * kTcBM, m, valid);
+                tc_fused_certify(p, x, fin, (item_of(j) / nsplit) * kTcBM, m, valid, ltid, kTcLoadWarps * 32);
             mbar_arrive(fin_empty);
         };
         bool loading = true;
         for (int i = 0; i < my_items; i++) {
             const int w = item_of(i);
             const int ab = i % NB;
-            if (loading && !mbar_wait(&a_empty[ab], ((uint32_t)(i / NB) & 1u) ^ 1u, abort_flag, kTcCtlSleepNs))
+            if (!FP8 && (i == 0 || NB == 1)) {
+                // loaded by the epilogue warps
+            } else if (loading && !mbar_wait(&a_empty[ab], ((uint32_t)(i / NB) & 1u) ^ 1u, abort_flag, kTcCtlSleepNs))
                 loading = false;
-            if (loading) {
+            if (!FP8 && (i == 0 || NB == 1)) {
+                if (!fuse && NB == 1) break;  // nothing left to do
+            } else if (loading) {
                 uint8_t* a = smem + ab * L.a_buf;
                 if (FP8)
                     tc_load_rows_fp8(a, rscale_s + (i % kTcRowScaleSlots) * kTcBM, x, p, (w / nsplit) * kTcBM, m,
@@ -1109,7 +1123,6 @@ k_assign_tc(const T* __restrict__ x, const __grid_constant__ CUtensorMap map_hi,
             }
             if (fuse && i > 0) certify_item(i - 1);
         }
-        if (fuse && my_items > 0) certify_item(my_items - 1);
     } else {
         // ---- epilogue: warps 4..19. Thread = row (TMEM lane); warp w takes the
         // 64-column quarter (w - 4) / 4 of every tile, as four 16-column halves.
@@ -1124,6 +1137,21 @@ k_assign_tc(const T* __restrict__ x, const __grid_constant__ CUtensorMap map_hi,
             const int w = item_of(i), split = w % nsplit;
             const int nt = tiles_of(split);
             const int row = (w / nsplit) * kTcBM + r;
+            if (!FP8 && (i == 0 || NB == 1) && ok) {
+                // The epilogue's 512 threads load the rows wherever nothing could hide the
+                // loaders' time (64 threads take about 10 us for 128 gathered rows of 128):
+                // a CTA's first item, and every item of a single row buffer (whose MMAs
+                // have all completed: the last tile's accumulator was full). Four lanes per
+                // warp make the loaders' 64 arrivals. 16,384 x 96 rows, k = 1024, three
+                // terms: 34 -> 20 us; the refine pass of 5% of 1M x 128 rows at k = 16384:
+                // 902 -> 675 us.
+                uint8_t* a = smem + (i % NB) * L.a_buf;
+                tc_load_rows(a, a + L.a_lo, x, p, (w / nsplit) * kTcBM, m, (int)threadIdx.x - 32 * kTcEpi0,
+                             kTcEpiWarps * 32, NM);
+                asm volatile("fence.proxy.async.shared::cta;" ::: "memory");  // visible to the tensor cores
+                __syncwarp();
+                if (lane < kTcLoadWarps * 32 / kTcEpiWarps) mbar_arrive(&a_full[i % NB]);
+            }
             TcBest best{INFINITY, INFINITY, 0xffffffffu};
             float theta = 0.0f;
             if (COLLECT) theta = row < m ? p.theta[row] : __int_as_float(0x7fc00000);
@@ -1282,7 +1310,15 @@ k_assign_tc(const T* __restrict__ x, const __grid_constant__ CUtensorMap map_hi,
                 asm volatile("bar.sync 1, %0;" ::"n"(kTcEpiWarps * 32) : "memory");
                 // The item's results are complete unless some role gave up (every failed
                 // wait raises the abort flag): hand them to the row loaders.
-                if (NM && p.fuse && warp == kTcEpi0 && lane == 0 && !*abort_flag) mbar_arrive(fin_full);
+                if (NM && p.fuse) {
+                    if (i + 1 < my_items) {
+                        if (warp == kTcEpi0 && lane == 0 && !*abort_flag) mbar_arrive(fin_full);
+                    } else if constexpr (std::is_same<T, float>::value) {
+                        const bool valid = __all_sync(0xffffffffu, !*abort_flag);
+                        tc_fused_certify(p, x, fin, (w / nsplit) * kTcBM, m, valid, (int)threadIdx.x - 32 * kTcEpi0,
+                                         kTcEpiWarps * 32);
+                    }
+                }
             }
         }
     }
