@@ -664,6 +664,35 @@ int tc_nsplit(const emb200_handle* h, size_t m) {
     return best;
 }
 
+// Tile and column splits of the FP32 SIMT search: 128 x 256 tiles (one CTA per SM),
+// or 64 x 64 (two) while those would leave SMs without work; the split with the
+// fewest waves of CTAs times the tiles each takes plus half a tile for its start and
+// merge.
+struct SimtPlan {
+    bool small;
+    int row_tiles, nsplit;
+};
+SimtPlan simt_plan(int sms, size_t m, size_t k) {
+    SimtPlan p;
+    sms = std::max(1, sms);
+    p.small = (m + SimtLarge::BM - 1) / SimtLarge::BM * ((k + SimtLarge::BN - 1) / SimtLarge::BN) < (size_t)sms;
+    const size_t bm = p.small ? SimtSmall::BM : SimtLarge::BM, bn = p.small ? SimtSmall::BN : SimtLarge::BN;
+    const long slots = p.small ? 2L * sms : sms;
+    p.row_tiles = (int)((m + bm - 1) / bm);
+    const int ntiles = (int)((k + bn - 1) / bn);
+    p.nsplit = 1;
+    double best = 0.0;
+    for (int ns = 1; ns <= std::min(ntiles, 64); ns++) {
+        const int per = (ntiles + ns - 1) / ns;
+        const double cost = (double)(((long)p.row_tiles * ns + slots - 1) / slots) * (per + 0.5);
+        if (ns == 1 || cost < 0.97 * best) {
+            best = cost;
+            p.nsplit = ns;
+        }
+    }
+    return p;
+}
+
 template <typename T, bool COLLECT, bool FP8, bool NM = false>
 int launch_tc_kernel(emb200_handle* h, const T* x, const TcParams& p, int nsplit, cudaStream_t st) {
     const TcLayout L = tc_layout(p.kpad, p.nterms, FP8, NM);
@@ -798,17 +827,10 @@ int assign_rows_dev(emb200_handle* h, const T* x, const uint32_t* gather, size_t
     // FP8 operands for f32 rows when prepared (d <= 256); otherwise the single-term BF16 search.
     const bool fp8 = prec == EMB200_PREC_FP8 && dtype == EMB200_F32 && tc_supported(h, 1, true);
     if (prec == EMB200_PREC_FP8 && !fp8) prec = EMB200_PREC_BF16X1;
-    const int row_tiles = (int)((m + kSimtBM - 1) / kSimtBM);
-    const int ntiles = (k + kSimtBN - 1) / kSimtBN;
     const int fast_terms = tc_terms(prec, dtype);
     const bool tc = prec != EMB200_PREC_FP32 && (fp8 || tc_supported(h, fast_terms));
-    int nsplit = 1;
-    if (tc) {
-        nsplit = tc_nsplit(h, m);
-    } else {
-        int target = 2 * h->sm_count;
-        if (row_tiles < target) nsplit = std::min(ntiles, (target + row_tiles - 1) / row_tiles);
-    }
+    const SimtPlan plan = simt_plan(h->sm_count, m, h->k);
+    const int nsplit = tc ? tc_nsplit(h, m) : plan.nsplit;
     // Inside the training loop (graph = true) nothing may allocate while an epoch is
     // captured, and a smaller batch can need more split partials than a full one
     // (fewer row tiles, more splits): size them for every batch of up to m rows.
@@ -819,13 +841,7 @@ int assign_rows_dev(emb200_handle* h, const T* x, const uint32_t* gather, size_t
     } else if (graph) {
         for (size_t rt = 1; rt * kTcBM < m + kTcBM; rt++) {
             const size_t mm = std::min(rt * kTcBM, m);
-            int ns = 1;
-            if (tc) {
-                ns = tc_nsplit(h, mm);
-            } else {
-                const int rtiles = (int)((mm + kSimtBM - 1) / kSimtBM), target = 2 * h->sm_count;
-                if (rtiles < target) ns = std::min(ntiles, (target + rtiles - 1) / rtiles);
-            }
+            const int ns = tc ? tc_nsplit(h, mm) : simt_plan(h->sm_count, mm, h->k).nsplit;
             part_rows = std::max(part_rows, (size_t)ns * mm);
         }
         h->part_size_m = m;
@@ -867,10 +883,17 @@ int assign_rows_dev(emb200_handle* h, const T* x, const uint32_t* gather, size_t
                                      (int*)(ctr + 2), st, nullptr, 0, fp8, fzp, &fused);
         if (rc) return rc;
     } else {
-        dim3 grid(row_tiles, nsplit);
-        int vec4 = (d % 4 == 0 && ((uintptr_t)x & 15) == 0) ? 1 : 0;
-        k_assign_simt<T><<<grid, kSimtThreads, 0, st>>>(x, gather, (int)m, d, h->c.p, h->norms.p, k, h->part_s.p,
-                                                         h->part_i.p, vec4);
+        const dim3 grid(plan.row_tiles, nsplit);
+        const int vec4 = (d % 4 == 0 && ((uintptr_t)x & 15) == 0) ? 1 : 0;
+        if (plan.small) {
+            SMEM_ATTR_ONCE((k_assign_simt<T, 1, 1>), SimtSmall::smem);
+            k_assign_simt<T, 1, 1><<<grid, kSimtThreads, SimtSmall::smem, st>>>(
+                x, gather, (int)m, d, h->c.p, h->norms.p, k, h->part_s.p, h->part_i.p, vec4);
+        } else {
+            SMEM_ATTR_ONCE((k_assign_simt<T, 2, 4>), SimtLarge::smem);
+            k_assign_simt<T, 2, 4><<<grid, kSimtThreads, SimtLarge::smem, st>>>(
+                x, gather, (int)m, d, h->c.p, h->norms.p, k, h->part_s.p, h->part_i.p, vec4);
+        }
         CKL();
     }
     if (!graph) CK(cudaEventRecord(h->evk1, st));
@@ -1514,15 +1537,12 @@ extern "C" int emb200_assign_f32_noalloc(const float* x_dev, size_t m, size_t d,
     uint32_t* ctr = (uint32_t*)(p + 256);  // [0] rows to re-search, [1] certified rows
     float* norms = (float*)(p + 512);
     float* part_s = (float*)(p + 512 + kNoAllocMaxK * 4);
-    const int row_tiles = (int)((m + kSimtBM - 1) / kSimtBM);
-    const int ntiles = (int)((k + kSimtBN - 1) / kSimtBN);
     const size_t pair_bytes = 2 * sizeof(float) + 2 * sizeof(uint32_t);
-    int nsplit = 1;
     int sms = 148;
     int dev = 0;
     if (cudaGetDevice(&dev) == cudaSuccess) cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
-    if (row_tiles < 2 * sms) nsplit = std::min(ntiles, (2 * sms + row_tiles - 1) / row_tiles);
-    nsplit = (int)std::max<size_t>(1, std::min<size_t>((size_t)nsplit, kNoAllocPartBytes / (m * pair_bytes)));
+    const SimtPlan plan = simt_plan(sms, m, k);
+    const int nsplit = (int)std::max<size_t>(1, std::min<size_t>((size_t)plan.nsplit, kNoAllocPartBytes / (m * pair_bytes)));
     uint32_t* part_i = (uint32_t*)(part_s + (size_t)nsplit * m * 2);
     uint32_t* redo = (uint32_t*)(p + 512 + kNoAllocMaxK * 4 + kNoAllocPartBytes);
     float* redo_theta = (float*)(redo + kNoAllocMaxRows);  // written by the certification, unused without refine
@@ -1531,8 +1551,18 @@ extern "C" int emb200_assign_f32_noalloc(const float* x_dev, size_t m, size_t d,
     k_prep_centroids<<<(unsigned)((k + 7) / 8), 256, 0, st>>>(centroids_dev, (int)k, (int)d, norms, bounds, nullptr,
                                                               nullptr, (int)((d + 63) / 64 * 64));
     const int vec4 = (d % 4 == 0 && ((uintptr_t)x_dev & 15) == 0 && ((uintptr_t)centroids_dev & 15) == 0) ? 1 : 0;
-    k_assign_simt<float><<<dim3(row_tiles, nsplit), kSimtThreads, 0, st>>>(
-        x_dev, nullptr, (int)m, (int)d, centroids_dev, norms, (int)k, part_s, part_i, vec4);
+    // Set on every call: the attribute belongs to the current context (see noalloc_scratch).
+    const void* search = plan.small ? (const void*)k_assign_simt<float, 1, 1> : (const void*)k_assign_simt<float, 2, 4>;
+    const size_t search_smem = plan.small ? SimtSmall::smem : SimtLarge::smem;
+    if (cudaFuncSetAttribute(search, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)search_smem) != cudaSuccess)
+        return EMB200_ECUDA;
+    const dim3 grid(plan.row_tiles, nsplit);
+    if (plan.small)
+        k_assign_simt<float, 1, 1><<<grid, kSimtThreads, search_smem, st>>>(
+            x_dev, nullptr, (int)m, (int)d, centroids_dev, norms, (int)k, part_s, part_i, vec4);
+    else
+        k_assign_simt<float, 2, 4><<<grid, kSimtThreads, search_smem, st>>>(
+            x_dev, nullptr, (int)m, (int)d, centroids_dev, norms, (int)k, part_s, part_i, vec4);
     float ka, kb;
     bound_coefficients(EMB200_PREC_FP32, EMB200_F32, d, false, &ka, &kb);
     // No refine pass here: uncertified rows (rare with FP32 scores) go straight to the exact search.

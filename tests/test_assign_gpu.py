@@ -454,3 +454,24 @@ def test_fp8_search_bit_exact(emb, orc, assigners, d, extreme):
     a.load_rows(x)
     lab, dist = a.assign_resident()
     assert np.array_equal(lab, rl) and same_f32(dist, rd)
+
+
+@pytest.mark.parametrize("dtype", ["f32", "u8", "i8"])
+@pytest.mark.parametrize("m,k,d", [(1, 1, 1), (63, 64, 16), (65, 63, 17), (128, 257, 4), (129, 255, 33),
+                                   (9472, 4096, 5), (19000, 256, 31), (19073, 769, 8)])
+def test_fp32_search_tile_edges(emb, orc, m, k, d, dtype):
+    # both tile forms of the FP32 search at their row, centroid and K remainders: the
+    # certified labels and distances are the reference's bits
+    rng = np.random.default_rng(m + k + d)
+    if dtype == "f32":
+        x = rng.standard_normal((m, d), dtype=np.float32)
+    else:
+        x = rng.integers(-120 if dtype == "i8" else 0, 121, (m, d)).astype({"i8": np.int8, "u8": np.uint8}[dtype])
+    c = rng.standard_normal((k, d), dtype=np.float32) * np.float32(1.0 if dtype == "f32" else 60.0)
+    a = emb.B200Assigner(0, precision="fp32")
+    a.set_centroids(c)
+    lab, dist = a.assign(x)
+    a.close()
+    ref_l, ref_d = orc.cpu_assign(x, c, kernel="avx512", emulate=not orc.has_kernel("avx512"))
+    assert np.array_equal(lab, ref_l)
+    assert np.array_equal(dist.view(np.uint32), ref_d.view(np.uint32))
