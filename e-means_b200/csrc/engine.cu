@@ -131,7 +131,7 @@ struct TrainState {
     DevBuf<float> usage, sums, pass_sums, batch_dist, alphas, xbatch;
     DevBuf<int> ctl;  // [0] step, [1] epoch, [2] last pass
     DevBuf<double> pass_sums64, keys, scalars, obj, gstream;
-    DevBuf<uint32_t> counts, offsets, slot, list, scratch, batch_labels, labels_all, order, didx, unused;
+    DevBuf<uint32_t> counts, offsets, slot, list, scratch, batch_labels, labels_all, order, didx, unused, crowded;
     DevBuf<unsigned long long> pass_counts;
     uint32_t* order_host = nullptr;  // pinned staging of the epoch's row order
     size_t order_host_n = 0;
@@ -144,6 +144,7 @@ struct TrainState {
         pass_sums64.release(); keys.release(); scalars.release(); obj.release(); gstream.release();
         counts.release(); offsets.release(); slot.release(); list.release(); scratch.release();
         batch_labels.release(); labels_all.release(); order.release(); didx.release(); unused.release();
+        crowded.release();
         pass_counts.release();
     }
 };
@@ -189,8 +190,13 @@ struct emb200_handle {
     CUtensorMap map_hi{}, map_lo{};  // TMA descriptors of c_hi / c_lo (128B swizzle, 64 x 128 boxes)
     bool maps_ok = false;
     // Half-norms split into BF16 parts for the single-term search that sums the
-    // norms inside the contraction ([whole tiles][16], k_prep_nrm16)
+    // norms inside the contraction ([whole tiles][16], nrm16_row); nrm16_ok: they
+    // match the norms (a bias changes those)
     DevBuf<__nv_bfloat16> nrm16;
+    bool nrm16_ok = false;
+    // A training loop is running whose step end zeroes the certification bounds, the
+    // search counters and the candidate counts for the next step.
+    bool steady = false;
     DevBuf<int8_t> c8;   // I8 centroids (CpuI8Assigner)
     DevBuf<int16_t> c16; // I16 centroids: round(c * 2^ishift)
     int ishift = 0;      // I16 scale exponent (src/cpu_i8.rs:97)
@@ -234,6 +240,7 @@ struct emb200_handle {
     DevBuf<uint32_t> cand, cand_count, redo2_rows;  // refine pass
     DevBuf<uint32_t> counters;  // see assign_rows_dev
     DevBuf<unsigned long long> rkeys;  // exhaustive search: per listed row (score, index) keys
+    DevBuf<uint32_t> rdone;            // and the slices of its centroids scored so far
 
     // training state
     TrainState train;
@@ -410,12 +417,8 @@ int encode_bf16_map(emb200_handle* h, CUtensorMap* map, void* base) {
 int prepare_centroids(emb200_handle* h) {
     cudaStream_t st = h->stream;
     const int k = (int)h->k, d = (int)h->d;
-    CK(cudaMemsetAsync(h->bounds.p, 0, sizeof(Bounds), st));
-    // Norms are padded to whole tiles with 3e38 (never a candidate, and finite
-    // so the packed top-2 keys of the padding stay numbers).
+    if (!h->steady) CK(cudaMemsetAsync(h->bounds.p, 0, sizeof(Bounds), st));
     const size_t kp = (h->k + kTcBN - 1) / kTcBN * kTcBN;
-    k_fill<<<(unsigned)((kp + 255) / 256), 256, 0, st>>>(h->norms.p, (int)kp, 3.0e38f);
-    CKL();
     h->kpad = (h->d + 63) / 64 * 64;
     __nv_bfloat16 *hi = nullptr, *lo = nullptr;
     h->maps_ok = false;
@@ -429,13 +432,13 @@ int prepare_centroids(emb200_handle* h) {
         if (rc) return rc;
         rc = encode_bf16_map(h, &h->map_lo, lo);
         if (rc) return rc;
-        // Allocated here, outside any captured epoch; filled before each search.
         if (h->nrm16.ensure(kp * 16)) return fail(h, EMB200_ENOMEM, "BF16 norm allocation failed");
         h->maps_ok = true;
     }
-    k_prep_centroids<<<(unsigned)((k + 7) / 8), 256, 0, st>>>(h->c.p, k, d, h->norms.p, h->bounds.p, hi, lo,
-                                                              (int)h->kpad);
+    k_prep_centroids<<<(unsigned)((kp + 7) / 8), 256, 0, st>>>(h->c.p, k, (int)kp, d, h->norms.p, h->bounds.p, hi, lo,
+                                                               (int)h->kpad, hi ? h->nrm16.p : nullptr);
     CKL();
+    h->nrm16_ok = hi != nullptr;
     h->f8_ok = false;
     if (h->opts.precision == EMB200_PREC_FP8 && h->d <= 256) {
         // e4m3 codes in rows of one or two 128-byte swizzle atoms; scoring norms are
@@ -504,6 +507,7 @@ int apply_bias(emb200_handle* h, const float* bias_dev) {
     const int k = (int)h->k;
     k_add_bias<<<(unsigned)((k + 255) / 256), 256, 0, st>>>(h->norms.p, bias_dev, k, h->bounds.p);
     CKL();
+    h->nrm16_ok = false;
     if (h->f8_ok) {
         k_add_bias_f8<<<(unsigned)((k + 255) / 256), 256, 0, st>>>(h->nf8.p, bias_dev, k);
         CKL();
@@ -743,8 +747,11 @@ int launch_tc(emb200_handle* h, const T* x, const uint32_t* gather, const uint32
         // (the certification bound allows for it whenever this mode is searched).
         const size_t kp = (h->k + kTcBN - 1) / kTcBN * kTcBN;
         if (nterms == 1 && h->nrm16.n >= kp * 16) {
-            k_prep_nrm16<<<(unsigned)((kp + 255) / 256), 256, 0, st>>>(h->norms.p, (int)kp, h->nrm16.p);
-            CKL();
+            if (!h->nrm16_ok) {
+                k_prep_nrm16<<<(unsigned)((kp + 255) / 256), 256, 0, st>>>(h->norms.p, (int)kp, h->nrm16.p);
+                CKL();
+                h->nrm16_ok = true;
+            }
             p.nrm16 = h->nrm16.p;
             if (fuse && nsplit == 1) {  // certification at the end of each item
                 p.fuse = 1;
@@ -811,12 +818,15 @@ int assign_rows_dev(emb200_handle* h, const T* x, const uint32_t* gather, size_t
     if (m > kMaxSearchRows) {
         // Pieces of at most 2^26 rows: the search kernels index rows (up to 32
         // threads each) in 32 bits.
+        const bool steady = h->steady;
+        h->steady = false;  // each piece starts from counters of its own
         for (size_t r0 = 0; r0 < m; r0 += kMaxSearchRows) {
             const size_t mc = std::min(kMaxSearchRows, m - r0);
             const T* xs = gather ? x : x + r0 * (size_t)d;
             int rc = assign_rows_dev(h, xs, gather ? gather + r0 : nullptr, mc, labels + r0, dist + r0, st, graph);
             if (rc) return rc;
         }
+        h->steady = steady;
         return EMB200_OK;
     }
     if (use_i8_mode(h, dtype)) {
@@ -853,7 +863,7 @@ int assign_rows_dev(emb200_handle* h, const T* x, const uint32_t* gather, size_t
         h->redo_theta.ensure(m) || h->counters.ensure(8))
         return fail(h, EMB200_ENOMEM, "scratch allocation failed for %zu rows", m);
     uint32_t* ctr = h->counters.p;
-    CK(cudaMemsetAsync(ctr, 0, 8 * sizeof(uint32_t), st));
+    if (!(graph && h->steady)) CK(cudaMemsetAsync(ctr, 0, 8 * sizeof(uint32_t), st));
     h->stats.fast_kernel = fp8 ? 4 : tc ? 1 : 0;
     if (!graph) CK(cudaEventRecord(h->evk0, st));
     bool fused = false;
@@ -902,21 +912,23 @@ int assign_rows_dev(emb200_handle* h, const T* x, const uint32_t* gather, size_t
 }
 
 // Exhaustive exact search of the rows listed in rows[0 .. *count) (count on the
-// device, at most m): each row's centroids are split over several CTAs.
+// device): each row's centroids are split over several CTAs. keys / done hold the
+// listed rows' start values already (k_rescore_cands), or are set here for m rows
+// (`init`: the rows come straight from the certification).
 template <typename T>
-int launch_research(emb200_handle* h, const T* x, const uint32_t* gather, size_t m, const uint32_t* rows,
-                    const uint32_t* count, uint32_t* labels, float* dist, cudaStream_t st) {
+int launch_research(emb200_handle* h, const T* x, const uint32_t* gather, size_t m, bool init, const uint32_t* rows,
+                    const uint32_t* count, unsigned long long* keys, uint32_t* done, uint32_t* labels, float* dist,
+                    cudaStream_t st) {
     const int k = (int)h->k;
     const int slices = std::max(1, std::min(64, (k + 2047) / 2048));
     const int span = (k + slices - 1) / slices;
-    if (h->rkeys.ensure(m)) return fail(h, EMB200_ENOMEM, "scratch allocation failed for %zu rows", m);
-    k_research_keys_init<<<(unsigned)((m + 255) / 256), 256, 0, st>>>(h->rkeys.p, m);
-    CKL();
+    if (init) {
+        k_research_keys_init<<<(unsigned)((m + 255) / 256), 256, 0, st>>>(keys, done, m);
+        CKL();
+    }
     k_research_split<T><<<h->sm_count * 4, 256, 0, st>>>(x, gather, (int)h->d, h->c.p, h->norms.p, k,
-                                                          h->opts.match_kernel, rows, count, slices, span, h->rkeys.p);
-    CKL();
-    k_research_finish<T><<<(unsigned)((m * 32 + 255) / 256), 256, 0, st>>>(x, gather, (int)h->d, rows, count,
-                                                                           h->rkeys.p, labels, dist);
+                                                          h->opts.match_kernel, rows, count, slices, span, keys, done,
+                                                          labels, dist);
     CKL();
     return EMB200_OK;
 }
@@ -973,35 +985,42 @@ int settle_rows(emb200_handle* h, const T* x, const uint32_t* gather, size_t m, 
         const uint32_t* exhaustive_count = ctr;
         const int ntiles = (int)((h->k + kTcBN - 1) / kTcBN);
         Scratch scratch(h->device, st);
-        if (tc_supported(h, refine_terms)) {
-            const int cap = kRefineCap;
-            uint32_t *cand = nullptr, *cand_count = nullptr, *redo2 = nullptr;
-            if (blind) {  // room for all m rows, most of it untouched: from the shared pool
-                if (scratch.alloc(m * (cap + 2) * sizeof(uint32_t)))
-                    return fail(h, EMB200_ENOMEM, "refine allocation failed for %zu rows", m);
-                cand = (uint32_t*)scratch.p;
-                cand_count = cand + m * cap;
-                redo2 = cand_count + m;
-            } else {
-                if (h->cand.ensure(m * cap) || h->cand_count.ensure(m) || h->redo2_rows.ensure(m))
-                    return fail(h, EMB200_ENOMEM, "refine allocation failed for %zu rows", m);
-                cand = h->cand.p;
-                cand_count = h->cand_count.p;
-                redo2 = h->redo2_rows.p;
-            }
-            CK(cudaMemsetAsync(cand_count, 0, m * sizeof(uint32_t), st));
+        const int cap = kRefineCap;
+        uint32_t *cand = nullptr, *cand_count = nullptr, *redo2 = nullptr, *done = nullptr;
+        unsigned long long* keys = nullptr;
+        const bool refine = tc_supported(h, refine_terms);
+        if (blind) {  // room for all m rows, most of it untouched: from the shared pool
+            if (scratch.alloc(m * ((cap + 3) * sizeof(uint32_t) + sizeof *keys)))
+                return fail(h, EMB200_ENOMEM, "refine allocation failed for %zu rows", m);
+            keys = (unsigned long long*)scratch.p;
+            cand = (uint32_t*)(keys + m);
+            cand_count = cand + m * cap;
+            redo2 = cand_count + m;
+            done = redo2 + m;
+        } else {
+            if ((refine && (h->cand.ensure(m * cap) || h->cand_count.ensure(m) || h->redo2_rows.ensure(m))) ||
+                h->rkeys.ensure(m) || h->rdone.ensure(m))
+                return fail(h, EMB200_ENOMEM, "refine allocation failed for %zu rows", m);
+            cand = h->cand.p;
+            cand_count = h->cand_count.p;
+            redo2 = h->redo2_rows.p;
+            keys = h->rkeys.p;
+            done = h->rdone.p;
+        }
+        if (refine) {
+            if (!(graph && h->steady)) CK(cudaMemsetAsync(cand_count, 0, m * sizeof(uint32_t), st));
             // (nsplit: the kernel picks its own from the rows there are)
             int rc = launch_tc<T, true>(h, x, gather, h->redo_rows.p, m, refine_terms, h->redo_theta.p, cand,
                                         cand_count, cap, (int*)(ctr + 4), st, ctr, ntiles);
             if (rc) return rc;
             k_rescore_cands<T><<<(unsigned)((m + 7) / 8), 256, 0, st>>>(
                 x, gather, d, h->c.p, h->norms.p, match, h->redo_rows.p, ctr, cand, cand_count, cap,
-                (const int*)(ctr + 4), labels, dist, redo2, ctr + 3);
+                (const int*)(ctr + 4), labels, dist, redo2, ctr + 3, keys, done);
             CKL();
             exhaustive = redo2;
             exhaustive_count = ctr + 3;
         }
-        const int rc = launch_research(h, x, gather, m, exhaustive, exhaustive_count, labels, dist, st);
+        const int rc = launch_research(h, x, gather, m, !refine, exhaustive, exhaustive_count, keys, done, labels, dist, st);
         if (rc || graph) return rc;
         uint32_t c[5];
         const int rc2 = read_counters(h, st, c);
@@ -1021,7 +1040,10 @@ int settle_rows(emb200_handle* h, const T* x, const uint32_t* gather, size_t m, 
     }
     const uint32_t* exhaustive = h->redo_rows.p;
     const uint32_t* exhaustive_count = ctr;
-    if (tc_supported(h, refine_terms)) {
+    if (h->rkeys.ensure(nredo) || h->rdone.ensure(nredo))
+        return fail(h, EMB200_ENOMEM, "refine allocation failed for %u rows", nredo);
+    const bool refine = tc_supported(h, refine_terms);
+    if (refine) {
         const int cap = kRefineCap;
         if (h->cand.ensure((size_t)nredo * cap) || h->cand_count.ensure(nredo) || h->redo2_rows.ensure(nredo))
             return fail(h, EMB200_ENOMEM, "refine allocation failed for %u rows", nredo);
@@ -1032,13 +1054,14 @@ int settle_rows(emb200_handle* h, const T* x, const uint32_t* gather, size_t m, 
         k_rescore_cands<T><<<(nredo + 7) / 8, 256, 0, st>>>(x, gather, d, h->c.p, h->norms.p, match, h->redo_rows.p,
                                                            ctr, h->cand.p, h->cand_count.p, cap,
                                                            (const int*)(ctr + 4), labels, dist, h->redo2_rows.p,
-                                                           ctr + 3);
+                                                           ctr + 3, h->rkeys.p, h->rdone.p);
         CKL();
         exhaustive = h->redo2_rows.p;
         exhaustive_count = ctr + 3;
     }
     // at most nredo rows reach the exhaustive list: grids sized by it, not by m
-    const int rc = launch_research(h, x, gather, nredo, exhaustive, exhaustive_count, labels, dist, st);
+    const int rc = launch_research(h, x, gather, nredo, !refine, exhaustive, exhaustive_count, h->rkeys.p, h->rdone.p,
+                                   labels, dist, st);
     if (rc) return rc;
     CK(cudaMemcpyAsync(c0, ctr, sizeof c0, cudaMemcpyDeviceToHost, st));
     CK(cudaStreamSynchronize(st));
@@ -1181,7 +1204,7 @@ int emb200_destroy(emb200_handle* h) {
     h->stage.release(); h->st_labels.release(); h->st_dist.release();
     h->part_s.release(); h->part_i.release(); h->redo_rows.release(); h->counters.release();
     h->redo_theta.release(); h->cand.release(); h->cand_count.release(); h->redo2_rows.release();
-    h->rkeys.release();
+    h->rkeys.release(); h->rdone.release();
     h->qshift.release(); h->qsel.release(); h->qclip.release(); h->qx.release(); h->qcodes.release();
     h->train.release();
     h->bat.release();
@@ -1548,8 +1571,8 @@ extern "C" int emb200_assign_f32_noalloc(const float* x_dev, size_t m, size_t d,
     float* redo_theta = (float*)(redo + kNoAllocMaxRows);  // written by the certification, unused without refine
     if (cudaMemsetAsync(p, 0, 512, st) != cudaSuccess) return EMB200_ECUDA;  // bounds and counters start at zero
     // Norms and the certification bounds (no BF16 split: the search here is FP32).
-    k_prep_centroids<<<(unsigned)((k + 7) / 8), 256, 0, st>>>(centroids_dev, (int)k, (int)d, norms, bounds, nullptr,
-                                                              nullptr, (int)((d + 63) / 64 * 64));
+    k_prep_centroids<<<(unsigned)((k + 7) / 8), 256, 0, st>>>(centroids_dev, (int)k, (int)k, (int)d, norms, bounds,
+                                                              nullptr, nullptr, (int)((d + 63) / 64 * 64), nullptr);
     const int vec4 = (d % 4 == 0 && ((uintptr_t)x_dev & 15) == 0 && ((uintptr_t)centroids_dev & 15) == 0) ? 1 : 0;
     // Set on every call: the attribute belongs to the current context (see noalloc_scratch).
     const void* search = plan.small ? (const void*)k_assign_simt<float, 1, 1> : (const void*)k_assign_simt<float, 2, 4>;

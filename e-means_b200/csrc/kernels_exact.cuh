@@ -93,43 +93,82 @@ EMB_DEV float group_dot_ref(int match, const T* x, const float* cg, int d, int l
     }
 }
 
-// set_centroids (src/cpu.rs:84-93): norms_j = sqnorm_ref(c_j); bounds for the
-// certification; optionally the BF16 hi/lo split (hi = bf16(c), lo = bf16(c - hi)),
-// written K-major into `split` with row stride `kpad` (hi at column t, lo at column kpad/2 + t).
-// One warp per centroid.
-__global__ void k_prep_centroids(const float* __restrict__ c, int k, int d, float* __restrict__ norms,
-                                 Bounds* __restrict__ bounds, __nv_bfloat16* __restrict__ hi,
-                                 __nv_bfloat16* __restrict__ lo, int kpad) {
-    int warp = (blockIdx.x * blockDim.x + threadIdx.x) >> 5;
-    int lane = threadIdx.x & 31;
-    if (warp >= k) return;
-    const float* cj = c + (size_t)warp * d;
-    float nrm = warp_sqnorm_ref(cj, d, lane);
-    float ss = 0.0f, ssh = 0.0f, ssd = 0.0f;
-    for (int i = lane; i < kpad; i += 32) {
-        float v = i < d ? cj[i] : 0.0f;
-        ss = __fmaf_ru(v, v, ss);
-        ssd = bf16_resid_sq(v, ssd);
-        if (hi) {
-            __nv_bfloat16 h = __float2bfloat16_rn(v);
-            float hf = __bfloat162float(h);
-            __nv_bfloat16 l = __float2bfloat16_rn(v - hf);
-            hi[(size_t)warp * kpad + i] = h;
-            lo[(size_t)warp * kpad + i] = l;
-            ssh = __fmaf_ru(hf, hf, ssh);
+// Norms inside the contraction (single-term BF16 search): row j of `out` (16 BF16)
+// holds the three BF16 parts of h = norms[j] / 2 (p1 = bf16(h), p2 = bf16(h - p1), p3 = bf16(h - p1 - p2);
+// both differences are exact in f32 and p3 is exact in BF16, so p1 + p2 + p3 = h
+// for every h in the normal range), then zeros. A non-finite h keeps p1 = h and
+// zeros after it, so the MMA sums the same +-inf or NaN the epilogue's
+// norm - 2 acc would give.
+EMB_DEV void nrm16_row(float norm, __nv_bfloat16* __restrict__ out) {
+    const float h = 0.5f * norm;
+    const __nv_bfloat16 p1 = __float2bfloat16_rn(h);
+    __nv_bfloat16 p2 = __float2bfloat16_rn(0.0f), p3 = p2;
+    if (isfinite(h)) {
+        const float r1 = h - __bfloat162float(p1);
+        p2 = __float2bfloat16_rn(r1);
+        p3 = __float2bfloat16_rn(r1 - __bfloat162float(p2));
+    }
+    uint4* o = reinterpret_cast<uint4*>(out);
+    o[0] = make_uint4((uint32_t)__bfloat16_as_ushort(p1) | ((uint32_t)__bfloat16_as_ushort(p2) << 16),
+                      (uint32_t)__bfloat16_as_ushort(p3), 0u, 0u);
+    o[1] = make_uint4(0u, 0u, 0u, 0u);
+}
+
+constexpr float kPadNorm = 3.0e38f;  // norms of the padding: never a candidate, and finite, so that keys stay numbers
+
+// set_centroids (src/cpu.rs:84-93): norms_j = sqnorm_ref(c_j), kPadNorm up to kp;
+// bounds for the certification (max-ed into *bounds, which starts at zero);
+// optionally the BF16 hi/lo split (hi = bf16(c), lo = bf16(c - hi)) with row stride
+// kpad, and the half-norms of nrm16_row. One warp per centroid; a block's maxima are
+// joined before the four atomics: one per centroid on the same addresses was most of
+// the kernel's 13 us at 4096 x 128 (now 3.4).
+__global__ void __launch_bounds__(256) k_prep_centroids(const float* __restrict__ c, int k, int kp, int d,
+                                                        float* __restrict__ norms, Bounds* __restrict__ bounds,
+                                                        __nv_bfloat16* __restrict__ hi, __nv_bfloat16* __restrict__ lo,
+                                                        int kpad, __nv_bfloat16* __restrict__ nrm16) {
+    __shared__ float4 part[8];
+    const int w = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    const int j = (int)blockIdx.x * 8 + w;
+    float4 mx = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
+    if (j < k) {
+        const float* cj = c + (size_t)j * d;
+        const float nrm = warp_sqnorm_ref(cj, d, lane);
+        float ss = 0.0f, ssh = 0.0f, ssd = 0.0f;
+        for (int i = lane; i < kpad; i += 32) {
+            const float v = i < d ? cj[i] : 0.0f;
+            ss = __fmaf_ru(v, v, ss);
+            ssd = bf16_resid_sq(v, ssd);
+            if (hi) {
+                const __nv_bfloat16 h = __float2bfloat16_rn(v);
+                const float hf = __bfloat162float(h);
+                hi[(size_t)j * kpad + i] = h;
+                lo[(size_t)j * kpad + i] = __float2bfloat16_rn(v - hf);
+                ssh = __fmaf_ru(hf, hf, ssh);
+            }
         }
+        for (int o = 16; o; o >>= 1) {
+            ss = __fadd_ru(ss, __shfl_xor_sync(kFull, ss, o));
+            ssh = __fadd_ru(ssh, __shfl_xor_sync(kFull, ssh, o));
+            ssd = __fadd_ru(ssd, __shfl_xor_sync(kFull, ssd, o));
+        }
+        if (lane == 0) {
+            norms[j] = nrm;
+            if (nrm16) nrm16_row(nrm, nrm16 + (size_t)j * 16);
+        }
+        mx = make_float4(__fmul_ru(__fsqrt_ru(ss), 1.0000005f), fabsf(nrm), __fmul_ru(__fsqrt_ru(ssh), 1.0000005f),
+                         __fmul_ru(__fsqrt_ru(ssd), 1.0000005f));
+    } else if (j < kp && lane == 0) {
+        norms[j] = kPadNorm;
+        if (nrm16) nrm16_row(kPadNorm, nrm16 + (size_t)j * 16);
     }
-    for (int o = 16; o; o >>= 1) {
-        ss = __fadd_ru(ss, __shfl_xor_sync(kFull, ss, o));
-        ssh = __fadd_ru(ssh, __shfl_xor_sync(kFull, ssh, o));
-        ssd = __fadd_ru(ssd, __shfl_xor_sync(kFull, ssd, o));
-    }
-    if (lane == 0) {
-        norms[warp] = nrm;
-        atomic_max_pos(&bounds->cmax, __fmul_ru(__fsqrt_ru(ss), 1.0000005f));
-        atomic_max_pos(&bounds->nmax, fabsf(nrm));
-        atomic_max_pos(&bounds->cmax_hi, __fmul_ru(__fsqrt_ru(ssh), 1.0000005f));
-        atomic_max_pos(&bounds->dmax, __fmul_ru(__fsqrt_ru(ssd), 1.0000005f));
+    if (lane == 0) part[w] = mx;
+    __syncthreads();
+    if (threadIdx.x < 4) {
+        // The maxima as bit patterns: the values are non-negative or NaN, and a NaN's
+        // pattern is above every number's, as in atomic_max_pos.
+        uint32_t m = 0;
+        for (int q = 0; q < 8; q++) m = max(m, __float_as_uint(reinterpret_cast<const float*>(&part[q])[threadIdx.x]));
+        if (m) atomicMax(reinterpret_cast<unsigned int*>(bounds) + threadIdx.x, m);
     }
 }
 
@@ -424,6 +463,9 @@ __global__ void k_certify16v(const float* __restrict__ x, const uint32_t* __rest
     certify_tally(ok, redo, row, theta, cert_count, redo_count, redo_rows, redo_theta);
 }
 
+// (+inf, label 0): a row of the exhaustive search that nothing has scored yet.
+constexpr unsigned long long kResearchNone = (unsigned long long)0xff800000u << 32;
+
 // Exact re-score of the refine pass's candidates (one warp per refined row):
 // the reference's label is the lowest-index minimum of the exact scores of the
 // candidates, because every centroid whose exact score could reach sb was
@@ -435,14 +477,21 @@ __global__ void k_rescore_cands(const T* __restrict__ x, const uint32_t* __restr
                                 const uint32_t* __restrict__ cand, const uint32_t* __restrict__ cand_count, int cap,
                                 const int* __restrict__ refine_err, uint32_t* __restrict__ labels,
                                 float* __restrict__ dist, uint32_t* __restrict__ redo2_rows,
-                                uint32_t* __restrict__ redo2_count) {
+                                uint32_t* __restrict__ redo2_count, unsigned long long* __restrict__ keys,
+                                uint32_t* __restrict__ done) {
     int i = (blockIdx.x * blockDim.x + threadIdx.x) >> 5;
     int lane = threadIdx.x & 31;
     if (i >= (int)*redo_count) return;
     uint32_t row = redo_rows[i];
     uint32_t cnt = cand_count[i];
+    auto list_exhaustive = [&]() {  // and start the row's exhaustive search (k_research_split)
+        const uint32_t slot = atomicAdd(redo2_count, 1u);
+        redo2_rows[slot] = row;
+        keys[slot] = kResearchNone;
+        done[slot] = 0u;
+    };
     if (cnt == 0 || cnt > (uint32_t)cap || *refine_err) {
-        if (lane == 0) redo2_rows[atomicAdd(redo2_count, 1u)] = row;
+        if (lane == 0) list_exhaustive();
         return;
     }
     size_t src = gather ? gather[row] : (size_t)row;
@@ -475,7 +524,7 @@ __global__ void k_rescore_cands(const T* __restrict__ x, const uint32_t* __restr
             labels[row] = lab;
             dist[row] = fmaxf(__fadd_rn(best, xn), 0.0f);
         } else {
-            redo2_rows[atomicAdd(redo2_count, 1u)] = row;
+            list_exhaustive();
         }
     }
 }
@@ -565,9 +614,12 @@ EMB_DEV float research_key_score(unsigned long long key) {
     return __uint_as_float((o & 0x80000000u) ? (o & 0x7fffffffu) : ~o);
 }
 
-__global__ void k_research_keys_init(unsigned long long* __restrict__ keys, size_t n) {
+__global__ void k_research_keys_init(unsigned long long* __restrict__ keys, uint32_t* __restrict__ done, size_t n) {
     const size_t i = (size_t)blockIdx.x * blockDim.x + threadIdx.x;
-    if (i < n) keys[i] = ((unsigned long long)0xff800000u << 32);  // (+inf, label 0)
+    if (i < n) {
+        keys[i] = kResearchNone;
+        done[i] = 0u;
+    }
 }
 
 template <typename T>
@@ -576,8 +628,11 @@ __global__ void __launch_bounds__(256) k_research_split(const T* __restrict__ x,
                                                         const float* __restrict__ norms, int k, int match,
                                                         const uint32_t* __restrict__ rows,
                                                         const uint32_t* __restrict__ count, int slices, int span,
-                                                        unsigned long long* __restrict__ keys) {
+                                                        unsigned long long* __restrict__ keys,
+                                                        uint32_t* __restrict__ done, uint32_t* __restrict__ labels,
+                                                        float* __restrict__ dist) {
     __shared__ unsigned long long sk[32];
+    __shared__ bool last_s;
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
     const int gsz = match == kMatchAvx512 ? 16 : 8;
     const int gpw = 32 / gsz;
@@ -612,29 +667,22 @@ __global__ void __launch_bounds__(256) k_research_split(const T* __restrict__ x,
             unsigned long long b = ~0ull;
             for (int q = 0; q < G; q++) b = min(b, sk[q]);
             if (b != ~0ull) atomicMin(&keys[r], b);
+            __threadfence();  // the key before the count
+            last_s = atomicAdd(&done[r], 1u) == (uint32_t)slices - 1u;
+        }
+        __syncthreads();
+        // The row's last slice writes its label and distance, max(best + sqnorm(x), 0).
+        if (last_s && warp == 0) {
+            const float xn = warp_sqnorm_ref(xr, d, lane);
+            if (lane == 0) {
+                __threadfence();
+                const unsigned long long key = atomicMin(&keys[r], ~0ull);
+                labels[row] = (uint32_t)(key & 0xffffffffu);
+                dist[row] = fmaxf(__fadd_rn(research_key_score(key), xn), 0.0f);
+            }
         }
         __syncthreads();
     }
 }
-
-// Labels and distances of the split search: dist = max(best + sqnorm(x), 0). One warp per row.
-template <typename T>
-__global__ void k_research_finish(const T* __restrict__ x, const uint32_t* __restrict__ gather, int d,
-                                  const uint32_t* __restrict__ rows, const uint32_t* __restrict__ count,
-                                  const unsigned long long* __restrict__ keys, uint32_t* __restrict__ labels,
-                                  float* __restrict__ dist) {
-    const uint32_t r = (uint32_t)(((size_t)blockIdx.x * blockDim.x + threadIdx.x) >> 5);
-    const int lane = threadIdx.x & 31;
-    if (r >= *count) return;
-    const uint32_t row = rows[r];
-    const size_t src = gather ? gather[row] : (size_t)row;
-    const float xn = warp_sqnorm_ref(x + src * (size_t)d, d, lane);
-    if (lane == 0) {
-        const unsigned long long key = keys[r];
-        labels[row] = (uint32_t)(key & 0xffffffffu);
-        dist[row] = fmaxf(__fadd_rn(research_key_score(key), xn), 0.0f);
-    }
-}
-
 
 }  // namespace emb

@@ -671,27 +671,11 @@ EMB_DEV void mma_e4m3(uint32_t d_tmem, uint64_t adesc, uint64_t bdesc, uint32_t 
         ::"r"(d_tmem), "l"(adesc), "l"(bdesc), "r"(idesc), "r"(accumulate));
 }
 
-// Norms inside the contraction: row j of `out` (16 BF16) holds the three BF16
-// parts of h = norms[j] / 2 (p1 = bf16(h), p2 = bf16(h - p1), p3 = bf16(h - p1 - p2);
-// both differences are exact in f32 and p3 is exact in BF16, so p1 + p2 + p3 = h
-// for every h in the normal range), then zeros. A non-finite h keeps p1 = h and
-// zeros after it, so the MMA sums the same +-inf or NaN the epilogue's
-// norm - 2 acc would give. Rows up to kp (whole tiles): the padding's 3e38 too.
+// The half-norms again after a bias changed the norms (k_prep_centroids writes them
+// otherwise). Rows up to kp (whole tiles): the padding too.
 __global__ void k_prep_nrm16(const float* __restrict__ norms, int kp, __nv_bfloat16* __restrict__ out) {
     const int j = blockIdx.x * blockDim.x + threadIdx.x;
-    if (j >= kp) return;
-    const float h = 0.5f * norms[j];
-    const __nv_bfloat16 p1 = __float2bfloat16_rn(h);
-    __nv_bfloat16 p2 = __float2bfloat16_rn(0.0f), p3 = p2;
-    if (isfinite(h)) {
-        const float r1 = h - __bfloat162float(p1);
-        p2 = __float2bfloat16_rn(r1);
-        p3 = __float2bfloat16_rn(r1 - __bfloat162float(p2));
-    }
-    uint4* o = reinterpret_cast<uint4*>(out + (size_t)j * 16);
-    o[0] = make_uint4((uint32_t)__bfloat16_as_ushort(p1) | ((uint32_t)__bfloat16_as_ushort(p2) << 16),
-                      (uint32_t)__bfloat16_as_ushort(p3), 0u, 0u);
-    o[1] = make_uint4(0u, 0u, 0u, 0u);
+    if (j < kp) nrm16_row(norms[j], out + (size_t)j * 16);
 }
 
 // Scores of 16 accumulator columns (in place): s = norm - 2 acc (BF16), or

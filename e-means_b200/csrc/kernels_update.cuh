@@ -3,7 +3,10 @@
 // closing mean, all in the reference's f32 operation order so that a training
 // run on the device follows the CPU trajectory bit for bit.
 #pragma once
+#include <type_traits>
+
 #include "common.cuh"
+#include "kernels_exact.cuh"
 
 namespace emb {
 
@@ -20,14 +23,6 @@ __global__ void k_gather_centroids(const T* __restrict__ x, const uint32_t* __re
 __global__ void k_fill_u32(uint32_t* __restrict__ p, size_t n, uint32_t v) {
     size_t i = (size_t)blockIdx.x * blockDim.x + threadIdx.x;
     if (i < n) p[i] = v;
-}
-
-// counts[l]++ per batch row; slot[i] = this row's arrival order within its label
-// (arbitrary; put back in row order by k_segment_sums).
-__global__ void k_label_hist(const uint32_t* __restrict__ labels, int m, uint32_t* __restrict__ counts,
-                             uint32_t* __restrict__ slot) {
-    int i = blockIdx.x * blockDim.x + threadIdx.x;
-    if (i < m) slot[i] = atomicAdd(&counts[labels[i]], 1u);
 }
 
 // Exclusive prefix sum of counts[0..k) -> offsets (one CTA of 1024 threads).
@@ -58,6 +53,55 @@ __global__ void k_label_scatter(const uint32_t* __restrict__ labels, const uint3
                                 const uint32_t* __restrict__ offsets, uint32_t* __restrict__ list) {
     int i = blockIdx.x * blockDim.x + threadIdx.x;
     if (i < m) list[offsets[labels[i]] + slot[i]] = (uint32_t)i;
+}
+
+// k_exclusive_scan and k_label_scatter in one launch (k <= kScanScatterMaxK): every
+// block of 1024 scans all k counts into its shared memory (16 KB from L2 at k = 4096,
+// less than the launch it saves) and places its own rows; block 0 keeps the offsets.
+// 6 -> 3 us a batch with the gap between them.
+constexpr int kScanScatterMaxK = 8192;
+__global__ void __launch_bounds__(1024) k_scan_scatter(const uint32_t* __restrict__ counts, int k,
+                                                       const uint32_t* __restrict__ labels,
+                                                       const uint32_t* __restrict__ slot, int m,
+                                                       uint32_t* __restrict__ offsets, uint32_t* __restrict__ list) {
+    __shared__ uint32_t off_s[kScanScatterMaxK];
+    __shared__ uint32_t wsum[32];
+    const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+    const int per = (k + 1023) / 1024, lo = tid * per;
+    uint32_t v[kScanScatterMaxK / 1024], sum = 0;
+#pragma unroll
+    for (int u = 0; u < kScanScatterMaxK / 1024; u++) {
+        v[u] = u < per && lo + u < k ? counts[lo + u] : 0u;
+        sum += v[u];
+    }
+    uint32_t incl = sum;
+    for (int o = 1; o < 32; o <<= 1) {
+        const uint32_t y = __shfl_up_sync(0xffffffffu, incl, o);
+        if (lane >= o) incl += y;
+    }
+    if (lane == 31) wsum[warp] = incl;
+    __syncthreads();
+    if (warp == 0) {
+        uint32_t w = wsum[lane];
+        for (int o = 1; o < 32; o <<= 1) {
+            const uint32_t y = __shfl_up_sync(0xffffffffu, w, o);
+            if (lane >= o) w += y;
+        }
+        wsum[lane] = w;
+    }
+    __syncthreads();
+    uint32_t base = (warp ? wsum[warp - 1] : 0u) + incl - sum;
+#pragma unroll
+    for (int u = 0; u < kScanScatterMaxK / 1024; u++) {
+        if (u < per && lo + u < k) {
+            off_s[lo + u] = base;
+            if (blockIdx.x == 0) offsets[lo + u] = base;
+            base += v[u];
+        }
+    }
+    __syncthreads();
+    const int i = blockIdx.x * 1024 + tid;
+    if (i < m) list[off_s[labels[i]] + slot[i]] = (uint32_t)i;
 }
 
 // Bitonic sort of E * 32 entries held E per lane (entry lane + 32 h in v[h]),
@@ -314,88 +358,230 @@ __global__ void k_segment_sums(const T* __restrict__ x, const uint32_t* __restri
                                *last_pass, pass_counts, pass_sums, pass_sums64, lane, stage, R);
 }
 
-// Per-cluster sums with the dimensions split over warps (f32 rows, d % 4 == 0,
-// 16-byte aligned rows, d <= kDgMaxD): block l sums cluster l, warp g dimensions
-// [32 g, 32 g + 32). Warp 0 puts the cluster's batch positions in row order
-// (as segment_sums_warp) and the block shares the sorted list; each warp then
+// The EMA step's weights of one cluster (State::apply, src/lib.rs:287-309): N *= (1 - a);
+// with n > 0 batch rows mass = N + a n, w = a n / mass, c += w (s/n - c) (c = s/n when w == 1).
+struct ApplyStep {
+    float n, w, usage;
+};
+EMB_DEV ApplyStep apply_step(float alpha, float usage, uint32_t cnt) {
+    const bool replace = alpha == 1.0f;
+    ApplyStep s;
+    s.usage = replace ? usage : __fmul_rn(usage, __fsub_rn(1.0f, alpha));
+    s.n = (float)cnt;
+    s.w = 0.0f;
+    if (cnt > 0) {
+        const float an = __fmul_rn(alpha, s.n);
+        const float mass = __fadd_rn(replace ? 0.0f : s.usage, an);
+        s.w = __fdiv_rn(an, mass);
+        s.usage = mass;
+    }
+    return s;
+}
+EMB_DEV float apply_dim(const ApplyStep& s, float c, float sum) {
+    const float mean = __fdiv_rn(sum, s.n);
+    return (s.w == 1.0f) ? mean : __fadd_rn(c, __fmul_rn(s.w, __fsub_rn(mean, c)));
+}
+
+// The update of the clusters of a batch (f32 rows, d % 4 == 0, 16-byte aligned rows,
+// d <= kDgMaxD): per-cluster sums in row order, the last pass's sums, and the EMA step
+// right from the registers that hold the sums. Two kernels:
+//   k_update_small  clusters of up to kSmallRows batch rows (most: a batch has 4 to 16
+//                   rows per cluster), one warp per 32 dimensions, no shared memory, so
+//                   that every SM holds all the warps it can; lists the others.
+//   k_update_big    the listed clusters, one block each: their rows stream through a
+//                   ring in shared memory (below).
+// With the ring's 16 KB per warp for every cluster, three blocks fitted an SM and the
+// 4096 clusters of a 16,384 x 128 batch took nine rounds of them: 27 us, and 4 us
+// for the EMA step's own kernel; now 12.6 + 1.3 us (1024 clusters of 96, some with
+// 200 rows: 15 + 4 -> 9 + 11).
+// counts[l] is zero again afterwards, for the next batch's histogram.
+constexpr uint32_t kSmallRows = 64;
+
+struct UpdateArgs {
+    const float* x;
+    const uint32_t* rows;
+    int d, k;
+    uint32_t* counts;
+    const uint32_t* offsets;
+    uint32_t *list, *scratch;
+    float *c, *usage;
+    const float* alphas;
+    const int* step;
+    const int* last_pass;
+    unsigned long long* pass_counts;
+    float* pass_sums;
+    double* pass_sums64;
+    uint32_t* crowded;        // clusters of more than kSmallRows rows
+    uint32_t* crowded_count;  // zero before the batch
+};
+
+// One cluster's sum of one dimension into the centroid and the pass sums.
+EMB_DEV void update_dim(const UpdateArgs& a, int l, int t, float acc, double acc64, const ApplyStep& s, bool last) {
+    const size_t e = (size_t)l * a.d + t;
+    a.c[e] = apply_dim(s, a.c[e], acc);
+    if (last) {
+        if (a.pass_sums64) a.pass_sums64[e] += acc64;
+        else a.pass_sums[e] = __fadd_rn(a.pass_sums[e], acc);
+    }
+}
+
+// blockDim (32 ceil(d / 32), clusters per block).
+__global__ void __launch_bounds__(384) k_update_small(const UpdateArgs a) {
+    const int l = blockIdx.x * blockDim.y + threadIdx.y, lane = threadIdx.x & 31, t = threadIdx.x;
+    const uint32_t c = l < a.k ? a.counts[l] : 0u;
+    const bool mine = l < a.k && c <= kSmallRows;
+    ApplyStep s{0.0f, 0.0f, 0.0f};
+    if (mine) {
+        const float alpha = a.alphas[*a.step];
+        s = apply_step(alpha, a.usage[l], c);
+        if (c > 0) {
+            // Batch positions back in row order (two registers hold up to 64), then
+            // the rows they name.
+            const uint32_t* seg = a.list + a.offsets[l];
+            uint32_t v[2] = {(uint32_t)lane < c ? seg[lane] : 0xffffffffu,
+                             (uint32_t)(lane + 32) < c ? seg[lane + 32] : 0xffffffffu};
+            if (c > 32) {
+                warp_bitonic_regs<2>(v, lane);
+            } else {
+                uint32_t u[1] = {v[0]};
+                warp_bitonic_regs<1>(u, lane);
+                v[0] = u[0];
+            }
+            const uint32_t r0 = (uint32_t)lane < c ? a.rows[v[0]] : 0u;
+            const uint32_t r1 = (uint32_t)(lane + 32) < c ? a.rows[v[1]] : 0u;
+            float acc = 0.0f;
+            double acc64 = 0.0;
+            const bool last = *a.last_pass;
+            auto rows_at = [&](uint32_t j0, auto width) {  // the loads of several rows, then their adds in order
+                constexpr uint32_t W = decltype(width)::value;
+                float xv[W];
+#pragma unroll
+                for (uint32_t u = 0; u < W; u++) {
+                    const uint32_t j = j0 + u;
+                    const uint32_t src = __shfl_sync(0xffffffffu, j0 < 32 ? r0 : r1, (int)(j & 31));
+                    xv[u] = j < c && t < a.d ? __ldg(a.x + (size_t)src * a.d + t) : 0.0f;
+                }
+#pragma unroll
+                for (uint32_t u = 0; u < W; u++) {
+                    if (j0 + u < c) {
+                        acc = __fadd_rn(acc, xv[u]);
+                        if (a.pass_sums64) acc64 += (double)xv[u];
+                    }
+                }
+            };
+            for (uint32_t j0 = 0; j0 < c; j0 += 16) {
+                if (c - j0 <= 4) rows_at(j0, std::integral_constant<uint32_t, 4>{});
+                else if (c - j0 <= 8) rows_at(j0, std::integral_constant<uint32_t, 8>{});
+                else rows_at(j0, std::integral_constant<uint32_t, 16>{});
+            }
+            if (t < a.d) update_dim(a, l, t, acc, acc64, s, last);
+            if (last && t == 0) a.pass_counts[l] += c;
+        }
+    }
+    __syncthreads();  // every warp of the cluster has read its count and usage
+    if (t == 0 && l < a.k) {
+        if (mine) {
+            a.usage[l] = s.usage;
+            a.counts[l] = 0;
+        } else {
+            a.crowded[atomicAdd(a.crowded_count, 1u)] = (uint32_t)l;
+        }
+    }
+}
+
+// The crowded clusters: block b takes entries b, b + gridDim.x, ...; warp g sums
+// dimensions [32 g, 32 g + 32). Warp 0 puts the cluster's batch positions in row
+// order (as segment_sums_warp) and the block shares the sorted list; each warp then
 // streams its 128-byte slice of every row through a ring of kDgStages chunks of
 // kDgRows rows (cp.async, kDgStages - 1 chunks in flight) and adds them in row
 // order, lane t one dimension. A crowded cluster's rows are read by d / 32 warps
-// with up to 14 KB in flight each, where the one-warp form has 12 KB for all d.
+// with up to 14 KB in flight each, where the one-warp form has 12 KB for all d. The
+// rows' numbers are looked up once, by all threads, before the ring starts: looked up
+// by each chunk, two dependent loads stood before each of its first seven copies.
 constexpr int kDgRows = 16, kDgStages = 8;
+constexpr uint32_t kDgIds = 2048;  // row numbers kept in shared memory
 constexpr size_t kDgWarpBytes = (size_t)kDgStages * kDgRows * 32 * sizeof(float);
 constexpr int kDgMaxD = 384;  // 12 warps x 16 KB of ring
 
-__global__ void __launch_bounds__(384) k_segment_sums_dg(const float* __restrict__ x,
-                                                         const uint32_t* __restrict__ rows, int d,
-                                                         const uint32_t* __restrict__ counts,
-                                                         const uint32_t* __restrict__ offsets,
-                                                         uint32_t* __restrict__ list, uint32_t* __restrict__ scratch,
-                                                         float* __restrict__ sums, const int* __restrict__ last_pass,
-                                                         unsigned long long* __restrict__ pass_counts,
-                                                         float* __restrict__ pass_sums,
-                                                         double* __restrict__ pass_sums64) {
+__global__ void __launch_bounds__(384) k_update_big(const UpdateArgs a) {
     extern __shared__ float dg_stage[];  // (blockDim / 32) x kDgStages x kDgRows x 32 floats
     __shared__ int use_scratch;
-    const int l = blockIdx.x, warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-    const uint32_t c = counts[l];
-    if (c == 0) return;  // uniform over the block
-    uint32_t* seg_list = list + offsets[l];
-    uint32_t* seg_scratch = scratch + 2 * (size_t)offsets[l];
-    if (warp == 0) {
-        const uint32_t* sorted = warp_sort_segment(seg_list, c, seg_scratch, lane);
-        if (lane == 0) use_scratch = sorted != seg_list;
-    }
-    __syncthreads();
-    const uint32_t* seg = use_scratch ? seg_scratch : seg_list;
-    const int t0 = warp * 32;
-    const int nd = min(32, d - t0);  // dimensions of this warp (a multiple of 4)
-    const int ppr = nd >> 2;         // 16-byte pieces per row
-    float* ring = dg_stage + (size_t)warp * kDgStages * kDgRows * 32;
-    const uint32_t nq = (c + kDgRows - 1) / kDgRows;
-    auto issue = [&](uint32_t q) {
-        if (q < nq) {
-            const uint32_t j0 = q * kDgRows, n = min((uint32_t)kDgRows, c - j0);
-            const uint32_t myrow = (uint32_t)lane < n ? rows[seg[j0 + lane]] : 0u;
-            float* buf = ring + (size_t)(q % kDgStages) * kDgRows * 32;
-            for (uint32_t e0 = 0; e0 < n * (uint32_t)ppr; e0 += 32) {
-                const uint32_t e = e0 + lane, jj = e / (uint32_t)ppr, pc = e - jj * (uint32_t)ppr;
-                const uint32_t src = __shfl_sync(0xffffffffu, myrow, (int)min(jj, 31u));
-                if (e < n * (uint32_t)ppr) cp_async16(buf + jj * 32 + 4 * pc, x + (size_t)src * d + t0 + 4 * pc);
-            }
+    __shared__ uint32_t ids[kDgIds];
+    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, d = a.d;
+    const uint32_t ncrowded = *a.crowded_count;
+    const float alpha = a.alphas[*a.step];
+    const bool last = *a.last_pass;
+    for (uint32_t e = blockIdx.x; e < ncrowded; e += gridDim.x) {
+        const int l = (int)a.crowded[e];
+        const uint32_t c = a.counts[l];
+        const ApplyStep step = apply_step(alpha, a.usage[l], c);
+        uint32_t* seg_list = a.list + a.offsets[l];
+        uint32_t* seg_scratch = a.scratch + 2 * (size_t)a.offsets[l];
+        if (warp == 0) {
+            const uint32_t* sorted = warp_sort_segment(seg_list, c, seg_scratch, lane);
+            if (lane == 0) use_scratch = sorted != seg_list;
         }
-        cp_async_commit();  // an empty group past the end keeps the group count uniform
-    };
+        __syncthreads();
+        const uint32_t* seg = use_scratch ? seg_scratch : seg_list;
+        for (uint32_t j = threadIdx.x; j < min(c, kDgIds); j += blockDim.x) ids[j] = a.rows[seg[j]];
+        __syncthreads();
+        const int t0 = warp * 32;
+        const int nd = min(32, d - t0);  // dimensions of this warp (a multiple of 4)
+        const int ppr = nd >> 2;         // 16-byte pieces per row
+        float* ring = dg_stage + (size_t)warp * kDgStages * kDgRows * 32;
+        const uint32_t nq = (c + kDgRows - 1) / kDgRows;
+        auto issue = [&](uint32_t q) {
+            if (q < nq) {
+                const uint32_t j0 = q * kDgRows, n = min((uint32_t)kDgRows, c - j0);
+                const uint32_t j = j0 + lane;
+                const uint32_t myrow = (uint32_t)lane < n ? (j < kDgIds ? ids[j] : a.rows[seg[j]]) : 0u;
+                float* buf = ring + (size_t)(q % kDgStages) * kDgRows * 32;
+                for (uint32_t e0 = 0; e0 < n * (uint32_t)ppr; e0 += 32) {
+                    const uint32_t p = e0 + lane, jj = p / (uint32_t)ppr, pc = p - jj * (uint32_t)ppr;
+                    const uint32_t src = __shfl_sync(0xffffffffu, myrow, (int)min(jj, 31u));
+                    if (p < n * (uint32_t)ppr) cp_async16(buf + jj * 32 + 4 * pc, a.x + (size_t)src * d + t0 + 4 * pc);
+                }
+            }
+            cp_async_commit();  // an empty group past the end keeps the group count uniform
+        };
 #pragma unroll
-    for (int q = 0; q < kDgStages - 1; q++) issue((uint32_t)q);
-    float acc = 0.0f;
-    double acc64 = 0.0;
-    const bool mine = lane < nd;
-    for (uint32_t q = 0; q < nq; q++) {
-        cp_async_wait<kDgStages - 2>();  // chunk q has landed
-        __syncwarp();
-        const float* buf = ring + (size_t)(q % kDgStages) * kDgRows * 32;
-        const uint32_t n = min((uint32_t)kDgRows, c - q * kDgRows);
-        if (mine) {
-            for (uint32_t jj = 0; jj < n; jj++) {
-                const float v = buf[jj * 32 + lane];
-                acc = __fadd_rn(acc, v);
-                if (pass_sums64) acc64 += (double)v;
+        for (int q = 0; q < kDgStages - 1; q++) issue((uint32_t)q);
+        float acc = 0.0f;
+        double acc64 = 0.0;
+        const bool mine = lane < nd;
+        for (uint32_t q = 0; q < nq; q++) {
+            cp_async_wait<kDgStages - 2>();  // chunk q has landed
+            __syncwarp();
+            const float* buf = ring + (size_t)(q % kDgStages) * kDgRows * 32;
+            const uint32_t n = min((uint32_t)kDgRows, c - q * kDgRows);
+            if (mine && n == kDgRows) {  // a whole chunk: its loads ahead of the dependent adds
+                float v[kDgRows];
+#pragma unroll
+                for (int jj = 0; jj < kDgRows; jj++) v[jj] = buf[jj * 32 + lane];
+#pragma unroll
+                for (int jj = 0; jj < kDgRows; jj++) {
+                    acc = __fadd_rn(acc, v[jj]);
+                    if (a.pass_sums64) acc64 += (double)v[jj];
+                }
+            } else if (mine) {
+                for (uint32_t jj = 0; jj < n; jj++) {
+                    const float v = buf[jj * 32 + lane];
+                    acc = __fadd_rn(acc, v);
+                    if (a.pass_sums64) acc64 += (double)v;
+                }
             }
+            __syncwarp();  // this buffer is refilled below, kDgStages - 1 chunks on
+            issue(q + kDgStages - 1);
         }
-        __syncwarp();  // this buffer is refilled below, kDgStages - 1 chunks on
-        issue(q + kDgStages - 1);
-    }
-    cp_async_wait<0>();
-    if (mine) {
-        const int t = t0 + lane;
-        sums[(size_t)l * d + t] = acc;
-        if (*last_pass) {
-            if (pass_sums64) pass_sums64[(size_t)l * d + t] += acc64;
-            else pass_sums[(size_t)l * d + t] = __fadd_rn(pass_sums[(size_t)l * d + t], acc);
+        cp_async_wait<0>();
+        if (mine) update_dim(a, l, t0 + lane, acc, acc64, step, last);
+        __syncthreads();  // every warp has read the cluster's count and usage
+        if (threadIdx.x == 0) {
+            if (last) a.pass_counts[l] += c;
+            a.usage[l] = step.usage;
+            a.counts[l] = 0;
         }
     }
-    if (*last_pass && threadIdx.x == 0) pass_counts[l] += c;
 }
 
 // The batch's rows gathered into one contiguous block (the proposer's search
@@ -406,13 +592,6 @@ __global__ void k_gather_rows(const float* __restrict__ x, const uint32_t* __res
     if (e >= (size_t)m * d) return;
     const size_t i = e / d, t = e - i * d;
     out[e] = x[(size_t)rows[i] * d + t];
-}
-
-// Last pass: labels[i] = l for every row of the batch (src/lib.rs:438-440).
-__global__ void k_store_labels(const uint32_t* __restrict__ batch_labels, const uint32_t* __restrict__ rows, int m,
-                               uint32_t* __restrict__ labels_all, const int* __restrict__ last_pass) {
-    int i = blockIdx.x * blockDim.x + threadIdx.x;
-    if (i < m && *last_pass) labels_all[rows[i]] = batch_labels[i];
 }
 
 // State::apply (src/lib.rs:287-309), one warp per cluster: N *= (1 - a) for all
@@ -480,13 +659,34 @@ __global__ void k_unbias_dist(float* __restrict__ dist, const uint32_t* __restri
     if (i < m && *penalized) dist[i] = fmaxf(__fsub_rn(dist[i], bias[labels[i]]), 0.0f);
 }
 
-// Batch objective (src/lib.rs:442-445): sum of distances in f64. A fixed-shape
-// tree (deterministic, ~1e-16 relative from the reference's sequential sum), or
-// the sequential sum itself when the value feeds the balance penalty.
-// One CTA of 1024; writes obj[0] += batch, mean_sqdist = batch / m.
-__global__ void __launch_bounds__(1024) k_batch_objective(const float* __restrict__ dist, int m, int sequential,
-                                                          double* __restrict__ objective, const int* __restrict__ epoch,
-                                                          double* __restrict__ mean_sqdist) {
+// What follows a batch's search and needs nothing but its labels and distances, in
+// one launch. Blocks 1 ..: per row, counts[l]++ and slot[i] = the row's arrival order
+// within its label (arbitrary; put back in row order by the sums); on a recorded pass
+// labels_all[rows[i]] = l (src/lib.rs:438-440); cand_count (optional) zeroed for the
+// next batch's search. Block 0: the batch objective (src/lib.rs:442-445), the sum of
+// distances in f64: a fixed-shape tree (deterministic, ~1e-16 relative from the
+// reference's sequential sum), or the sequential sum itself when the value feeds the
+// balance penalty; objective[epoch] += batch, mean_sqdist = batch / m; and the
+// crowded list emptied.
+__global__ void __launch_bounds__(1024) k_batch_tail(const uint32_t* __restrict__ labels,
+                                                     const uint32_t* __restrict__ rows, int m,
+                                                     uint32_t* __restrict__ counts, uint32_t* __restrict__ slot,
+                                                     uint32_t* __restrict__ labels_all,
+                                                     const int* __restrict__ record, uint32_t* __restrict__ cand_count,
+                                                     const float* __restrict__ dist, int sequential,
+                                                     double* __restrict__ objective, const int* __restrict__ epoch,
+                                                     double* __restrict__ mean_sqdist,
+                                                     uint32_t* __restrict__ crowded_count) {
+    if (blockIdx.x > 0) {
+        const int i = (blockIdx.x - 1) * 1024 + threadIdx.x;
+        if (i < m) {
+            const uint32_t l = labels[i];
+            slot[i] = atomicAdd(&counts[l], 1u);
+            if (*record) labels_all[rows[i]] = l;
+            if (cand_count) cand_count[i] = 0u;
+        }
+        return;
+    }
     __shared__ double part[1024];
     double s = 0.0;
     if (sequential) {
@@ -514,6 +714,7 @@ __global__ void __launch_bounds__(1024) k_batch_objective(const float* __restric
     if (threadIdx.x == 0) {
         objective[*epoch] += s;
         *mean_sqdist = s / (double)m;
+        *crowded_count = 0u;
     }
 }
 
@@ -689,20 +890,34 @@ EMB_DEV void revive_cta(int k, int d, float* __restrict__ c, float* __restrict__
     }
 }
 
+// The end of a step: the counter moves on, and what the next batch's search adds to
+// starts at zero: the certification bounds and (nctr of) the search counters.
+EMB_DEV void step_end(int now, int* __restrict__ step, Bounds* __restrict__ bounds, uint32_t* __restrict__ ctr,
+                      int nctr) {
+    *step = now + 1;
+    *bounds = Bounds{0.0f, 0.0f, 0.0f, 0.0f};
+    for (int i = 0; i < nctr; i++) ctr[i] = 0u;
+}
+__global__ void k_step_end(int* __restrict__ step, Bounds* __restrict__ bounds, uint32_t* __restrict__ ctr, int nctr) {
+    step_end(*step, step, bounds, ctr, nctr);
+}
+
+// Revival on every `every`-th step (src/lib.rs:463-465), and the step's end.
 __global__ void __launch_bounds__(1024) k_revive(int k, int d, float* __restrict__ c, float* __restrict__ usage,
                                                  float tau, const double* __restrict__ gstream,
                                                  unsigned long long* __restrict__ cursor, double* __restrict__ keys,
                                                  uint32_t* __restrict__ didx, uint32_t* __restrict__ unused,
                                                  unsigned long long* __restrict__ n_splits,
-                                                 unsigned long long capacity, const int* __restrict__ step,
-                                                 int every) {
+                                                 unsigned long long capacity, int* __restrict__ step, int every,
+                                                 Bounds* __restrict__ bounds, uint32_t* __restrict__ ctr, int nctr) {
     extern __shared__ double sort_keys[];
-    if ((*step + 1) % every != 0 || !(tau > 0.0f)) return;  // every 5th step (src/lib.rs:463-465)
+    const int now = *step;
+    __syncthreads();  // read by all before it moves on
+    if (threadIdx.x == 0) step_end(now, step, bounds, ctr, nctr);
+    if ((now + 1) % every != 0 || !(tau > 0.0f)) return;
     revive_cta(k, d, c, usage, tau, gstream, cursor, keys, didx, unused, n_splits, capacity, sort_keys,
                kReviveSmemSort);
 }
-
-__global__ void k_step_incr(int* step) { *step += 1; }
 
 // Closing mean (src/lib.rs:481-489): c_j = pass_sum_j * (1 / pass_count_j) when
 // the last pass assigned rows to j (f32), or the FP64 sums divided in f64.

@@ -303,3 +303,24 @@ def test_lockstep_graph_eager_streams_agree(emb, orc, tmp_path, monkeypatch):
     check_same(res[0][0], ref)
     lines = open(tmp_path / "tune.txt").read().split()
     assert lines[0].startswith("b_search:d=16:") and 0 <= int(lines[1]) < 11  # eleven search variants
+
+
+@pytest.mark.parametrize("n,d,k", [(3000, 4, 3), (9000, 36, 700), (12000, 132, 9), (30000, 16, 9000), (6000, 384, 50)])
+@pytest.mark.parametrize("closing_f64", [False, True])
+def test_update_kernels_cluster_sizes(emb, orc, n, d, k, closing_f64):
+    # Batches whose clusters have none, up to 32, up to 64 and hundreds of rows (the
+    # small and the crowded update), one to twelve warps a cluster, and label counts
+    # on both sides of the one-launch scan's limit; the last batch is short.
+    rng = np.random.default_rng(n + d)
+    centre = rng.standard_normal((max(4, k // 2), d), dtype=np.float32) * np.float32(6.0)
+    which = np.minimum(rng.geometric(0.05, n) - 1, centre.shape[0] - 1)
+    x = centre[which] + rng.standard_normal((n, d), dtype=np.float32)
+    cfg = dict(nepochs=2.3, batch_size=n // 3 + 7, closing_f64=closing_f64)
+    out, ref, _ = run_both(emb, orc, x, k, "bf16", **{k_: v for k_, v in cfg.items() if k_ != "closing_f64"})
+    check_same(out, ref)
+    if closing_f64:
+        a = emb.B200Assigner(0, precision="bf16")
+        f64 = emb.train(x, d, k, emb.Config(**cfg), assigner=a)
+        a.close()
+        assert np.array_equal(f64.labels, ref["labels"]) and f64.n_splits == ref["n_splits"]
+        np.testing.assert_allclose(f64.centroids, ref["centroids"], rtol=2e-5, atol=2e-5)
