@@ -398,11 +398,11 @@ EncodeTiledFn encode_tiled_fn() {
 
 // 2-D map over a k x kpad BF16 matrix (row stride kpad), boxes of 64 x 256
 // (one 128-byte swizzle atom wide); rows past k read as zeros.
-int encode_bf16_map(emb200_handle* h, CUtensorMap* map, void* base) {
+int encode_bf16_map(emb200_handle* h, CUtensorMap* map, void* base, size_t k, size_t kpad) {
     EncodeTiledFn fn = encode_tiled_fn();
     if (!fn) return fail(h, EMB200_ECUDA, "cuTensorMapEncodeTiled unavailable");
-    cuuint64_t dims[2] = {(cuuint64_t)h->kpad, (cuuint64_t)h->k};
-    cuuint64_t strides[1] = {(cuuint64_t)h->kpad * 2};
+    cuuint64_t dims[2] = {(cuuint64_t)kpad, (cuuint64_t)k};
+    cuuint64_t strides[1] = {(cuuint64_t)kpad * 2};
     cuuint32_t box[2] = {64, (cuuint32_t)kTcBN};
     cuuint32_t estr[2] = {1, 1};
     CUresult r = fn(map, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 2, base, dims, strides, box, estr,
@@ -428,9 +428,9 @@ int prepare_centroids(emb200_handle* h) {
             return fail(h, EMB200_ENOMEM, "BF16 centroid allocation failed");
         hi = h->c_hi.p;
         lo = h->c_lo.p;
-        int rc = encode_bf16_map(h, &h->map_hi, hi);
+        int rc = encode_bf16_map(h, &h->map_hi, hi, h->k, h->kpad);
         if (rc) return rc;
-        rc = encode_bf16_map(h, &h->map_lo, lo);
+        rc = encode_bf16_map(h, &h->map_lo, lo, h->k, h->kpad);
         if (rc) return rc;
         if (h->nrm16.ensure(kp * 16)) return fail(h, EMB200_ENOMEM, "BF16 norm allocation failed");
         h->maps_ok = true;
@@ -648,9 +648,9 @@ bool tc_supported(const emb200_handle* h, int nterms, bool fp8 = false) {
 // a run the waves never decrease with the count, so only the first count of each
 // run can be chosen: visiting those (O(sqrt(tiles)) of them) picks the same split
 // as trying every count from 1 to the number of tiles.
-int tc_nsplit(const emb200_handle* h, size_t m) {
+int tc_nsplit(const emb200_handle* h, size_t m, size_t k) {
     const long row_tiles = (long)((m + kTcBM - 1) / kTcBM);
-    const int ntiles = (int)((h->k + kTcBN - 1) / kTcBN);
+    const int ntiles = (int)((k + kTcBN - 1) / kTcBN);
     const long sms = std::max(1, h->sm_count);
     int best = 1;
     double best_cost = 0.0;
@@ -698,7 +698,8 @@ SimtPlan simt_plan(int sms, size_t m, size_t k) {
 }
 
 template <typename T, bool COLLECT, bool FP8, bool NM = false>
-int launch_tc_kernel(emb200_handle* h, const T* x, const TcParams& p, int nsplit, cudaStream_t st) {
+int launch_tc_kernel(emb200_handle* h, const T* x, const TcParams& p, int nsplit, cudaStream_t st,
+                     const CUtensorMap* hi = nullptr, const CUtensorMap* lo = nullptr) {
     const TcLayout L = tc_layout(p.kpad, p.nterms, FP8, NM);
     // At least 120 KB so that two CTAs never share an SM: each holds all 512 TMEM columns.
     const size_t smem = std::max<size_t>(L.total + 1024, 120 * 1024);
@@ -706,7 +707,8 @@ int launch_tc_kernel(emb200_handle* h, const T* x, const TcParams& p, int nsplit
     // Persistent: one CTA per SM, or one per work item when there are fewer.
     const size_t items = (p.m + (size_t)kTcBM - 1) / kTcBM * (size_t)nsplit;
     const unsigned grid = (unsigned)std::max<size_t>(1, std::min(items, (size_t)h->sm_count));
-    k_assign_tc<T, COLLECT, FP8, NM><<<grid, kTcPThreads, smem, st>>>(x, FP8 ? h->map_f8 : h->map_hi, h->map_lo, p);
+    k_assign_tc<T, COLLECT, FP8, NM><<<grid, kTcPThreads, smem, st>>>(
+        x, FP8 ? h->map_f8 : hi ? *hi : h->map_hi, lo ? *lo : h->map_lo, p);
     CKL();
     return EMB200_OK;
 }
@@ -739,7 +741,7 @@ int launch_tc(emb200_handle* h, const T* x, const uint32_t* gather, const uint32
         p.stall_tile = h->stall_tile;
         p.stall_ns = h->stall_ns;
     }
-    const int nsplit = nsplit_override > 0 ? nsplit_override : tc_nsplit(h, m);
+    const int nsplit = nsplit_override > 0 ? nsplit_override : tc_nsplit(h, m, h->k);
     p.nsplit = nsplit;
     if constexpr (!COLLECT && std::is_same<T, float>::value) {
         if (fp8) return launch_tc_kernel<T, false, true>(h, x, p, nsplit, st);
@@ -840,7 +842,7 @@ int assign_rows_dev(emb200_handle* h, const T* x, const uint32_t* gather, size_t
     const int fast_terms = tc_terms(prec, dtype);
     const bool tc = prec != EMB200_PREC_FP32 && (fp8 || tc_supported(h, fast_terms));
     const SimtPlan plan = simt_plan(h->sm_count, m, h->k);
-    const int nsplit = tc ? tc_nsplit(h, m) : plan.nsplit;
+    const int nsplit = tc ? tc_nsplit(h, m, h->k) : plan.nsplit;
     // Inside the training loop (graph = true) nothing may allocate while an epoch is
     // captured, and a smaller batch can need more split partials than a full one
     // (fewer row tiles, more splits): size them for every batch of up to m rows.
@@ -851,7 +853,7 @@ int assign_rows_dev(emb200_handle* h, const T* x, const uint32_t* gather, size_t
     } else if (graph) {
         for (size_t rt = 1; rt * kTcBM < m + kTcBM; rt++) {
             const size_t mm = std::min(rt * kTcBM, m);
-            const int ns = tc ? tc_nsplit(h, mm) : simt_plan(h->sm_count, mm, h->k).nsplit;
+            const int ns = tc ? tc_nsplit(h, mm, h->k) : simt_plan(h->sm_count, mm, h->k).nsplit;
             part_rows = std::max(part_rows, (size_t)ns * mm);
         }
         h->part_size_m = m;

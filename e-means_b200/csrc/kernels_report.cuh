@@ -12,13 +12,15 @@
 //    median and MAD and the medians over clusters;
 //  * k_rep_pairs: the exact O(k^2 d) pair pass in the reference's sqdist
 //    rounding (src/report.rs:104-114), as a nearest-other-centroid search or as
-//    the adjacency bitset of the families' radius test;
+//    the adjacency bitset of the families' radius test; from 2048 centroids on the
+//    tensor-core search finds the few pairs that need that rounding (k_pair_exact);
 //  * k_rep_families: the greedy family pass (src/report.rs:198-216) in one CTA.
 #pragma once
 #include <cfloat>
 #include <cstdint>
 
 #include "common.cuh"
+#include "kernels_exact.cuh"
 
 namespace emb {
 
@@ -597,6 +599,166 @@ __global__ void __launch_bounds__(kPairThreads, 2) k_rep_pairs(const float* __re
         }
     }
     asm volatile("cp.async.wait_group 0;\n" ::: "memory");
+}
+
+// ---- pair pass on the tensor cores ---------------------------------------------
+//
+// The pair pass above spends 3 FP32 operations on each of the k^2 d / 2 terms to
+// keep the reference's rounding, although a row needs it for a few partners only.
+// Here the three-term BF16 search (k_assign_tc) scores every pair approximately,
+// collects per row each partner that the bound below cannot rule out, and only those
+// are evaluated in the reference's rounding (k_pair_exact); a row whose list overflows,
+// or holds no partner, is scanned exactly (k_pair_scan). k = 16384, d = 128: 3.43 +
+// 3.26 ms for the two passes, 0.33 + 0.82 ms here (the second keeps about 50
+// partners a row).
+//
+// Bound. With s(j) the reference's squared distance of i and j, S(j) the exact one and
+// a(j) = |c_j|^2 - 2 c_i . c_j approximated: a(j) is within E1 = ka |c_i| cmax + kb nmax
+// of norm_j - 2 dot (bound_coefficients), norm_j within (d / 16 + 20) u |c_j|^2 of
+// |c_j|^2, and s(j) within (d / 16 + 36) u S(j), S(j) <= 4 cmax^2 (u = 2^-24). For
+// d <= 256 the last two are below 2^-16 cmax^2 together: E = E1 + 2^-15 cmax^2 bounds
+// |a(j) + |c_i|^2 - s(j)|.
+//  * nearest: with v the second smallest a of the row (its own column is one of the two
+//    smallest or the smallest is a partner nearer than it), the nearest partner has
+//    a <= v + 2 E.
+//  * radius r: s(j) <= r^2 (1 + 2^-20) is necessary for sqrt(s(j)) <= r, so
+//    a(j) <= r^2 (1 + 2^-20) - |c_i|^2 + E.
+
+constexpr int kPairNearCap = 32;   // partners kept per row
+constexpr int kPairAdjCap = 256;
+
+// Scoring norms: the dead clusters' never pass a threshold.
+__global__ void k_pair_mask(const float* __restrict__ norms, const uint32_t* __restrict__ start, uint32_t k,
+                            float* __restrict__ masked, uint32_t kp) {
+    const uint32_t j = blockIdx.x * blockDim.x + threadIdx.x;
+    if (j < kp) masked[j] = j < k && start[j + 1] > start[j] ? norms[j] : kPadNorm;
+}
+
+EMB_DEV float pair_bound(float norm, const Bounds& b, float ka, float kb) {
+    const float xn = __fmul_ru(__fsqrt_ru(fmaxf(norm, 0.0f)), 1.00001f);
+    const float e = __fadd_ru(__fmul_ru(__fmul_ru(ka, xn), b.cmax), __fmul_ru(kb, b.nmax));
+    return __fadd_ru(e, __fmul_ru(0x1p-15f, __fmul_ru(b.cmax, b.cmax)));
+}
+
+// Collection thresholds (NaN: none) from the rows' two smallest scores.
+__global__ void k_pair_theta_near(const float* __restrict__ part_s, int nsplit, uint32_t k,
+                                  const float* __restrict__ norms, const Bounds* __restrict__ bounds, float ka, float kb,
+                                  float* __restrict__ theta) {
+    const uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
+    if (i >= k) return;
+    float m1 = INFINITY, m2 = INFINITY;
+    for (int s = 0; s < nsplit; s++)
+        for (int e = 0; e < 2; e++) {
+            const float v = part_s[((size_t)s * k + i) * 2 + e];
+            m2 = fminf(m2, fmaxf(m1, v));
+            m1 = fminf(m1, v);
+        }
+    const float E = pair_bound(norms[i], *bounds, ka, kb);
+    const float t = __fadd_ru(__fadd_ru(m2, __fmul_ru(2.0f, E)), __fmul_ru(0x1p-17f, fabsf(m2)));
+    theta[i] = isfinite(t) && m2 < 1e38f ? t : __int_as_float(0x7fc00000);
+}
+
+__global__ void k_pair_theta_adj(const uint32_t* __restrict__ start, uint32_t k, const float* __restrict__ norms,
+                                 const Bounds* __restrict__ bounds, const RepScalars* __restrict__ sc, float ka, float kb,
+                                 float* __restrict__ theta) {
+    const uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
+    if (i >= k) return;
+    const float r2 = __fmul_ru(__fmul_ru(sc->radius, sc->radius), 1.0f + 0x1p-20f);
+    const float E = pair_bound(norms[i], *bounds, ka, kb);
+    const float t = __fadd_ru(__fadd_ru(__fsub_ru(r2, norms[i]), E), __fmul_ru(0x1p-18f, r2));
+    theta[i] = start[i + 1] > start[i] && isfinite(t) ? t : __int_as_float(0x7fc00000);
+}
+
+// The reference's squared distance (as k_rep_pairs) by 16 lanes of a half-warp; both
+// halves must call it. Every lane of a half returns its value.
+EMB_DEV float half_sqdist_ref(const float* __restrict__ x, const float* __restrict__ y, uint32_t d, int lane) {
+    const uint32_t d16 = d / 16 * 16;
+    float acc = 0.0f;
+    for (uint32_t t = lane & 15; t < d16; t += 16) {
+        const float u = __fsub_rn(x[t], y[t]);
+        acc = __fadd_rn(acc, __fmul_rn(u, u));
+    }
+    float s = __shfl_sync(0xffffffffu, acc, lane & 16);
+#pragma unroll
+    for (int l = 1; l < 16; l++) s = __fadd_rn(s, __shfl_sync(0xffffffffu, acc, (lane & 16) + l));
+    float tail = 0.0f;
+    for (uint32_t t = d16; t < d; t++) {
+        const float u = __fsub_rn(x[t], y[t]);
+        tail = __fadd_rn(tail, __fmul_rn(u, u));
+    }
+    return __fadd_rn(s, tail);
+}
+
+// The collected partners of one row (a warp each, two at a time) in the reference's
+// rounding. Nearest: near_key[i] = min of (bits of s, j). ADJ: the row's adjacency
+// bits (zero before). Rows that the lists do not settle go to `rest`.
+template <bool ADJ>
+__global__ void __launch_bounds__(256) k_pair_exact(const float* __restrict__ c, uint32_t k, uint32_t d,
+                                                    const uint32_t* __restrict__ start,
+                                                    const uint32_t* __restrict__ cand,
+                                                    const uint32_t* __restrict__ cand_count, uint32_t cap,
+                                                    const int* __restrict__ err, unsigned long long* __restrict__ near_key,
+                                                    const RepScalars* __restrict__ sc, uint32_t* __restrict__ adj,
+                                                    uint32_t words, uint32_t* __restrict__ rest,
+                                                    uint32_t* __restrict__ rest_count) {
+    const uint32_t i = (blockIdx.x * blockDim.x + threadIdx.x) >> 5;
+    const int lane = threadIdx.x & 31;
+    if (i >= k) return;
+    if (ADJ && start[i + 1] == start[i]) return;  // dead: no neighbours
+    const uint32_t cnt = cand_count[i];
+    unsigned long long best = ~0ull;
+    const bool listed = cnt > 0 && cnt <= cap && !*err;
+    if (listed) {
+        const float* ci = c + (size_t)i * d;
+        for (uint32_t e = 0; e < cnt; e += 2) {
+            const uint32_t q = e + (lane >> 4);
+            const uint32_t j = cand[(size_t)i * cap + (q < cnt ? q : e)];
+            const float s = half_sqdist_ref(ci, c + (size_t)j * d, d, lane);
+            const bool partner = q < cnt && j != i && start[j + 1] > start[j];
+            if (ADJ) {
+                if (partner && (lane & 15) == 0 && __fsqrt_rn(s) <= sc->radius)
+                    atomicOr(&adj[(size_t)i * words + (j >> 5)], 1u << (j & 31));
+            } else if (partner && s < INFINITY) {
+                best = min(best, ((unsigned long long)__float_as_uint(s) << 32) | j);
+            }
+        }
+    }
+    if (!ADJ) best = min(best, __shfl_xor_sync(0xffffffffu, best, 16));
+    if (lane == 0) {
+        if (!ADJ && best != ~0ull) near_key[i] = best;
+        if (!listed || (!ADJ && best == ~0ull)) rest[atomicAdd(rest_count, 1u)] = i;
+    }
+}
+
+// The rows of `rest` against every live partner, a CTA per row.
+template <bool ADJ>
+__global__ void __launch_bounds__(256) k_pair_scan(const float* __restrict__ c, uint32_t k, uint32_t d,
+                                                   const uint32_t* __restrict__ start,
+                                                   unsigned long long* __restrict__ near_key,
+                                                   const RepScalars* __restrict__ sc, uint32_t* __restrict__ adj,
+                                                   uint32_t words, const uint32_t* __restrict__ rest,
+                                                   const uint32_t* __restrict__ rest_count) {
+    const int lane = threadIdx.x & 31, half = threadIdx.x >> 4;
+    for (uint32_t r = blockIdx.x; r < *rest_count; r += gridDim.x) {
+        const uint32_t i = rest[r];
+        const float* ci = c + (size_t)i * d;
+        unsigned long long best = ~0ull;
+        for (uint32_t j0 = 0; j0 < k; j0 += 16) {
+            const uint32_t j = j0 + half, jc = j < k ? j : k - 1;
+            const float s = half_sqdist_ref(ci, c + (size_t)jc * d, d, lane);
+            if (j >= k || j == i || start[j + 1] == start[j]) continue;  // no shuffles follow in this round
+            if (ADJ) {
+                if ((lane & 15) == 0 && __fsqrt_rn(s) <= sc->radius)
+                    atomicOr(&adj[(size_t)i * words + (j >> 5)], 1u << (j & 31));
+            } else if (s < INFINITY) {
+                best = min(best, ((unsigned long long)__float_as_uint(s) << 32) | j);
+            }
+        }
+        if (!ADJ) {
+            best = min(best, __shfl_xor_sync(0xffffffffu, best, 16));
+            if (lane == 0 && best != ~0ull) atomicMin(&near_key[i], best);
+        }
+    }
 }
 
 // near_key -> (nearest centroid, squared distance), or (i, inf) without one.

@@ -169,3 +169,29 @@ def test_report_argument_errors(emb):
     with pytest.raises(emb.EngineError, match="assign_resident"):
         emb.report_resident(a)
     a.close()
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("case", ["spread", "duplicates", "wide_radius", "far_from_origin", "nonfinite", "few_live"])
+@pytest.mark.parametrize("k,d", [(2048, 16), (2303, 37), (4100, 100), (2600, 200)])
+def test_report_pair_search_matches_oracle(emb, orc, case, k, d):
+    # Enough clusters for the tensor-core pair search: partners it collects, lists that
+    # overflow (more than 32 coincident centroids, a radius over everything), rows it
+    # cannot score, dead clusters nearer than any live one.
+    labels, sq, c = _synthetic(6 * k, k, d, seed=k + d, empty=0.2)
+    cfg = emb.ReportConfig(family_pass=2)
+    if case == "duplicates":
+        c[100:180] = c[100]
+        c[np.unique(labels)[:40]] = c[7]
+    elif case == "wide_radius":
+        cfg = emb.ReportConfig(family_radius=6.0, family_pass=2)
+    elif case == "far_from_origin":  # differences small beside the norms: many partners within the bound
+        c = (c * np.float32(0.01) + np.float32(3.0)).astype(np.float32)
+    elif case == "nonfinite":
+        c[5, 0] = np.inf
+        c[int(labels[0]), d - 1] = np.nan
+        c[17] = 3e38
+    elif case == "few_live":
+        live = np.unique(labels)[:3]
+        labels = live[labels % 3].astype(np.uint32)
+    _assert_same(emb.report(labels, sq, c, d, cfg), _oracle_report(emb, orc, labels, sq, c, cfg))
