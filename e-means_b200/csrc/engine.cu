@@ -189,11 +189,12 @@ struct emb200_handle {
     size_t kpad = 0;
     CUtensorMap map_hi{}, map_lo{};  // TMA descriptors of c_hi / c_lo (128B swizzle, 64 x 128 boxes)
     bool maps_ok = false;
-    // Half-norms split into BF16 parts for the single-term search that sums the
-    // norms inside the contraction ([whole tiles][16], nrm16_row); nrm16_ok: they
-    // match the norms (a bias changes those)
-    DevBuf<__nv_bfloat16> nrm16;
-    bool nrm16_ok = false;
+    // Operands of the single-term search of f32 rows (k_prep_f16): scaled FP16 centroids
+    // and the half-norms it sums inside the contraction; f16_ok: they match the
+    // centroids and norms (a bias changes those)
+    DevBuf<__half> c_f16, nrm16;
+    CUtensorMap map_f16{};
+    bool f16_ok = false;
     // A training loop is running whose step end zeroes the certification bounds, the
     // search counters and the candidate counts for the next step.
     bool steady = false;
@@ -321,15 +322,14 @@ size_t elt_size(int dtype) { return dtype == EMB200_F32 ? 4 : 1; }
 // significant bits, round to nearest); the
 // tensor-core accumulation is allowed one f32 truncation (2u) per product term.
 //
-// The single-term BF16 search of f32 rows (norm_mma) sums the half-norm's three
-// BF16 parts in the same tensor-core accumulation as the d products: three more
+// The single-term search of f32 rows (norm_mma) sums the half-norm's three parts in the same tensor-core accumulation as the d products: three more
 // truncated terms, whose magnitudes add |norm| / 2 to the sum they are relative to,
 // so the score (twice the accumulator) gains gamma(d + 5, 2u) |norm|.
 //
-// kr (single-term BF16, when the caller asks for it): the operands' rounding is
-// bounded per row instead, by kr (xr cmax + (|x| + xr) dmax) with xr = |x - bf16(x)|
-// of the row and dmax >= max_j |c_j - bf16(c_j)| (exact identity plus Cauchy-Schwarz,
-// in score units), and leaves ka.
+// kr (the same search, when the caller asks for it): the operands' rounding is bounded
+// per row instead, by kr (xr cmax + (|x| + xr) dmax) with xr = |x - x^| of the row and
+// dmax >= max_j |c_j - c^_j| (exact identity plus Cauchy-Schwarz, in score units), and
+// leaves ka.
 void bound_coefficients(int precision, int dtype, size_t d, bool packed, float* ka, float* kb, bool norm_mma = false,
                         float* kr = nullptr) {
     if (kr) *kr = 0.0f;
@@ -432,13 +432,19 @@ int prepare_centroids(emb200_handle* h) {
         if (rc) return rc;
         rc = encode_bf16_map(h, &h->map_lo, lo, h->k, h->kpad);
         if (rc) return rc;
-        if (h->nrm16.ensure(kp * 16)) return fail(h, EMB200_ENOMEM, "BF16 norm allocation failed");
+        if (h->opts.precision == EMB200_PREC_BF16X1 || h->opts.precision == EMB200_PREC_FP8) {
+            // (FP8 takes this search where its own operands do not fit.) Allocated here, outside any captured epoch; filled before the first search.
+            if (h->nrm16.ensure(kp * 16) || h->c_f16.ensure((size_t)k * h->kpad))
+                return fail(h, EMB200_ENOMEM, "FP16 centroid allocation failed");
+            rc = encode_bf16_map(h, &h->map_f16, h->c_f16.p, h->k, h->kpad);
+            if (rc) return rc;
+        }
         h->maps_ok = true;
     }
     k_prep_centroids<<<(unsigned)((kp + 7) / 8), 256, 0, st>>>(h->c.p, k, (int)kp, d, h->norms.p, h->bounds.p, hi, lo,
-                                                               (int)h->kpad, hi ? h->nrm16.p : nullptr);
+                                                               (int)h->kpad);
     CKL();
-    h->nrm16_ok = hi != nullptr;
+    h->f16_ok = false;
     h->f8_ok = false;
     if (h->opts.precision == EMB200_PREC_FP8 && h->d <= 256) {
         // e4m3 codes in rows of one or two 128-byte swizzle atoms; scoring norms are
@@ -507,7 +513,7 @@ int apply_bias(emb200_handle* h, const float* bias_dev) {
     const int k = (int)h->k;
     k_add_bias<<<(unsigned)((k + 255) / 256), 256, 0, st>>>(h->norms.p, bias_dev, k, h->bounds.p);
     CKL();
-    h->nrm16_ok = false;
+    h->f16_ok = false;
     if (h->f8_ok) {
         k_add_bias_f8<<<(unsigned)((k + 255) / 256), 256, 0, st>>>(h->nf8.p, bias_dev, k);
         CKL();
@@ -745,20 +751,23 @@ int launch_tc(emb200_handle* h, const T* x, const uint32_t* gather, const uint32
     p.nsplit = nsplit;
     if constexpr (!COLLECT && std::is_same<T, float>::value) {
         if (fp8) return launch_tc_kernel<T, false, true>(h, x, p, nsplit, st);
-        // Single-term BF16 search of f32 rows: norms summed inside the contraction
-        // (the certification bound allows for it whenever this mode is searched).
+        // Single-term search of f32 rows: FP16 operands, norms summed inside the
+        // contraction (the certification bound allows for both whenever this mode is
+        // searched).
         const size_t kp = (h->k + kTcBN - 1) / kTcBN * kTcBN;
-        if (nterms == 1 && h->nrm16.n >= kp * 16) {
-            if (!h->nrm16_ok) {
-                k_prep_nrm16<<<(unsigned)((kp + 255) / 256), 256, 0, st>>>(h->norms.p, (int)kp, h->nrm16.p);
+        if (nterms == 1) {
+            if (!h->f16_ok) {
+                k_prep_f16<<<(unsigned)((kp + 7) / 8), 256, 0, st>>>(h->c.p, (int)h->k, (int)kp, (int)h->d,
+                                                                     (int)h->kpad, h->norms.p, h->bounds.p, h->c_f16.p,
+                                                                     h->nrm16.p);
                 CKL();
-                h->nrm16_ok = true;
+                h->f16_ok = true;
             }
             p.nrm16 = h->nrm16.p;
+            p.bounds = h->bounds.p;
             if (fuse && nsplit == 1) {  // certification at the end of each item
                 p.fuse = 1;
                 p.cx = fuse->cx;
-                p.bounds = fuse->bounds;
                 p.ka = fuse->ka;
                 p.kb = fuse->kb;
                 p.kr = fuse->kr;
@@ -772,7 +781,7 @@ int launch_tc(emb200_handle* h, const T* x, const uint32_t* gather, const uint32
                 p.cert_count = fuse->cert_count;
                 if (fused) *fused = true;
             }
-            return launch_tc_kernel<T, false, false, true>(h, x, p, nsplit, st);
+            return launch_tc_kernel<T, false, false, true>(h, x, p, nsplit, st, &h->map_f16);
         }
     }
     return launch_tc_kernel<T, COLLECT, false>(h, x, p, nsplit, st);
@@ -1201,6 +1210,7 @@ int emb200_destroy(emb200_handle* h) {
     cudaSetDevice(h->device);
     if (h->stream) cudaStreamSynchronize(h->stream);
     h->c.release(); h->norms.release(); h->bias.release(); h->bounds.release(); h->nrm16.release();
+    h->c_f16.release();
     h->c_hi.release(); h->c_lo.release(); h->c8.release(); h->c16.release(); h->off8.release();
     h->rows.release(); h->res_labels.release(); h->res_dist.release();
     h->stage.release(); h->st_labels.release(); h->st_dist.release();
@@ -1574,7 +1584,7 @@ extern "C" int emb200_assign_f32_noalloc(const float* x_dev, size_t m, size_t d,
     if (cudaMemsetAsync(p, 0, 512, st) != cudaSuccess) return EMB200_ECUDA;  // bounds and counters start at zero
     // Norms and the certification bounds (no BF16 split: the search here is FP32).
     k_prep_centroids<<<(unsigned)((k + 7) / 8), 256, 0, st>>>(centroids_dev, (int)k, (int)k, (int)d, norms, bounds,
-                                                              nullptr, nullptr, (int)((d + 63) / 64 * 64), nullptr);
+                                                              nullptr, nullptr, (int)((d + 63) / 64 * 64));
     const int vec4 = (d % 4 == 0 && ((uintptr_t)x_dev & 15) == 0 && ((uintptr_t)centroids_dev & 15) == 0) ? 1 : 0;
     // Set on every call: the attribute belongs to the current context (see noalloc_scratch).
     const void* search = plan.small ? (const void*)k_assign_simt<float, 1, 1> : (const void*)k_assign_simt<float, 2, 4>;

@@ -2,6 +2,7 @@
 // exact re-search, all in the reference CpuAssigner's own f32 rounding.
 #pragma once
 #include <cuda_bf16.h>
+#include <cuda_fp16.h>
 #include "common.cuh"
 
 namespace emb {
@@ -13,12 +14,36 @@ struct Bounds {
     float cmax;  // >= max_j |c_j| (upper-rounded)
     float nmax;  // >= max_j |norms_j| (norms include the bias)
     float cmax_hi;  // >= max_j |bf16(c_j)| (three-term split bound)
-    float dmax;     // >= max_j |c_j - bf16(c_j)| (single-term residual bound)
+    float dmax;     // >= max_j |c_j - c^_j| of the single-term search's operands (k_prep_f16)
+    float s16;      // their power-of-two scale
 };
 
-// Upper bound of |v - bf16(v)|^2 summed into acc (v - bf16(v) is exact in f32).
-EMB_DEV float bf16_resid_sq(float v, float acc) {
-    const float r = v - __bfloat162float(__float2bfloat16_rn(v));
+// ---- operands of the single-term search (f32 rows) ------------------------------
+//
+// FP16 values of the rows and centroids scaled by one power of two S, which puts the
+// largest centroid norm at 64 .. 128 and the scaled half-norms at 2^14 at most. Eleven
+// significant bits where BF16 has eight, at the same MMA rate: the operands' rounding,
+// nearly all of the certification bound, is eight times smaller, so rows that need the
+// three-term refine pass are rare (1M x 128 embeddings, k = 16384: the refine pass
+// 675 -> 106 us; k = 65536, heavy-tailed: 4.4 -> 0.7 ms). FP16's
+// narrow range costs values far below the largest one some of those bits, which only
+// enters through the residuals |x - x^| and |c - c^| that the bound is made of;
+// anything out of range (a row hundreds of times the centroids) has an infinite
+// residual and is refined.
+EMB_DEV float f16_scale(const Bounds& b) {
+    if (!(b.cmax > 0.0f) || !isfinite(b.cmax) || !isfinite(b.nmax)) return 1.0f;
+    int e = 6 - ((int)(__float_as_uint(b.cmax) >> 23) - 127);
+    const int en = (int)(__float_as_uint(b.nmax) >> 23) - 127;
+    if (b.nmax > 0.0f) e = min(e, (14 - en) >> 1);
+    return __uint_as_float((uint32_t)(max(-60, min(60, e)) + 127) << 23);
+}
+
+// |x - x^| from the sum of the scaled squares, rounded up.
+EMB_DEV float f16_resid(float sum, float S) { return __fmul_ru(__fmul_ru(__fsqrt_ru(sum), 1.0000005f), 1.0f / S); }
+
+// Upper bound of |v - half(v)|^2 summed into acc (v - half(v) is exact in f32).
+EMB_DEV float f16_resid_sq(float v, float acc) {
+    const float r = v - __half2float(__float2half_rn(v));
     return __fmaf_ru(r, r, acc);
 }
 
@@ -93,39 +118,17 @@ EMB_DEV float group_dot_ref(int match, const T* x, const float* cg, int d, int l
     }
 }
 
-// Norms inside the contraction (single-term BF16 search): row j of `out` (16 BF16)
-// holds the three BF16 parts of h = norms[j] / 2 (p1 = bf16(h), p2 = bf16(h - p1), p3 = bf16(h - p1 - p2);
-// both differences are exact in f32 and p3 is exact in BF16, so p1 + p2 + p3 = h
-// for every h in the normal range), then zeros. A non-finite h keeps p1 = h and
-// zeros after it, so the MMA sums the same +-inf or NaN the epilogue's
-// norm - 2 acc would give.
-EMB_DEV void nrm16_row(float norm, __nv_bfloat16* __restrict__ out) {
-    const float h = 0.5f * norm;
-    const __nv_bfloat16 p1 = __float2bfloat16_rn(h);
-    __nv_bfloat16 p2 = __float2bfloat16_rn(0.0f), p3 = p2;
-    if (isfinite(h)) {
-        const float r1 = h - __bfloat162float(p1);
-        p2 = __float2bfloat16_rn(r1);
-        p3 = __float2bfloat16_rn(r1 - __bfloat162float(p2));
-    }
-    uint4* o = reinterpret_cast<uint4*>(out);
-    o[0] = make_uint4((uint32_t)__bfloat16_as_ushort(p1) | ((uint32_t)__bfloat16_as_ushort(p2) << 16),
-                      (uint32_t)__bfloat16_as_ushort(p3), 0u, 0u);
-    o[1] = make_uint4(0u, 0u, 0u, 0u);
-}
-
 constexpr float kPadNorm = 3.0e38f;  // norms of the padding: never a candidate, and finite, so that keys stay numbers
 
 // set_centroids (src/cpu.rs:84-93): norms_j = sqnorm_ref(c_j), kPadNorm up to kp;
 // bounds for the certification (max-ed into *bounds, which starts at zero);
 // optionally the BF16 hi/lo split (hi = bf16(c), lo = bf16(c - hi)) with row stride
-// kpad, and the half-norms of nrm16_row. One warp per centroid; a block's maxima are
-// joined before the four atomics: one per centroid on the same addresses was most of
-// the kernel's 13 us at 4096 x 128 (now 3.4).
+// kpad. One warp per centroid; a block's maxima are joined before the atomics: one per
+// centroid on the same addresses was most of the kernel's 13 us at 4096 x 128 (now 3.4).
 __global__ void __launch_bounds__(256) k_prep_centroids(const float* __restrict__ c, int k, int kp, int d,
                                                         float* __restrict__ norms, Bounds* __restrict__ bounds,
                                                         __nv_bfloat16* __restrict__ hi, __nv_bfloat16* __restrict__ lo,
-                                                        int kpad, __nv_bfloat16* __restrict__ nrm16) {
+                                                        int kpad) {
     __shared__ float4 part[8];
     const int w = threadIdx.x >> 5, lane = threadIdx.x & 31;
     const int j = (int)blockIdx.x * 8 + w;
@@ -133,11 +136,10 @@ __global__ void __launch_bounds__(256) k_prep_centroids(const float* __restrict_
     if (j < k) {
         const float* cj = c + (size_t)j * d;
         const float nrm = warp_sqnorm_ref(cj, d, lane);
-        float ss = 0.0f, ssh = 0.0f, ssd = 0.0f;
+        float ss = 0.0f, ssh = 0.0f;
         for (int i = lane; i < kpad; i += 32) {
             const float v = i < d ? cj[i] : 0.0f;
             ss = __fmaf_ru(v, v, ss);
-            ssd = bf16_resid_sq(v, ssd);
             if (hi) {
                 const __nv_bfloat16 h = __float2bfloat16_rn(v);
                 const float hf = __bfloat162float(h);
@@ -149,26 +151,79 @@ __global__ void __launch_bounds__(256) k_prep_centroids(const float* __restrict_
         for (int o = 16; o; o >>= 1) {
             ss = __fadd_ru(ss, __shfl_xor_sync(kFull, ss, o));
             ssh = __fadd_ru(ssh, __shfl_xor_sync(kFull, ssh, o));
-            ssd = __fadd_ru(ssd, __shfl_xor_sync(kFull, ssd, o));
         }
-        if (lane == 0) {
-            norms[j] = nrm;
-            if (nrm16) nrm16_row(nrm, nrm16 + (size_t)j * 16);
-        }
+        if (lane == 0) norms[j] = nrm;
         mx = make_float4(__fmul_ru(__fsqrt_ru(ss), 1.0000005f), fabsf(nrm), __fmul_ru(__fsqrt_ru(ssh), 1.0000005f),
-                         __fmul_ru(__fsqrt_ru(ssd), 1.0000005f));
+                         0.0f);
     } else if (j < kp && lane == 0) {
         norms[j] = kPadNorm;
-        if (nrm16) nrm16_row(kPadNorm, nrm16 + (size_t)j * 16);
     }
     if (lane == 0) part[w] = mx;
     __syncthreads();
-    if (threadIdx.x < 4) {
+    if (threadIdx.x < 3) {
         // The maxima as bit patterns: the values are non-negative or NaN, and a NaN's
         // pattern is above every number's, as in atomic_max_pos.
         uint32_t m = 0;
         for (int q = 0; q < 8; q++) m = max(m, __float_as_uint(reinterpret_cast<const float*>(&part[q])[threadIdx.x]));
         if (m) atomicMax(reinterpret_cast<unsigned int*>(bounds) + threadIdx.x, m);
+    }
+}
+
+// The single-term search's centroid operands, from the norms (bias included) and bounds:
+// c16 [k][kpad] = half(S c), zeros past d, its residual into bounds->dmax, S into
+// bounds->s16; nrm16 [kp][16]: the norms inside the contraction. Row j holds the three
+// FP16 parts of h = S^2 norms[j] / 2 / kNrm16One (p1 = half(h), p2 = half(h - p1),
+// p3 = half(h - p1 - p2); the differences are exact in f32), then zeros: p1 + p2 + p3 is
+// within 2^-25 of h, so the score's norm within 2^-24 cmax^2 (a constant the bound
+// carries; S cmax >= 64, or the half-norms reach 2^12). A non-finite norm keeps its value in p1, so the
+// MMA sums the same inf or NaN the epilogue's norm - 2 acc would give. The padding up
+// to kp is the largest finite value: never a candidate. One warp per centroid.
+constexpr float kNrm16One = 1024.0f;  // the constant row operand against the parts
+__global__ void __launch_bounds__(256) k_prep_f16(const float* __restrict__ c, int k, int kp, int d, int kpad,
+                                                  const float* __restrict__ norms, Bounds* __restrict__ bounds,
+                                                  __half* __restrict__ c16, __half* __restrict__ nrm16) {
+    __shared__ float part[8];
+    const int w = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    const int j = (int)blockIdx.x * 8 + w;
+    const float S = f16_scale(*bounds);
+    float dm = 0.0f;
+    if (j < k) {
+        const float* cj = c + (size_t)j * d;
+        float ssd = 0.0f;
+        for (int i = 2 * lane; i < kpad; i += 64) {
+            const float a = i < d ? S * cj[i] : 0.0f, b = i + 1 < d ? S * cj[i + 1] : 0.0f;
+            ssd = f16_resid_sq(b, f16_resid_sq(a, ssd));
+            *reinterpret_cast<__half2*>(c16 + (size_t)j * kpad + i) = __floats2half2_rn(a, b);
+        }
+        for (int o = 16; o; o >>= 1) ssd = __fadd_ru(ssd, __shfl_xor_sync(kFull, ssd, o));
+        dm = __fmul_ru(__fmul_ru(__fsqrt_ru(ssd), 1.0000005f), 1.0f / S);
+    }
+    if (lane == 0 && j < kp) {
+        __half p1 = __float2half_rn(65504.0f), p2 = p1, p3 = p1;
+        if (j < k) {
+            const float h = norms[j] * (0.5f * S * S / kNrm16One);
+            if (!(fabsf(h) > 65504.0f) || !isfinite(h)) {
+                p1 = __float2half_rn(h);
+                p2 = p3 = __float2half_rn(0.0f);
+                if (isfinite(h)) {
+                    const float r1 = h - __half2float(p1);
+                    p2 = __float2half_rn(r1);
+                    p3 = __float2half_rn(r1 - __half2float(p2));
+                }
+            }
+        }
+        uint4* o = reinterpret_cast<uint4*>(nrm16 + (size_t)j * 16);
+        o[0] = make_uint4((uint32_t)__half_as_ushort(p1) | ((uint32_t)__half_as_ushort(p2) << 16),
+                          (uint32_t)__half_as_ushort(p3), 0u, 0u);
+        o[1] = make_uint4(0u, 0u, 0u, 0u);
+    }
+    if (lane == 0) part[w] = dm;
+    __syncthreads();
+    if (threadIdx.x == 0) {
+        uint32_t m = 0;
+        for (int q = 0; q < 8; q++) m = max(m, __float_as_uint(part[q]));
+        if (m) atomicMax(reinterpret_cast<unsigned int*>(&bounds->dmax), m);
+        if (blockIdx.x == 0) bounds->s16 = S;
     }
 }
 
@@ -211,10 +266,12 @@ EMB_DEV bool certify_decide(int row, const Top2& t, uint32_t j1, uint32_t j2, fl
         const float cm = row_bounds ? row_bounds[row].x : bounds->cmax;
         float E = __fadd_ru(__fmul_ru(__fmul_ru(ka, xnorm), cm),
                             __fmul_ru(kb, row_bounds ? row_bounds[row].y : bounds->nmax));
-        // Single-term BF16: x.c - bf16(x).bf16(c) = (x - bf16(x)).c + bf16(x).(c - bf16(c)),
-        // at most xr cmax + (|x| + xr) dmax, with xr = |x - bf16(x)| of this row.
-        if (kr > 0.0f)
+        // Single-term search: x.c - x^.c^ = (x - x^).c + x^.(c - c^), at most xr cmax +
+        // (|x| + xr) dmax, with xr = |x - x^| of this row; and the norms' FP16 parts.
+        if (kr > 0.0f) {
             E = __fadd_ru(E, __fmul_ru(kr, __fadd_ru(__fmul_ru(xr, cm), __fmul_ru(__fadd_ru(xnorm, xr), bounds->dmax))));
+            E = __fadd_ru(E, __fmul_ru(0x1p-24f, __fmul_ru(cm, cm)));
+        }
         const float thr = __fsub_rd(t.s2, E);
         ok = isfinite(E) && sb < thr;  // NaN-safe: any NaN fails
     }
@@ -278,12 +335,13 @@ __global__ void k_certify(const T* __restrict__ x, const uint32_t* __restrict__ 
     float dg = group_dot_ref(match, xr, c + (size_t)jg * d, d, lane);
     float d1 = __shfl_sync(kFull, dg, 0);
     float d2 = __shfl_sync(kFull, dg, gsz);
-    float xres = 0.0f;  // |x - bf16(x)|, upper-rounded (single-term BF16 bound)
+    float xres = 0.0f;  // |x - x^|, upper-rounded (single-term bound)
     if (kr > 0.0f) {
+        const float S = bounds->s16;
         float acc = 0.0f;
-        for (int i = lane; i < d; i += 32) acc = bf16_resid_sq(to_f32(xr[i]), acc);
+        for (int i = lane; i < d; i += 32) acc = f16_resid_sq(S * to_f32(xr[i]), acc);
         for (int o = 16; o; o >>= 1) acc = __fadd_ru(acc, __shfl_xor_sync(kFull, acc, o));
-        xres = __fmul_ru(__fsqrt_ru(acc), 1.0000005f);
+        xres = f16_resid(acc, S);
     }
     if (lane != 0) return;
     float theta = 0.0f;
@@ -353,11 +411,12 @@ __global__ void k_certify16(const T* __restrict__ x, const uint32_t* __restrict_
     const float* c2 = c + (size_t)j2 * d;
     const int body = d & ~15, dr = (d + 15) & ~15;
     float sq = 0.0f, a1 = 0.0f, a2 = 0.0f, rs = 0.0f;
+    const float S = kr > 0.0f ? bounds->s16 : 1.0f;
     for (int i = l; i < dr; i += 16) {
         const bool in = i < d;
         const float xv = in ? to_f32(xr[i]) : 0.0f;
         if (i < body) sq = __fadd_rn(sq, __fmul_rn(xv, xv));
-        if (kr > 0.0f) rs = bf16_resid_sq(xv, rs);
+        if (kr > 0.0f) rs = f16_resid_sq(S * xv, rs);
         a1 = __fmaf_rn(xv, in ? c1[i] : 0.0f, a1);
         a2 = __fmaf_rn(xv, in ? c2[i] : 0.0f, a2);
     }
@@ -381,7 +440,7 @@ __global__ void k_certify16(const T* __restrict__ x, const uint32_t* __restrict_
     float theta = 0.0f;
     if (live && l == 0) {
         ok = certify_decide(row, t, j1, j2, a1, a2, xn, k, norms, bounds, ka, kb, labels, dist, fast_err, ka2, kb2,
-                              row_bounds, &theta, kr, __fmul_ru(__fsqrt_ru(rs), 1.0000005f));
+                              row_bounds, &theta, kr, f16_resid(rs, S));
         redo = !ok;
     }
     certify_tally(ok, redo, row, theta, cert_count, redo_count, redo_rows, redo_theta);
@@ -419,6 +478,7 @@ __global__ void k_certify16v(const float* __restrict__ x, const uint32_t* __rest
     const float* c2 = c + (size_t)j2 * d;
     float sq[4] = {0.0f, 0.0f, 0.0f, 0.0f}, p1[4] = {0.0f, 0.0f, 0.0f, 0.0f}, p2[4] = {0.0f, 0.0f, 0.0f, 0.0f};
     float rs = 0.0f;
+    const float S = kr > 0.0f ? bounds->s16 : 1.0f;
     for (int i = 4 * q; i < d; i += 16) {
         const float4 xv = *reinterpret_cast<const float4*>(xr + i);
         const float4 u = *reinterpret_cast<const float4*>(c1 + i);
@@ -429,7 +489,7 @@ __global__ void k_certify16v(const float* __restrict__ x, const uint32_t* __rest
             sq[j] = __fadd_rn(sq[j], __fmul_rn(xs[j], xs[j]));
             p1[j] = __fmaf_rn(xs[j], us[j], p1[j]);
             p2[j] = __fmaf_rn(xs[j], ws[j], p2[j]);
-            if (kr > 0.0f) rs = bf16_resid_sq(xs[j], rs);
+            if (kr > 0.0f) rs = f16_resid_sq(S * xs[j], rs);
         }
     }
     rs = __fadd_ru(rs, __shfl_xor_sync(kFull, rs, 2));
@@ -457,7 +517,7 @@ __global__ void k_certify16v(const float* __restrict__ x, const uint32_t* __rest
     float theta = 0.0f;
     if (live && q == 0) {
         ok = certify_decide(row, t, j1, j2, a1, a2, xn, k, norms, bounds, ka, kb, labels, dist, fast_err, ka2, kb2,
-                              row_bounds, &theta, kr, __fmul_ru(__fsqrt_ru(rs), 1.0000005f));
+                              row_bounds, &theta, kr, f16_resid(rs, S));
         redo = !ok;
     }
     certify_tally(ok, redo, row, theta, cert_count, redo_count, redo_rows, redo_theta);

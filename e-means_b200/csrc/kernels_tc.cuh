@@ -52,14 +52,15 @@ constexpr int kTcLoadWarps = 2;
 constexpr int kTcEpi0 = 2 + kTcLoadWarps;
 constexpr int kTcPThreads = 32 * (kTcEpi0 + kTcEpiWarps);
 constexpr int kTcRowScaleSlots = 4;  // FP8 per-row scales, a ring over work items
-// Norms inside the contraction (single-term BF16 search of f32 rows): each tile
-// starts with one K = 16 MMA of a constant row operand [1, 1, 1, 0, ...] against
-// the tile's half-norms split into three BF16 parts, so the accumulator holds
-// norm / 2 - x . c (the rows enter negated), half the score, and the epilogue
-// scores without loading norms or multiplying. A ring of two 8 KB slices.
+// Norms inside the contraction (single-term search of f32 rows, NM, FP16 operands
+// scaled by S: k_prep_f16): each tile starts with one K = 16 MMA of a constant row
+// operand [1024, 1024, 1024, 0, ...] against the tile's half-norms split into three
+// parts, so the accumulator holds S^2 (norm / 2 - x . c) (the rows enter negated), the
+// score times S^2 / 2, and the epilogue scores without loading norms or multiplying. A
+// ring of two 8 KB slices.
 constexpr int kTcNmSlots = 2;
-constexpr uint32_t kTcNmSlotBytes = (uint32_t)kTcBN * 32;  // 256 centroids x 16 BF16
-constexpr uint32_t kTcNmConstBytes = (uint32_t)kTcBM * 32;  // 128 rows x 16 BF16
+constexpr uint32_t kTcNmSlotBytes = (uint32_t)kTcBN * 32;  // 256 centroids x 16 FP16
+constexpr uint32_t kTcNmConstBytes = (uint32_t)kTcBM * 32;  // 128 rows x 16 FP16
 
 struct TcParams {
     int m, d, k, kpad;   // kpad: d rounded up to 64 (one 128-byte swizzle atom per 64 BF16)
@@ -93,16 +94,15 @@ struct TcParams {
     // centroid; wf8[j] = -2 / (centroid j's scale), 0 past k (score = norm + acc r w).
     const float* wf8;
     int nsplit;  // column splits of the search (work item = row tile x split)
-    // Norms inside the contraction: [tiles * 256][16] BF16, row j = the three BF16
-    // parts of norms[j] / 2, then zeros (k_prep_nrm16).
-    const __nv_bfloat16* nrm16;
+    // Norms inside the contraction: [tiles * 256][16] FP16 (k_prep_f16).
+    const __half* nrm16;
     // Certification at the end of each work item (norms inside the contraction,
     // one column split, f32 rows with d % 16 == 0 and 16-byte aligned rows and
     // centroids, AVX-512 rounding): the decisions of k_certify16v, taken by the
     // epilogue warps from the row tile's merged top-2, in place of that kernel.
     int fuse;
     const float* cx;  // f32 centroids [k][d]
-    const Bounds* bounds;
+    const Bounds* bounds;  // (NM: also the operands' scale)
     float ka, kb, kr, ka2, kb2;
     uint32_t* labels;
     float* dist;
@@ -226,6 +226,10 @@ EMB_DEV uint64_t sw32_desc(uint32_t saddr) {
     return d;
 }
 
+// Instruction descriptor, kind::f16: F16 x F16 -> F32, both K-major, M x N.
+__host__ __device__ constexpr uint32_t idesc_f16(int M, int N) {
+    return (1u << 4) | ((uint32_t)(N >> 3) << 17) | ((uint32_t)(M >> 4) << 24);
+}
 // Instruction descriptor, kind::f16: BF16 x BF16 -> F32, both K-major, M x N.
 __host__ __device__ constexpr uint32_t idesc_bf16(int M, int N) {
     return (1u << 4) | (1u << 7) | (1u << 10) | ((uint32_t)(N >> 3) << 17) | ((uint32_t)(M >> 4) << 24);
@@ -336,12 +340,11 @@ EMB_DEV size_t tc_src_row(const TcParams& p, int g) {
 // Row tile -> BF16 hi (and lo for three terms) in the K-major 128B-swizzled layout,
 // by threads tid = 0 .. nthr-1: 128 rows x (kpad / 8) chunks of 8 elements. Each
 // thread issues the loads of up to four chunks before converting any of them, so
-// that the gathered rows' latencies overlap. neg: the rows negated (exact; BF16
-// rounding to nearest is symmetric), for the norms-in-the-contraction search.
-template <typename T>
+// that the gathered rows' latencies overlap. F16 (the norms-in-the-contraction search):
+// the rows times sg, minus a power of two, as one FP16 part.
+template <bool F16, typename T>
 EMB_DEV void tc_load_rows(uint8_t* a_hi, uint8_t* a_lo, const T* __restrict__ x, const TcParams& p, int row0, int m,
-                          int tid, int nthr, bool neg = false) {
-    const float sg = neg ? -1.0f : 1.0f;
+                          int tid, int nthr, float sg) {
     constexpr int kBatch = 4;
     const int nchunk = p.kpad / 8;
     const int total = kTcBM * nchunk;
@@ -374,18 +377,27 @@ EMB_DEV void tc_load_rows(uint8_t* a_hi, uint8_t* a_lo, const T* __restrict__ x,
             if (t >= total) continue;
             const int r = t / nchunk, kc = t % nchunk;
             uint32_t hw[4], lw[4];
-#pragma unroll
-            for (int i = 0; i < 4; i++) {
-                const float v0 = sg * v[u][2 * i], v1 = sg * v[u][2 * i + 1];
-                __nv_bfloat16 h0 = __float2bfloat16_rn(v0), h1 = __float2bfloat16_rn(v1);
-                __nv_bfloat16 l0 = __float2bfloat16_rn(v0 - __bfloat162float(h0));
-                __nv_bfloat16 l1 = __float2bfloat16_rn(v1 - __bfloat162float(h1));
-                hw[i] = (uint32_t)__bfloat16_as_ushort(h0) | ((uint32_t)__bfloat16_as_ushort(h1) << 16);
-                lw[i] = (uint32_t)__bfloat16_as_ushort(l0) | ((uint32_t)__bfloat16_as_ushort(l1) << 16);
-            }
             const uint32_t off = sw128_offset(r, kc, kTcBM);
-            *reinterpret_cast<uint4*>(a_hi + off) = make_uint4(hw[0], hw[1], hw[2], hw[3]);
-            if (p.nterms == 3) *reinterpret_cast<uint4*>(a_lo + off) = make_uint4(lw[0], lw[1], lw[2], lw[3]);
+            if constexpr (F16) {
+#pragma unroll
+                for (int i = 0; i < 4; i++) {
+                    const __half2 h = __floats2half2_rn(sg * v[u][2 * i], sg * v[u][2 * i + 1]);
+                    hw[i] = *reinterpret_cast<const uint32_t*>(&h);
+                }
+                *reinterpret_cast<uint4*>(a_hi + off) = make_uint4(hw[0], hw[1], hw[2], hw[3]);
+            } else {
+#pragma unroll
+                for (int i = 0; i < 4; i++) {
+                    const float v0 = v[u][2 * i], v1 = v[u][2 * i + 1];
+                    __nv_bfloat16 h0 = __float2bfloat16_rn(v0), h1 = __float2bfloat16_rn(v1);
+                    __nv_bfloat16 l0 = __float2bfloat16_rn(v0 - __bfloat162float(h0));
+                    __nv_bfloat16 l1 = __float2bfloat16_rn(v1 - __bfloat162float(h1));
+                    hw[i] = (uint32_t)__bfloat16_as_ushort(h0) | ((uint32_t)__bfloat16_as_ushort(h1) << 16);
+                    lw[i] = (uint32_t)__bfloat16_as_ushort(l0) | ((uint32_t)__bfloat16_as_ushort(l1) << 16);
+                }
+                *reinterpret_cast<uint4*>(a_hi + off) = make_uint4(hw[0], hw[1], hw[2], hw[3]);
+                if (p.nterms == 3) *reinterpret_cast<uint4*>(a_lo + off) = make_uint4(lw[0], lw[1], lw[2], lw[3]);
+            }
         }
     }
 }
@@ -671,13 +683,6 @@ EMB_DEV void mma_e4m3(uint32_t d_tmem, uint64_t adesc, uint64_t bdesc, uint32_t 
         ::"r"(d_tmem), "l"(adesc), "l"(bdesc), "r"(idesc), "r"(accumulate));
 }
 
-// The half-norms again after a bias changed the norms (k_prep_centroids writes them
-// otherwise). Rows up to kp (whole tiles): the padding too.
-__global__ void k_prep_nrm16(const float* __restrict__ norms, int kp, __nv_bfloat16* __restrict__ out) {
-    const int j = blockIdx.x * blockDim.x + threadIdx.x;
-    if (j < kp) nrm16_row(norms[j], out + (size_t)j * 16);
-}
-
 // Scores of 16 accumulator columns (in place): s = norm - 2 acc (BF16), or
 // s = norm + (acc r) w (FP8: acc r undoes the row's power-of-two scale exactly,
 // w = -2 / the centroid's scale), one rounding each.
@@ -778,6 +783,7 @@ EMB_DEV void tc_fused_certify(const TcParams& p, const float* __restrict__ x, co
                               int row0, int m, bool valid, int lt, int nthr) {
     const int q = lt & 3, lane = (int)threadIdx.x & 31;
     const int d = p.d, k = p.k;
+    const float S = p.bounds->s16;
     for (int r0 = 0; r0 < kTcBM; r0 += nthr / 4) {
         const int r = r0 + (lt >> 2);
         const int row = row0 + r;
@@ -805,7 +811,7 @@ EMB_DEV void tc_fused_certify(const TcParams& p, const float* __restrict__ x, co
                 for (int j = 0; j < 4; j++) {
                     sq[j] = __fadd_rn(sq[j], __fmul_rn(xs[j], xs[j]));
                     p1[j] = __fmaf_rn(xs[j], us[j], p1[j]);
-                    rs = bf16_resid_sq(xs[j], rs);
+                    rs = f16_resid_sq(S * xs[j], rs);
                 }
             }
             rs = __fadd_ru(rs, __shfl_xor_sync(kFull, rs, 2));
@@ -826,8 +832,7 @@ EMB_DEV void tc_fused_certify(const TcParams& p, const float* __restrict__ x, co
                 // pair), so one exact dot product serves both.
                 const int no_abort = 0;
                 ok = certify_decide(row, t, j1, j1, a1, a1, xn, k, p.norms, p.bounds, p.ka, p.kb, p.labels, p.dist,
-                                    &no_abort, p.ka2, p.kb2, nullptr, &theta, p.kr,
-                                    __fmul_ru(__fsqrt_ru(rs), 1.0000005f));
+                                    &no_abort, p.ka2, p.kb2, nullptr, &theta, p.kr, f16_resid(rs, S));
                 redo = !ok;
             }
         } else {
@@ -922,12 +927,12 @@ k_assign_tc(const T* __restrict__ x, const __grid_constant__ CUtensorMap map_hi,
         for (int i = threadIdx.x; i < 4 * kTcBM; i += blockDim.x) pub[i] = INFINITY;
     }
     if (NM) {
-        // The constant row operand of the norm MMA: every row [1, 1, 1, 0, 0, 0, 0, 0]
-        // in both 16-byte halves (BF16 one = 0x3F80), so whichever half the 32-byte
-        // swizzle pairs with the norm slice's parts, the product is p1 + p2 + p3.
+        // The constant row operand of the norm MMA: every row [1024, 1024, 1024, 0, 0, 0,
+        // 0, 0] (kNrm16One, FP16 0x6400) in both 16-byte halves, so whichever half the 32-byte
+        // swizzle pairs with the norm slice's parts, the product is 1024 (p1 + p2 + p3).
         uint4* nc = reinterpret_cast<uint4*>(smem + L.nconst);
         for (int i = threadIdx.x; i < (int)(kTcNmConstBytes / 16); i += blockDim.x)
-            nc[i] = make_uint4(0x3F803F80u, 0x00003F80u, 0u, 0u);
+            nc[i] = make_uint4(0x64006400u, 0x00006400u, 0u, 0u);
         asm volatile("fence.proxy.async.shared::cta;" ::: "memory");  // visible to the tensor cores
     }
     tc_fence_before();
@@ -995,7 +1000,7 @@ k_assign_tc(const T* __restrict__ x, const __grid_constant__ CUtensorMap map_hi,
     } else if (warp == 1) {
         if (lane == 0) {
             // ---- MMA issuer: per unit, nterms x 4 MMAs of M=128 N=256 (K=16 BF16 / K=32 e4m3)
-            const uint32_t idesc = FP8 ? idesc_e4m3(kTcBM, kTcBN) : idesc_bf16(kTcBM, kTcBN);
+            const uint32_t idesc = FP8 ? idesc_e4m3(kTcBM, kTcBN) : NM ? idesc_f16(kTcBM, kTcBN) : idesc_bf16(kTcBM, kTcBN);
             const uint32_t a_atom = (kTcBM * 128) >> 4;  // descriptor units (16 B) per A atom
             int u = 0, tg = 0;
             bool ok = true;
@@ -1095,7 +1100,8 @@ k_assign_tc(const T* __restrict__ x, const __grid_constant__ CUtensorMap map_hi,
                     tc_load_rows_fp8(a, rscale_s + (i % kTcRowScaleSlots) * kTcBM, x, p, (w / nsplit) * kTcBM, m,
                                      ltid);
                 else
-                    tc_load_rows(a, a + L.a_lo, x, p, (w / nsplit) * kTcBM, m, ltid, kTcLoadWarps * 32, NM);
+                    tc_load_rows<NM>(a, a + L.a_lo, x, p, (w / nsplit) * kTcBM, m, ltid, kTcLoadWarps * 32,
+                                     NM ? -p.bounds->s16 : 1.0f);
                 asm volatile("fence.proxy.async.shared::cta;" ::: "memory");  // visible to the tensor cores
                 mbar_arrive(&a_full[ab]);
                 // The epilogue reads slot i % 4 of the row scales at item i. The loader
@@ -1130,8 +1136,8 @@ k_assign_tc(const T* __restrict__ x, const __grid_constant__ CUtensorMap map_hi,
                 // terms: 34 -> 20 us; the refine pass of 5% of 1M x 128 rows at k = 16384:
                 // 902 -> 675 us.
                 uint8_t* a = smem + (i % NB) * L.a_buf;
-                tc_load_rows(a, a + L.a_lo, x, p, (w / nsplit) * kTcBM, m, (int)threadIdx.x - 32 * kTcEpi0,
-                             kTcEpiWarps * 32, NM);
+                tc_load_rows<NM>(a, a + L.a_lo, x, p, (w / nsplit) * kTcBM, m, (int)threadIdx.x - 32 * kTcEpi0,
+                                 kTcEpiWarps * 32, NM ? -p.bounds->s16 : 1.0f);
                 asm volatile("fence.proxy.async.shared::cta;" ::: "memory");  // visible to the tensor cores
                 __syncwarp();
                 if (lane < kTcLoadWarps * 32 / kTcEpiWarps) mbar_arrive(&a_full[i % NB]);
@@ -1272,7 +1278,8 @@ k_assign_tc(const T* __restrict__ x, const __grid_constant__ CUtensorMap map_hi,
                     // holds by construction (every value folded into s2 is at least
                     // the final best key); were it ever violated, raising s2 to s1
                     // leaves no margin, so the row goes to the refine pass.
-                    const float unit = NM ? 2.0f : 1.0f;  // NM: half-scores back to scores (exact)
+                    // NM: scaled half-scores back to scores (a power of two)
+                    const float unit = NM ? 2.0f / (p.bounds->s16 * p.bounds->s16) : 1.0f;
                     if (NM && p.fuse) {
                         // For the row loaders' certification, once they are done with
                         // the previous item's (never after a wait that gave up).

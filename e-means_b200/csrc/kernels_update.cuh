@@ -895,7 +895,7 @@ EMB_DEV void revive_cta(int k, int d, float* __restrict__ c, float* __restrict__
 EMB_DEV void step_end(int now, int* __restrict__ step, Bounds* __restrict__ bounds, uint32_t* __restrict__ ctr,
                       int nctr) {
     *step = now + 1;
-    *bounds = Bounds{0.0f, 0.0f, 0.0f, 0.0f};
+    *bounds = Bounds{};
     for (int i = 0; i < nctr; i++) ctr[i] = 0u;
 }
 __global__ void k_step_end(int* __restrict__ step, Bounds* __restrict__ bounds, uint32_t* __restrict__ ctr, int nctr) {

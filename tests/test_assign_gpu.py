@@ -475,3 +475,54 @@ def test_fp32_search_tile_edges(emb, orc, m, k, d, dtype):
     ref_l, ref_d = orc.cpu_assign(x, c, kernel="avx512", emulate=not orc.has_kernel("avx512"))
     assert np.array_equal(lab, ref_l)
     assert np.array_equal(dist.view(np.uint32), ref_d.view(np.uint32))
+
+
+@pytest.mark.parametrize("case", ["plain", "tiny", "huge", "wide", "one_large", "far_rows", "bias", "large_bias",
+                                  "zero", "nonfinite", "subnormal"])
+@pytest.mark.parametrize("m,k,d", [(700, 300, 33), (20000, 520, 64), (20003, 259, 128)])
+def test_single_term_operand_scale(emb, orc, assigners, case, m, k, d):
+    # The single-term search scales its FP16 operands by one power of two: magnitudes at
+    # the ends of the f32 range, spread over many binades, rows far beyond the
+    # centroids, biases beside and above the norms. Always the reference's bits.
+    rng = np.random.default_rng(m + k + d)
+    c = rng.standard_normal((k, d), dtype=np.float32)
+    x = c[rng.integers(0, k, m)] + rng.standard_normal((m, d), dtype=np.float32) * np.float32(0.3)
+    bias = None
+    if case == "tiny":
+        x, c = x * np.float32(1e-12), c * np.float32(1e-12)
+    elif case == "huge":
+        x, c = x * np.float32(1e15), c * np.float32(1e15)
+    elif case == "wide":
+        s = np.exp2(rng.integers(-20, 8, d)).astype(np.float32)
+        x, c = x * s, c * s
+    elif case == "one_large":
+        c[k // 2] *= np.float32(1e4)
+    elif case == "far_rows":
+        x[::3] *= np.float32(3000.0)
+        x[5] = 60000.0
+    elif case == "bias":
+        bias = rng.uniform(-1.0, 1.0, k).astype(np.float32)
+    elif case == "large_bias":
+        bias = rng.uniform(0, 3e6, k).astype(np.float32)
+    elif case == "zero":
+        c[::2] = 0.0
+        x[::5] = 0.0
+    elif case == "nonfinite":
+        c[3, 0] = np.inf
+        x[7, 1] = np.nan
+        x[8] = 3e38
+    elif case == "subnormal":
+        x, c = x * np.float32(1e-40), c * np.float32(1e-40)
+    x, c = x.astype(np.float32), c.astype(np.float32)
+    a = assigners("bf16x1")
+    a.set_centroids(c)
+    if bias is not None:
+        a.set_bias(bias)
+    lab, dist = a.assign(x)
+    rl, rd = orc.cpu_assign(x, c, bias=bias, emulate=not orc.has_kernel("avx512"))
+    assert np.array_equal(lab, rl)
+    assert np.array_equal(np.isnan(dist), np.isnan(rd)) and same_f32(np.nan_to_num(dist), np.nan_to_num(rd))
+    st = a.stats()
+    assert st["fast_aborted"] == 0 and st["fast_kernel"] == 1
+    if case in ("plain", "tiny", "huge"):  # the scale keeps the bound: nearly every row certified at once
+        assert st["rows_refined"] < 0.02 * m, st
