@@ -574,6 +574,8 @@ int launch_i8_assign(emb200_handle* h, const int8_t* x, const uint32_t* gather, 
         p.pkeys = h->pkeys.p;
         p.part_s = (long long*)h->part_s.p;
         p.part_i = h->part_i.p;
+        p.labels = labels;
+        p.dist = dist;
         p.err = (int*)(h->counters.p + 2);
         p.stall_tile = h->stall_tile;
         p.stall_ns = h->stall_ns;
@@ -597,9 +599,11 @@ int launch_i8_assign(emb200_handle* h, const int8_t* x, const uint32_t* gather, 
     }
     if (!graph) CK(cudaEventRecord(h->evk1, st));
     h->stats.fast_kernel = tc ? 3 : 2;
-    k_finish_i8<<<(unsigned)((m + 7) / 8), 256, 0, st>>>(x, gather, (int)m, d, (const long long*)h->part_s.p,
-                                                         h->part_i.p, nsplit, labels, dist, inv_unit);
-    CKL();
+    if (!tc || nsplit > 1) {
+        k_finish_i8<<<(unsigned)((m + 7) / 8), 256, 0, st>>>(x, gather, (int)m, d, (const long long*)h->part_s.p,
+                                                             h->part_i.p, nsplit, labels, dist, inv_unit);
+        CKL();
+    }
     if (tc && !graph) {  // the bounded waits gave up: redo the call with the exact dp4a kernel
         uint32_t err = 0;
         CK(cudaMemcpyAsync(&err, h->counters.p + 2, sizeof err, cudaMemcpyDeviceToHost, st));

@@ -28,6 +28,8 @@ struct TcI8Params {
     const int* pkeys;          // P_j, padded to whole tiles with 0x7f000000
     long long* part_s;         // [split][row] exact score
     uint32_t* part_i;          // [split][row] label
+    uint32_t* labels;          // one column split: the results themselves, no partials
+    float* dist;
     int* err;
     int stall_tile;            // abort-path test, as TcParams::stall_tile
     uint64_t stall_ns;
@@ -41,14 +43,15 @@ __host__ __device__ inline TcSmem tc_i8_smem_layout(int kpad) {
     s.b0 = a_bytes;
     s.term_bytes = (uint32_t)kTcBN * 128;
     s.stage_bytes = s.term_bytes;
-    const uint32_t fixed = kTcNormSlots * kTcBN * 4 + 3 * kTcBM * 16 + 256 + 1024;
+    const uint32_t fixed = kTcNormSlots * kTcBN * 4 + 3 * kTcBM * 16 + 256 + kTcBM * 4 + 1024;
     int st = 0;
     while (st < kTcMaxStages && a_bytes + (st + 1) * s.stage_bytes + fixed <= (uint32_t)kTcSmemLimit) st++;
     s.stages = st;
     s.norms = s.b0 + st * s.stage_bytes;
     s.merge = s.norms + kTcNormSlots * kTcBN * 4;
     s.bars = s.merge + 3 * kTcBM * 16;
-    s.total = s.bars + 256;
+    s.pub = s.bars + 256;  // the rows' norms
+    s.total = s.pub + kTcBM * 4;
     return s;
 }
 
@@ -80,6 +83,7 @@ k_assign_tc_i8(const int8_t* __restrict__ x, const __grid_constant__ CUtensorMap
     uint64_t* stall_bar = mma_done + 1;             // never completed (abort-path test)
     uint32_t* tmem_slot = (uint32_t*)(stall_bar + 1);
     volatile int* abort_flag = (volatile int*)(tmem_slot + 1);
+    int* xnorm_s = (int*)(smem + L.pub);  // |x|^2 of the rows: exact in 32 bits for d <= 512
     int* keys_s = (int*)(smem + L.norms);
 
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
@@ -105,26 +109,46 @@ k_assign_tc_i8(const int8_t* __restrict__ x, const __grid_constant__ CUtensorMap
         asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
     }
     if (warp == 1) tmem_alloc(tmem_slot, kTcTmemCols);
-    // Row tile: raw i8 copied into the 128B-swizzled K-major layout (16-byte chunks).
+    if (threadIdx.x < kTcBM) xnorm_s[threadIdx.x] = 0;
+    __syncthreads();
+    // Row tile: raw i8 copied into the 128B-swizzled K-major layout (16-byte chunks),
+    // up to eight chunks of a thread in flight before the first is stored: one at a
+    // time, seven memory latencies stood at the start of every CTA (500,000 x 512
+    // rows, k = 4096: 978 -> @@ us). The rows' norms come from the same registers, so
+    // that no later pass reads the rows again (113 us there).
     {
-        const int nchunk = p.kpad / 16;
-        for (int t = threadIdx.x; t < kTcBM * nchunk; t += blockDim.x) {
-            const int r = t / nchunk, kc = t % nchunk;
-            const int g = row0 + r;
-            uint4 v = make_uint4(0, 0, 0, 0);
-            if (g < p.m) {
+        constexpr int kBatch = 8;
+        const int nchunk = p.kpad / 16, total = kTcBM * nchunk;
+        const bool vec = (p.d & 15) == 0 && ((uintptr_t)x & 15) == 0;
+        for (int t0 = threadIdx.x; t0 < total; t0 += kBatch * blockDim.x) {
+            uint4 v[kBatch];
+#pragma unroll
+            for (int u = 0; u < kBatch; u++) {
+                const int t = t0 + u * (int)blockDim.x, r = t / nchunk, kc = t % nchunk, g = row0 + r;
+                v[u] = make_uint4(0, 0, 0, 0);
+                if (t >= total || g >= p.m) continue;
                 const size_t src = p.gather ? p.gather[g] : (size_t)g;
                 const int8_t* xr = x + src * (size_t)p.d + kc * 16;
-                if (kc * 16 + 16 <= p.d && ((uintptr_t)xr & 15) == 0) {
-                    v = *reinterpret_cast<const uint4*>(xr);
+                if (vec) {
+                    if (kc * 16 < p.d) v[u] = __ldg(reinterpret_cast<const uint4*>(xr));
                 } else {
                     uint32_t w[4] = {0, 0, 0, 0};
+#pragma unroll
                     for (int b = 0; b < 16; b++)
                         if (kc * 16 + b < p.d) w[b >> 2] |= (uint32_t)(uint8_t)xr[b] << (8 * (b & 3));
-                    v = make_uint4(w[0], w[1], w[2], w[3]);
+                    v[u] = make_uint4(w[0], w[1], w[2], w[3]);
                 }
             }
-            *reinterpret_cast<uint4*>(smem + sw128_offset(r, kc, kTcBM)) = v;
+#pragma unroll
+            for (int u = 0; u < kBatch; u++) {
+                const int t = t0 + u * (int)blockDim.x, r = t / nchunk, kc = t % nchunk;
+                if (t >= total) continue;
+                *reinterpret_cast<uint4*>(smem + sw128_offset(r, kc, kTcBM)) = v[u];
+                const int n = __dp4a((int)v[u].x, (int)v[u].x,
+                                     __dp4a((int)v[u].y, (int)v[u].y,
+                                            __dp4a((int)v[u].z, (int)v[u].z, __dp4a((int)v[u].w, (int)v[u].w, 0))));
+                if (n) atomicAdd(&xnorm_s[r], n);
+            }
         }
     }
     asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
@@ -258,9 +282,16 @@ k_assign_tc_i8(const int8_t* __restrict__ x, const __grid_constant__ CUtensorMap
                     best = ob;
                 }
             }
-            const size_t oo = (size_t)blockIdx.y * p.m + row;
-            p.part_s[oo] = best == 0x7fffffff ? 0x7fffffffffffffffll : bs;
-            p.part_i[oo] = best == 0x7fffffff ? 0u : bl;
+            const long long b = best == 0x7fffffff ? 0x7fffffffffffffffll : bs;
+            const uint32_t l = best == 0x7fffffff ? 0u : bl;
+            if (nsplit == 1) {  // as k_finish_i8
+                p.labels[row] = l;
+                p.dist[row] = (float)fmax(__dadd_rn((double)xnorm_s[r], (double)b), 0.0);
+            } else {
+                const size_t oo = (size_t)blockIdx.y * p.m + row;
+                p.part_s[oo] = b;
+                p.part_i[oo] = l;
+            }
         }
     }
     tc_fence_before();
