@@ -421,6 +421,156 @@ __global__ void __launch_bounds__(256, 1) k_b_search_res(const float* __restrict
     }
 }
 
+// The resident-row search with 8 x 8 values per thread on paired FMAs (fma.rn.f32x2,
+// see kernels_simt.cuh): 128 rows x 128 centroids per tile, the running top-2 in shared
+// memory, so that two CTAs fit an SM (d <= 64) and one loads while the other
+// multiplies. k_b_search_res holds 8 x 4 values: three 16-byte shared loads per 32 FMAs,
+// half again the shared-memory port's rate. 48 lists (d = 64, k = 16 .. 781), all steps:
+// 13.6 -> 10.8 ms with an item per centroid tile, 11.4 with all tiles in one item; d =
+// 32 / 96 / 128: 2.9 -> 2.3, 5.8 -> 4.3, 3.1 -> 2.8 ms.
+constexpr int kBTile = 128;
+inline size_t b_tile_smem(int d) {
+    return (size_t)d * 2 * kBTile * sizeof(float) + (size_t)8 * 256 * sizeof(float4);
+}
+constexpr size_t kBTileSmemMax = (size_t)kBResMaxD * 2 * kBTile * sizeof(float) + (size_t)8 * 256 * sizeof(float4);
+
+__global__ void __launch_bounds__(256, 2) k_b_search_tile(const float* __restrict__ x, BArgs a) {
+    extern __shared__ __align__(16) float res_smem[];
+    __shared__ uint32_t item_s;
+    const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+    const int d = a.d, dq = d >> 2;
+    float* As = res_smem;                                               // [d][128]
+    float* Bs = As + d * kBTile;                                        // [d][128]
+    float4* tops = reinterpret_cast<float4*>(Bs + d * kBTile);          // [8][256]: s1, i1, s2, i2
+    const int rbase = (warp >> 1) * 32 + (lane >> 3) * 4;  // + 16 g: this thread's row groups
+    const int cbase = (warp & 1) * 64 + (lane & 7) * 4;    // + 32 g: its column groups
+    const float inf = __int_as_float(0x7f800000), none = __uint_as_float(0xffffffffu);
+    for (;;) {
+        if (tid == 0) item_s = atomicAdd(&a.ctl->qhead, 1u);
+        __syncthreads();
+        const uint32_t it = item_s;
+        __syncthreads();
+        if (it >= a.total_items) break;
+        const int i = (int)a.item_inst[it];
+        BStep st;
+        if (!b_active(a, i, &st)) continue;  // uniform: every thread read the same item
+        const BInst& I = a.inst[i];
+        const uint32_t local = it - I.item_off;
+        const int rt = (int)(local / I.nsplit), split = (int)(local % I.nsplit);
+        const int row0 = rt * kBTile;
+        if (row0 >= (int)st.bn) continue;
+        const uint32_t* ids = b_rows(a, I, st);
+        const float* xi = x + I.row0 * (size_t)d;
+        const float* ci = a.c + I.c_off;
+        const float* ni = a.norms + I.k_off;
+        const int k = (int)I.k, m = (int)st.bn;
+        const int ntiles = (k + kBTile - 1) / kBTile;
+        // transposed: element e = (chunk c of four dimensions, row r) with r fastest; two
+        // threads per row, so a thread's row never changes
+        {
+            const int r = tid & (kBTile - 1);
+            const float* src = row0 + r < m ? xi + (size_t)ids[row0 + r] * d : nullptr;
+#pragma unroll 4
+            for (int c = tid >> 7; c < dq; c += 2) {
+                const float4 v = src ? *reinterpret_cast<const float4*>(src + 4 * c) : make_float4(0, 0, 0, 0);
+                As[(4 * c + 0) * kBTile + r] = v.x;
+                As[(4 * c + 1) * kBTile + r] = v.y;
+                As[(4 * c + 2) * kBTile + r] = v.z;
+                As[(4 * c + 3) * kBTile + r] = v.w;
+            }
+        }
+#pragma unroll
+        for (int q = 0; q < 8; q++) tops[q * 256 + tid] = make_float4(inf, none, inf, none);
+        for (int tile = split; tile < ntiles; tile += (int)I.nsplit) {
+            const int col0 = tile * kBTile;
+            __syncthreads();  // the previous tile's readers are done with Bs
+            {
+                const int cc = tid & (kBTile - 1);
+                const float* src = col0 + cc < k ? ci + (size_t)(col0 + cc) * d : nullptr;
+#pragma unroll 4
+                for (int c = tid >> 7; c < dq; c += 2) {
+                    const float4 v = src ? *reinterpret_cast<const float4*>(src + 4 * c) : make_float4(0, 0, 0, 0);
+                    Bs[(4 * c + 0) * kBTile + cc] = v.x;
+                    Bs[(4 * c + 1) * kBTile + cc] = v.y;
+                    Bs[(4 * c + 2) * kBTile + cc] = v.z;
+                    Bs[(4 * c + 3) * kBTile + cc] = v.w;
+                }
+            }
+            __syncthreads();
+            if (col0 + (warp & 1) * 64 >= k) continue;  // none of the warp's columns exist
+            float2 acc[8][4];
+#pragma unroll
+            for (int q = 0; q < 8; q++)
+#pragma unroll
+                for (int j = 0; j < 4; j++) acc[q][j] = make_float2(0.0f, 0.0f);
+#pragma unroll 4
+            for (int kk = 0; kk < d; kk++) {
+                float2 b[4];
+#pragma unroll
+                for (int g = 0; g < 2; g++) {
+                    const float4 v = *reinterpret_cast<const float4*>(Bs + kk * kBTile + cbase + 32 * g);
+                    b[2 * g] = make_float2(v.x, v.y);
+                    b[2 * g + 1] = make_float2(v.z, v.w);
+                }
+#pragma unroll
+                for (int g = 0; g < 2; g++) {
+                    const float4 v = *reinterpret_cast<const float4*>(As + kk * kBTile + rbase + 16 * g);
+                    const float r4[4] = {v.x, v.y, v.z, v.w};
+#pragma unroll
+                    for (int q = 0; q < 4; q++)
+#pragma unroll
+                        for (int j = 0; j < 4; j++)
+                            acc[4 * g + q][j] = __ffma2_rn(make_float2(r4[q], r4[q]), b[j], acc[4 * g + q][j]);
+                }
+            }
+            float n[8];
+#pragma unroll
+            for (int j = 0; j < 8; j++) {  // columns past k never enter
+                const int col = col0 + cbase + (j >> 2) * 32 + (j & 3);
+                n[j] = col < k ? ni[col] : inf;
+            }
+#pragma unroll
+            for (int q = 0; q < 8; q++) {
+                float sc[8], mn = inf;
+#pragma unroll
+                for (int j = 0; j < 4; j++) {
+                    const float2 s2 = __ffma2_rn(make_float2(-2.0f, -2.0f), acc[q][j], make_float2(n[2 * j], n[2 * j + 1]));
+                    sc[2 * j] = s2.x;
+                    sc[2 * j + 1] = s2.y;
+                    mn = fminf(mn, fminf(s2.x, s2.y));
+                }
+                const float4 t4 = tops[q * 256 + tid];
+                if (mn < t4.z) {  // a thread's columns ascend: only a strictly smaller score enters
+                    Top2 t;
+                    t.s1 = t4.x; t.i1 = __float_as_uint(t4.y); t.s2 = t4.z; t.i2 = __float_as_uint(t4.w);
+#pragma unroll
+                    for (int j = 0; j < 8; j++)
+                        t.push_fast(sc[j], (uint32_t)(col0 + cbase + (j >> 2) * 32 + (j & 3)));
+                    tops[q * 256 + tid] = make_float4(t.s1, __uint_as_float(t.i1), t.s2, __uint_as_float(t.i2));
+                }
+            }
+        }
+        __syncthreads();
+        if (tid < kBTile && row0 + tid < m) {  // one thread per row merges the 16 that share it
+            const int wr = tid / 32, g = (tid & 31) / 16, ly = (tid & 15) >> 2, q0 = 4 * g + (tid & 3);
+            Top2 t;
+            t.init();
+#pragma unroll
+            for (int q = 0; q < 16; q++) {
+                const float4 e = tops[q0 * 256 + (wr * 2 + (q >> 3)) * 32 + ly * 8 + (q & 7)];
+                t.push(e.x, __float_as_uint(e.y));
+                t.push(e.z, __float_as_uint(e.w));
+            }
+            const size_t o = (I.p_off + (size_t)split * I.batch + row0 + tid) * 2;
+            a.part_s[o] = t.s1;
+            a.part_i[o] = t.i1;
+            a.part_s[o + 1] = t.s2;
+            a.part_i[o + 1] = t.i2;
+        }
+        __syncthreads();  // As and the lists are rewritten by the next item
+    }
+}
+
 // The search for small d (d <= D <= 32): one thread per batch row, an item being
 // 256 rows against centroid chunks split, split + nsplit, ... of 512 centroids,
 // each chunk staged in shared memory 8192 / D centroids at a time (every thread
@@ -537,11 +687,10 @@ __global__ void k_b_certify_small(const T* __restrict__ x, BArgs a) {
 }
 
 // Exhaustive exact search with a CTA per listed row (256 threads): warp w scans
-// the centroids [w k / 8, (w + 1) k / 8) in ascending order in groups as
-// k_b_research does, and the warps' results merge by (score, index), finite
-// scores only: the lowest index among the smallest scores, label 0 when no score
-// beats +inf, as the reference's strict-< scan over all k. A row's centroid
-// loads are spread over eight warps, where k_b_research walks all k in one.
+// the centroids [w k / 8, (w + 1) k / 8) in ascending order in lane groups, and the
+// warps' results merge by (score, index), finite scores only: the lowest index
+// among the smallest scores, label 0 when no score beats +inf, as the reference's
+// strict-< scan over all k.
 template <typename T>
 __global__ void __launch_bounds__(256) k_b_research_cta(const T* __restrict__ x, BArgs a) {
     __shared__ float wbest[8];
@@ -576,6 +725,99 @@ __global__ void __launch_bounds__(256) k_b_research_cta(const T* __restrict__ x,
             }
         }
         for (int o = gsz; o < 32; o <<= 1) {
+            const float ob = __shfl_xor_sync(kFull, best, o);
+            const uint32_t ol = __shfl_xor_sync(kFull, lab, o);
+            if (ob < inf && (!(best < inf) || lex_less(ob, ol, best, lab))) {
+                best = ob;
+                lab = ol;
+            }
+        }
+        if (lane == 0) {
+            wbest[warp] = best;
+            wlab[warp] = lab;
+        }
+        const float xn = warp_sqnorm_ref(xr, d, lane);
+        __syncthreads();
+        if (threadIdx.x == 0) {
+            float b = inf;
+            uint32_t l = 0;
+            for (int w = 0; w < 8; w++)
+                if (wbest[w] < inf && (!(b < inf) || lex_less(wbest[w], wlab[w], b, l))) {
+                    b = wbest[w];
+                    l = wlab[w];
+                }
+            a.blabels[I.b_off + row] = l;
+            a.bdist[I.b_off + row] = fmaxf(__fadd_rn(b, xn), 0.0f);
+        }
+        __syncthreads();  // wbest / wlab are rewritten for the next row
+    }
+}
+
+// The same search for f32 rows with d % 16 == 0, d <= 128, under the AVX-512 rounding:
+// four threads per centroid with 16-byte loads, the row's values in registers, 128
+// centroids of the row in flight per CTA (two per quad); the 16 lanes' sums in the tree
+// of k_b_certify16v. The half-warp form loads 4 bytes at a time and reduces over 16
+// lanes: 6.3 ms of the 34 ms on the device of 48 lists' training (2.6% of the rows
+// come here), 3.0 ms this way.
+__global__ void __launch_bounds__(256) k_b_research16v(const float* __restrict__ x, BArgs a) {
+    __shared__ float wbest[8];
+    __shared__ uint32_t wlab[8];
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, q = lane & 3, g = threadIdx.x >> 2;
+    const uint32_t n = a.ctl->redo;
+    const int d = a.d;
+    const float inf = __int_as_float(0x7f800000);
+    for (uint32_t r = blockIdx.x; r < n; r += gridDim.x) {
+        const uint32_t e = a.redo_list[r];
+        const int i = (int)(e >> 24), row = (int)(e & 0xFFFFFFu);
+        BStep st;
+        b_active(a, i, &st);
+        const BInst& I = a.inst[i];
+        const int k = (int)I.k;
+        const float* xr = x + (I.row0 + b_rows(a, I, st)[row]) * (size_t)d;
+        const float* ci = a.c + I.c_off;
+        const float* ni = a.norms + I.k_off;
+        float4 xv[8];
+#pragma unroll
+        for (int u = 0; u < 8; u++)
+            xv[u] = 16 * u < d ? *reinterpret_cast<const float4*>(xr + 16 * u + 4 * q) : make_float4(0, 0, 0, 0);
+        float best = inf;
+        uint32_t lab = 0;
+        for (int j0 = 0; j0 < k; j0 += 128) {  // this quad: centroids j0 + g and j0 + 64 + g
+            float p[2][4];
+#pragma unroll
+            for (int h = 0; h < 2; h++) {
+                const float* cj = ci + (size_t)min(j0 + 64 * h + g, k - 1) * d + 4 * q;
+#pragma unroll
+                for (int t = 0; t < 4; t++) p[h][t] = 0.0f;
+#pragma unroll
+                for (int u = 0; u < 8; u++) {
+                    if (16 * u < d) {
+                        const float4 cv = *reinterpret_cast<const float4*>(cj + 16 * u);
+                        p[h][0] = __fmaf_rn(xv[u].x, cv.x, p[h][0]);
+                        p[h][1] = __fmaf_rn(xv[u].y, cv.y, p[h][1]);
+                        p[h][2] = __fmaf_rn(xv[u].z, cv.z, p[h][2]);
+                        p[h][3] = __fmaf_rn(xv[u].w, cv.w, p[h][3]);
+                    }
+                }
+            }
+#pragma unroll
+            for (int h = 0; h < 2; h++) {
+#pragma unroll
+                for (int t = 0; t < 4; t++) p[h][t] = __fadd_rn(p[h][t], __shfl_xor_sync(kFull, p[h][t], 2));
+#pragma unroll
+                for (int t = 0; t < 4; t++) p[h][t] = __fadd_rn(p[h][t], __shfl_xor_sync(kFull, p[h][t], 1));
+                const int j = j0 + 64 * h + g;
+                if (j < k) {
+                    const float sc =
+                        score_ref(ni[j], __fadd_rn(__fadd_rn(p[h][0], p[h][2]), __fadd_rn(p[h][1], p[h][3])));
+                    if (sc < best) {  // a quad's centroids ascend
+                        best = sc;
+                        lab = (uint32_t)j;
+                    }
+                }
+            }
+        }
+        for (int o = 4; o < 32; o <<= 1) {
             const float ob = __shfl_xor_sync(kFull, best, o);
             const uint32_t ol = __shfl_xor_sync(kFull, lab, o);
             if (ob < inf && (!(best < inf) || lex_less(ob, ol, best, lab))) {
@@ -713,65 +955,47 @@ __global__ void k_b_certify(const T* __restrict__ x, BArgs a) {
     }
 }
 
-// Exhaustive exact search of the listed rows (one warp per row): the reference's
-// strict-< scan over ascending centroids, lowest index on ties, as
-// k_research_cta; a group that never beats +inf reports (inf, 0).
-template <typename T>
-__global__ void k_b_research(const T* __restrict__ x, BArgs a) {
-    const int lane = threadIdx.x & 31;
-    const uint32_t n = a.ctl->redo;
-    const int gsz = a.match == kMatchAvx512 ? 16 : 8, gpw = 32 / gsz, g = lane / gsz;
-    const int d = a.d;
-    for (uint32_t r = (blockIdx.x * blockDim.x + threadIdx.x) >> 5; r < n; r += (gridDim.x * blockDim.x) >> 5) {
-        const uint32_t e = a.redo_list[r];
-        const int i = (int)(e >> 24), row = (int)(e & 0xFFFFFFu);
-        BStep st;
-        b_active(a, i, &st);
-        const BInst& I = a.inst[i];
-        const int k = (int)I.k;
-        const T* xr = x + (I.row0 + b_rows(a, I, st)[row]) * (size_t)d;
-        const float* ci = a.c + I.c_off;
-        const float* ni = a.norms + I.k_off;
-        float best = __int_as_float(0x7f800000);
-        uint32_t lab = 0;
-        for (int j0 = 0; j0 < k; j0 += gpw) {
-            const int j = j0 + g, jc = j < k ? j : k - 1;
-            const float dj = group_dot_ref(a.match, xr, ci + (size_t)jc * d, d, lane);
-            if (j < k) {
-                const float s = score_ref(ni[j], dj);
-                if (s < best) {
-                    best = s;
-                    lab = (uint32_t)j;
-                }
-            }
-        }
-        if (!(best < __int_as_float(0x7f800000))) lab = 0;
-        // Merge the groups of the warp: lowest (score, index), finite scores only.
-        for (int o = gsz; o < 32; o <<= 1) {
-            const float ob = __shfl_xor_sync(kFull, best, o);
-            const uint32_t ol = __shfl_xor_sync(kFull, lab, o);
-            if (ob < __int_as_float(0x7f800000) && (!(best < __int_as_float(0x7f800000)) || lex_less(ob, ol, best, lab))) {
-                best = ob;
-                lab = ol;
-            }
-        }
-        const float xn = warp_sqnorm_ref(xr, d, lane);
-        if (lane == 0) {
-            a.blabels[I.b_off + row] = lab;
-            a.bdist[I.b_off + row] = fmaxf(__fadd_rn(best, xn), 0.0f);
-        }
-    }
-}
-
-// counts[l]++ per batch row, slot = arrival order within the label.
-// Grid (ceil(max batch / 256), count).
-__global__ void k_b_hist(BArgs a) {
+// What follows a step's search and needs only labels and distances, in one launch
+// (k_batch_tail for every instance). Blocks x > 0: counts[l]++ per batch row, slot =
+// arrival order within the label, on the last pass the row's label (src/lib.rs:438-440).
+// Block x = 0: the batch objective (src/lib.rs:442-445), the same fixed-shape f64 tree.
+// Grid (1 + ceil(max batch / 1024), count).
+__global__ void __launch_bounds__(1024) k_b_tail(BArgs a) {
     const int i = blockIdx.y;
     BStep st;
     if (!b_active(a, i, &st)) return;
     const BInst& I = a.inst[i];
-    const int r = blockIdx.x * blockDim.x + threadIdx.x;
-    if (r < (int)st.bn) a.slot[I.b_off + r] = atomicAdd(&a.counts[I.k_off + a.blabels[I.b_off + r]], 1u);
+    if (blockIdx.x > 0) {
+        const int r = (blockIdx.x - 1) * 1024 + threadIdx.x;
+        if (r < (int)st.bn) {
+            const uint32_t l = a.blabels[I.b_off + r];
+            a.slot[I.b_off + r] = atomicAdd(&a.counts[I.k_off + l], 1u);
+            if (st.last) a.labels_all[I.n_off + b_rows(a, I, st)[r]] = l;
+        }
+        return;
+    }
+    __shared__ double part[1024];
+    double s = 0.0;
+    for (int r = threadIdx.x; r < (int)st.bn; r += 1024) s += (double)a.bdist[I.b_off + r];
+    part[threadIdx.x] = s;
+    __syncthreads();
+    for (int o = 512; o > 0; o >>= 1) {
+        if (threadIdx.x < o) part[threadIdx.x] += part[threadIdx.x + o];
+        __syncthreads();
+    }
+    if (threadIdx.x == 0) a.obj[I.obj_off + st.epoch] += part[0];
+}
+
+// k_b_scan and k_b_scatter in one launch (largest k <= kScanScatterMaxK), as
+// k_scan_scatter. Grid (ceil(max batch / 1024), count).
+__global__ void __launch_bounds__(1024) k_b_scan_scatter(BArgs a) {
+    const int i = blockIdx.y;
+    BStep st;
+    if (!b_active(a, i, &st)) return;
+    const BInst& I = a.inst[i];
+    if (blockIdx.x * 1024 >= st.bn) return;
+    scan_scatter_cta(a.counts + I.k_off, (int)I.k, a.blabels + I.b_off, a.slot + I.b_off, (int)st.bn,
+                     a.offsets + I.k_off, a.list + I.b_off);
 }
 
 // Exclusive prefix sum of each instance's counts (one CTA of 1024 per instance).
@@ -812,8 +1036,9 @@ __global__ void k_b_scatter(BArgs a) {
         a.list[I.b_off + a.offsets[I.k_off + a.blabels[I.b_off + r]] + a.slot[I.b_off + r]] = (uint32_t)r;
 }
 
-// Per-cluster sums in row order, last-pass sums (one warp per cluster, the
-// single-instance segment_sums_warp). Grid (ceil(kmax / 8), count).
+// Per-cluster sums in row order, last-pass sums, and the EMA step of the cluster
+// (src/lib.rs:455-456): one warp per cluster, the single-instance segment_sums_warp and
+// apply_warp (the lane that wrote a dimension's sum reads it). Grid (ceil(kmax / 8), count).
 template <typename T, int MAXG>
 __global__ void k_b_segsums(const T* __restrict__ x, BArgs a, int R) {
     extern __shared__ float seg_stage[];  // R > 0: (blockDim / 32) x 2 R d floats
@@ -824,53 +1049,14 @@ __global__ void k_b_segsums(const T* __restrict__ x, BArgs a, int R) {
     const int l = (blockIdx.x * blockDim.x + threadIdx.x) >> 5, lane = threadIdx.x & 31;
     if (l >= (int)I.k) return;
     const uint32_t c = a.counts[I.k_off + l];
-    if (c == 0) return;
     const uint32_t off = a.offsets[I.k_off + l];
-    segment_sums_warp<T, MAXG>(x + I.row0 * (size_t)a.d, b_rows(a, I, st), a.d, l, c, a.list + I.b_off + off,
+    if (c > 0)
+        segment_sums_warp<T, MAXG>(x + I.row0 * (size_t)a.d, b_rows(a, I, st), a.d, l, c, a.list + I.b_off + off,
                                a.scratch + 2 * ((size_t)I.b_off + off), a.sums + I.c_off, (int)st.last,
                                a.pass_counts + I.k_off, a.pass_sums ? a.pass_sums + I.c_off : nullptr,
                                a.pass_sums64 ? a.pass_sums64 + I.c_off : nullptr, lane,
                                R ? seg_stage + (size_t)(threadIdx.x >> 5) * 2 * R * a.d : nullptr, R);
-}
-
-// Last pass: the row's label (src/lib.rs:438-440).
-__global__ void k_b_store_labels(BArgs a) {
-    const int i = blockIdx.y;
-    BStep st;
-    if (!b_active(a, i, &st) || !st.last) return;
-    const BInst& I = a.inst[i];
-    const int r = blockIdx.x * blockDim.x + threadIdx.x;
-    if (r < (int)st.bn) a.labels_all[I.n_off + b_rows(a, I, st)[r]] = a.blabels[I.b_off + r];
-}
-
-// Batch objective (src/lib.rs:442-445), the same fixed-shape f64 tree as
-// k_batch_objective. One CTA of 1024 per instance.
-__global__ void __launch_bounds__(1024) k_b_objective(BArgs a) {
-    __shared__ double part[1024];
-    const int i = blockIdx.x;
-    BStep st;
-    if (!b_active(a, i, &st)) return;
-    const BInst& I = a.inst[i];
-    double s = 0.0;
-    for (int r = threadIdx.x; r < (int)st.bn; r += 1024) s += (double)a.bdist[I.b_off + r];
-    part[threadIdx.x] = s;
-    __syncthreads();
-    for (int o = 512; o > 0; o >>= 1) {
-        if (threadIdx.x < o) part[threadIdx.x] += part[threadIdx.x + o];
-        __syncthreads();
-    }
-    if (threadIdx.x == 0) a.obj[I.obj_off + st.epoch] += part[0];
-}
-
-// EMA step (src/lib.rs:455-456), one warp per cluster. Grid (ceil(kmax / 8), count).
-__global__ void k_b_apply(BArgs a) {
-    const int i = blockIdx.y;
-    BStep st;
-    if (!b_active(a, i, &st)) return;
-    const BInst& I = a.inst[i];
-    const int j = (blockIdx.x * blockDim.x + threadIdx.x) >> 5, lane = threadIdx.x & 31;
-    if (j >= (int)I.k) return;
-    apply_warp(j, a.d, a.alphas[I.step_off + a.ctl->gstep], a.c + I.c_off, a.usage + I.k_off, a.counts + I.k_off,
+    apply_warp(l, a.d, a.alphas[I.step_off + a.ctl->gstep], a.c + I.c_off, a.usage + I.k_off, a.counts + I.k_off,
                a.sums + I.c_off, lane);
 }
 

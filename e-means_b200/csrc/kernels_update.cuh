@@ -60,10 +60,9 @@ __global__ void k_label_scatter(const uint32_t* __restrict__ labels, const uint3
 // less than the launch it saves) and places its own rows; block 0 keeps the offsets.
 // 6 -> 3 us a batch with the gap between them.
 constexpr int kScanScatterMaxK = 8192;
-__global__ void __launch_bounds__(1024) k_scan_scatter(const uint32_t* __restrict__ counts, int k,
-                                                       const uint32_t* __restrict__ labels,
-                                                       const uint32_t* __restrict__ slot, int m,
-                                                       uint32_t* __restrict__ offsets, uint32_t* __restrict__ list) {
+EMB_DEV void scan_scatter_cta(const uint32_t* __restrict__ counts, int k, const uint32_t* __restrict__ labels,
+                              const uint32_t* __restrict__ slot, int m, uint32_t* __restrict__ offsets,
+                              uint32_t* __restrict__ list) {
     __shared__ uint32_t off_s[kScanScatterMaxK];
     __shared__ uint32_t wsum[32];
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
@@ -102,6 +101,13 @@ __global__ void __launch_bounds__(1024) k_scan_scatter(const uint32_t* __restric
     __syncthreads();
     const int i = blockIdx.x * 1024 + tid;
     if (i < m) list[off_s[labels[i]] + slot[i]] = (uint32_t)i;
+}
+
+__global__ void __launch_bounds__(1024) k_scan_scatter(const uint32_t* __restrict__ counts, int k,
+                                                       const uint32_t* __restrict__ labels,
+                                                       const uint32_t* __restrict__ slot, int m,
+                                                       uint32_t* __restrict__ offsets, uint32_t* __restrict__ list) {
+    scan_scatter_cta(counts, k, labels, slot, m, offsets, list);
 }
 
 // Bitonic sort of E * 32 entries held E per lane (entry lane + 32 h in v[h]),

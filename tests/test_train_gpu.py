@@ -324,3 +324,42 @@ def test_update_kernels_cluster_sizes(emb, orc, n, d, k, closing_f64):
         a.close()
         assert np.array_equal(f64.labels, ref["labels"]) and f64.n_splits == ref["n_splits"]
         np.testing.assert_allclose(f64.centroids, ref["centroids"], rtol=2e-5, atol=2e-5)
+
+
+@pytest.mark.parametrize("variant", [9, 10])
+@pytest.mark.parametrize("d", [4, 16, 64, 100, 128])
+def test_lockstep_wide_tile_search(emb, monkeypatch, d, variant):
+    # The 128 x 128 resident-row search forced, with k below, at and above its tile, rows
+    # that many centroids tie for (coincident blobs: the exhaustive search of the listed
+    # rows, in its four-thread form where d is a multiple of 16), a short last batch.
+    monkeypatch.setenv("EMB200_BATCHED_SEARCH_VARIANT", str(variant))
+    sizes, ks = [3000, 1000, 9000, 129], [128, 5, 300, 129]
+    parts, x, inst = _uneven_instances(emb, d, sizes, ks, 40 + d)
+    x[:600] = x[0]
+    x[4000:5000] = np.round(x[4000:5000])
+    cfg = emb.Config(nepochs=2.0, batch_size=1500)
+    a = emb.B200Assigner(0, precision="fp32")
+    a.load_rows(x)
+    outs = a.train_batched(inst, cfg)
+    a.close()
+    for (r0, n, k), o in zip(inst, outs):
+        b = emb.B200Assigner(0, precision="fp32")
+        s = emb.train(np.ascontiguousarray(x[r0:r0 + n]), d, k, cfg, assigner=b)
+        b.close()
+        assert np.array_equal(o.labels, s.labels) and same_f32(o.centroids, s.centroids) and o.n_splits == s.n_splits
+
+
+def test_lockstep_more_clusters_than_one_scan_block(emb):
+    # k above the one-launch scan's limit for one of the instances
+    sizes, ks = [30000, 700], [9000, 20]
+    parts, x, inst = _uneven_instances(emb, 20, sizes, ks, 5)
+    cfg = emb.Config(nepochs=1.0)
+    a = emb.B200Assigner(0, precision="fp32")
+    a.load_rows(x)
+    outs = a.train_batched(inst, cfg)
+    a.close()
+    for p, (_, n, k), o in zip(parts, inst, outs):
+        b = emb.B200Assigner(0, precision="fp32")
+        s = emb.train(p, 20, k, cfg, assigner=b)
+        b.close()
+        assert np.array_equal(o.labels, s.labels) and same_f32(o.centroids, s.centroids)
