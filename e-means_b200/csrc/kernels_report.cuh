@@ -606,11 +606,13 @@ __global__ void __launch_bounds__(kPairThreads, 2) k_rep_pairs(const float* __re
 // The pair pass above spends 3 FP32 operations on each of the k^2 d / 2 terms to
 // keep the reference's rounding, although a row needs it for a few partners only.
 // Here the three-term BF16 search (k_assign_tc) scores every pair approximately,
-// collects per row each partner that the bound below cannot rule out, and only those
-// are evaluated in the reference's rounding (k_pair_exact); a row whose list overflows,
-// or holds no partner, is scanned exactly (k_pair_scan). k = 16384, d = 128: 3.43 +
-// 3.26 ms for the two passes, 0.33 + 0.82 ms here (the second keeps about 50
-// partners a row).
+// collects each partner that the bound below cannot rule out, and only those are
+// evaluated in the reference's rounding: the nearest centroid's as a short list per row
+// (k_pair_exact; a row whose list overflows, or holds no partner, is scanned exactly by
+// k_pair_scan), the radius test's as the bits of the adjacency itself, which
+// k_pair_verify thins out in place. k = 16384, d = 128: 3.43 + 3.26 ms for the two
+// passes, 0.31 + 0.39 ms here (the second with about 50 partners a row; as lists filled
+// by atomics it took 0.82).
 //
 // Bound. With s(j) the reference's squared distance of i and j, S(j) the exact one and
 // a(j) = |c_j|^2 - 2 c_i . c_j approximated: a(j) is within E1 = ka |c_i| cmax + kb nmax
@@ -622,10 +624,10 @@ __global__ void __launch_bounds__(kPairThreads, 2) k_rep_pairs(const float* __re
 //    smallest or the smallest is a partner nearer than it), the nearest partner has
 //    a <= v + 2 E.
 //  * radius r: s(j) <= r^2 (1 + 2^-20) is necessary for sqrt(s(j)) <= r, so
-//    a(j) <= r^2 (1 + 2^-20) - |c_i|^2 + E.
+//    a(j) <= r^2 (1 + 2^-20) - |c_i|^2 + E. Where that is not finite, or a column's score
+//    may be NaN (a centroid with a non-finite element), the exact pass runs instead.
 
-constexpr int kPairNearCap = 32;   // partners kept per row
-constexpr int kPairAdjCap = 256;
+constexpr int kPairNearCap = 32;  // partners kept per row
 
 // Scoring norms: the dead clusters' never pass a threshold.
 __global__ void k_pair_mask(const float* __restrict__ norms, const uint32_t* __restrict__ start, uint32_t k,
@@ -660,13 +662,15 @@ __global__ void k_pair_theta_near(const float* __restrict__ part_s, int nsplit, 
 
 __global__ void k_pair_theta_adj(const uint32_t* __restrict__ start, uint32_t k, const float* __restrict__ norms,
                                  const Bounds* __restrict__ bounds, const RepScalars* __restrict__ sc, float ka, float kb,
-                                 float* __restrict__ theta) {
+                                 float* __restrict__ theta, uint32_t* __restrict__ unusable) {
     const uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
     if (i >= k) return;
     const float r2 = __fmul_ru(__fmul_ru(sc->radius, sc->radius), 1.0f + 0x1p-20f);
     const float E = pair_bound(norms[i], *bounds, ka, kb);
     const float t = __fadd_ru(__fadd_ru(__fsub_ru(r2, norms[i]), E), __fmul_ru(0x1p-18f, r2));
-    theta[i] = start[i + 1] > start[i] && isfinite(t) ? t : __int_as_float(0x7fc00000);
+    const bool live = start[i + 1] > start[i];
+    theta[i] = live ? t : __int_as_float(0x7fc00000);
+    if (live && !isfinite(t)) *unusable = 1u;
 }
 
 // The reference's squared distance (as k_rep_pairs) by 16 lanes of a half-warp; both
@@ -690,21 +694,17 @@ EMB_DEV float half_sqdist_ref(const float* __restrict__ x, const float* __restri
 }
 
 // The collected partners of one row (a warp each, two at a time) in the reference's
-// rounding. Nearest: near_key[i] = min of (bits of s, j). ADJ: the row's adjacency
-// bits (zero before). Rows that the lists do not settle go to `rest`.
-template <bool ADJ>
+// rounding: near_key[i] = min of (bits of s, j). Rows that the lists do not settle go
+// to `rest`.
 __global__ void __launch_bounds__(256) k_pair_exact(const float* __restrict__ c, uint32_t k, uint32_t d,
                                                     const uint32_t* __restrict__ start,
                                                     const uint32_t* __restrict__ cand,
                                                     const uint32_t* __restrict__ cand_count, uint32_t cap,
                                                     const int* __restrict__ err, unsigned long long* __restrict__ near_key,
-                                                    const RepScalars* __restrict__ sc, uint32_t* __restrict__ adj,
-                                                    uint32_t words, uint32_t* __restrict__ rest,
-                                                    uint32_t* __restrict__ rest_count) {
+                                                    uint32_t* __restrict__ rest, uint32_t* __restrict__ rest_count) {
     const uint32_t i = (blockIdx.x * blockDim.x + threadIdx.x) >> 5;
     const int lane = threadIdx.x & 31;
     if (i >= k) return;
-    if (ADJ && start[i + 1] == start[i]) return;  // dead: no neighbours
     const uint32_t cnt = cand_count[i];
     unsigned long long best = ~0ull;
     const bool listed = cnt > 0 && cnt <= cap && !*err;
@@ -715,28 +715,115 @@ __global__ void __launch_bounds__(256) k_pair_exact(const float* __restrict__ c,
             const uint32_t j = cand[(size_t)i * cap + (q < cnt ? q : e)];
             const float s = half_sqdist_ref(ci, c + (size_t)j * d, d, lane);
             const bool partner = q < cnt && j != i && start[j + 1] > start[j];
-            if (ADJ) {
-                if (partner && (lane & 15) == 0 && __fsqrt_rn(s) <= sc->radius)
-                    atomicOr(&adj[(size_t)i * words + (j >> 5)], 1u << (j & 31));
-            } else if (partner && s < INFINITY) {
-                best = min(best, ((unsigned long long)__float_as_uint(s) << 32) | j);
-            }
+            if (partner && s < INFINITY) best = min(best, ((unsigned long long)__float_as_uint(s) << 32) | j);
         }
     }
-    if (!ADJ) best = min(best, __shfl_xor_sync(0xffffffffu, best, 16));
+    best = min(best, __shfl_xor_sync(0xffffffffu, best, 16));
     if (lane == 0) {
-        if (!ADJ && best != ~0ull) near_key[i] = best;
-        if (!listed || (!ADJ && best == ~0ull)) rest[atomicAdd(rest_count, 1u)] = i;
+        if (best != ~0ull) near_key[i] = best;
+        else rest[atomicAdd(rest_count, 1u)] = i;
     }
 }
 
+// The adjacency of one live row (a warp each) from its candidate bits, in place: the
+// bits' columns go through a list in shared memory, eight pairs at a time are evaluated
+// in the reference's rounding (four threads each, thread q the lanes 4q .. 4q + 3), and
+// the bits whose pair is within the radius are set again. vec: 16-byte aligned rows.
+constexpr int kPairList = 256;
+__global__ void __launch_bounds__(256) k_pair_verify(const float* __restrict__ c, uint32_t k, uint32_t d,
+                                                     const uint32_t* __restrict__ start,
+                                                     const RepScalars* __restrict__ sc, uint32_t* __restrict__ adj,
+                                                     uint32_t words, bool vec) {
+    __shared__ uint32_t list_s[8][kPairList];
+    const uint32_t i = (blockIdx.x * blockDim.x + threadIdx.x) >> 5;
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, q = lane & 3, g = lane >> 2;
+    if (i >= k) return;
+    uint32_t* row = adj + (size_t)i * words;
+    const bool live = start[i + 1] > start[i];
+    const float radius = sc->radius;
+    const float* ci = c + (size_t)i * d;
+    const uint32_t d16 = d / 16 * 16;
+    uint32_t* list = list_s[warp];
+    uint32_t n = 0;
+    auto settle = [&]() {  // the listed columns
+        __syncwarp();
+        for (uint32_t e0 = 0; e0 < n; e0 += 8) {
+            const bool have = e0 + g < n;
+            const uint32_t j = list[have ? e0 + g : 0];
+            const float* cj = c + (size_t)j * d;
+            float a[4] = {0.0f, 0.0f, 0.0f, 0.0f};
+            for (uint32_t t = 4 * q; t < d16; t += 16) {
+                float xv[4], yv[4];
+                if (vec) {
+                    const float4 x4 = *reinterpret_cast<const float4*>(ci + t), y4 = *reinterpret_cast<const float4*>(cj + t);
+                    xv[0] = x4.x; xv[1] = x4.y; xv[2] = x4.z; xv[3] = x4.w;
+                    yv[0] = y4.x; yv[1] = y4.y; yv[2] = y4.z; yv[3] = y4.w;
+                } else {
+#pragma unroll
+                    for (int u = 0; u < 4; u++) {
+                        xv[u] = ci[t + u];
+                        yv[u] = cj[t + u];
+                    }
+                }
+#pragma unroll
+                for (int u = 0; u < 4; u++) {
+                    const float w = __fsub_rn(xv[u], yv[u]);
+                    a[u] = __fadd_rn(a[u], __fmul_rn(w, w));
+                }
+            }
+            // the 16 lanes in order: each thread of the quad adds its four to the sum so far
+            float s = __fadd_rn(__fadd_rn(__fadd_rn(a[0], a[1]), a[2]), a[3]);
+#pragma unroll
+            for (int p = 1; p < 4; p++) {
+                const float before = __shfl_sync(0xffffffffu, s, (lane & ~3) + p - 1);
+                if (q == p) s = __fadd_rn(__fadd_rn(__fadd_rn(__fadd_rn(before, a[0]), a[1]), a[2]), a[3]);
+            }
+            float tail = 0.0f;
+            for (uint32_t t = d16; t < d; t++) {
+                const float w = __fsub_rn(ci[t], cj[t]);
+                tail = __fadd_rn(tail, __fmul_rn(w, w));
+            }
+            s = __fadd_rn(s, tail);
+            if (have && q == 3 && start[j + 1] > start[j] && __fsqrt_rn(s) <= radius)
+                atomicOr(&row[j >> 5], 1u << (j & 31));
+        }
+        n = 0;
+        __syncwarp();
+    };
+    for (uint32_t w0 = 0; w0 < words; w0 += 32) {
+        const uint32_t w = w0 + lane;
+        uint32_t m = w < words && live ? row[w] : 0u;
+        if (w == (i >> 5)) m &= ~(1u << (i & 31));  // not its own neighbour
+        if (w < words) row[w] = 0u;
+        while (__any_sync(0xffffffffu, m != 0u)) {
+            const unsigned has = __ballot_sync(0xffffffffu, m != 0u);
+            if (m) {
+                const int b = __ffs((int)m) - 1;
+                m &= m - 1;
+                list[n + __popc(has & ((1u << lane) - 1u))] = w * 32 + b;
+            }
+            n += (uint32_t)__popc(has);
+            if (n + 32 > kPairList) settle();  // (a word's cleared store precedes its bits' atomics)
+        }
+    }
+    settle();
+}
+
+// Candidate pairs in the bitset (to choose between evaluating them and the exact pass).
+__global__ void __launch_bounds__(256) k_pair_count(const uint32_t* __restrict__ adj, size_t nwords,
+                                                    unsigned long long* __restrict__ total) {
+    unsigned long long s = 0;
+    for (size_t i = (size_t)blockIdx.x * blockDim.x + threadIdx.x; i < nwords; i += (size_t)gridDim.x * blockDim.x)
+        s += (unsigned long long)__popc(adj[i]);
+    for (int o = 16; o; o >>= 1) s += __shfl_xor_sync(0xffffffffu, s, o);
+    if ((threadIdx.x & 31) == 0 && s) atomicAdd(total, s);
+}
+
 // The rows of `rest` against every live partner, a CTA per row.
-template <bool ADJ>
 __global__ void __launch_bounds__(256) k_pair_scan(const float* __restrict__ c, uint32_t k, uint32_t d,
                                                    const uint32_t* __restrict__ start,
                                                    unsigned long long* __restrict__ near_key,
-                                                   const RepScalars* __restrict__ sc, uint32_t* __restrict__ adj,
-                                                   uint32_t words, const uint32_t* __restrict__ rest,
+                                                   const uint32_t* __restrict__ rest,
                                                    const uint32_t* __restrict__ rest_count) {
     const int lane = threadIdx.x & 31, half = threadIdx.x >> 4;
     for (uint32_t r = blockIdx.x; r < *rest_count; r += gridDim.x) {
@@ -747,17 +834,10 @@ __global__ void __launch_bounds__(256) k_pair_scan(const float* __restrict__ c, 
             const uint32_t j = j0 + half, jc = j < k ? j : k - 1;
             const float s = half_sqdist_ref(ci, c + (size_t)jc * d, d, lane);
             if (j >= k || j == i || start[j + 1] == start[j]) continue;  // no shuffles follow in this round
-            if (ADJ) {
-                if ((lane & 15) == 0 && __fsqrt_rn(s) <= sc->radius)
-                    atomicOr(&adj[(size_t)i * words + (j >> 5)], 1u << (j & 31));
-            } else if (s < INFINITY) {
-                best = min(best, ((unsigned long long)__float_as_uint(s) << 32) | j);
-            }
+            if (s < INFINITY) best = min(best, ((unsigned long long)__float_as_uint(s) << 32) | j);
         }
-        if (!ADJ) {
-            best = min(best, __shfl_xor_sync(0xffffffffu, best, 16));
-            if (lane == 0 && best != ~0ull) atomicMin(&near_key[i], best);
-        }
+        best = min(best, __shfl_xor_sync(0xffffffffu, best, 16));
+        if (lane == 0 && best != ~0ull) atomicMin(&near_key[i], best);
     }
 }
 
@@ -927,48 +1007,58 @@ __global__ void k_rep_nbrs(const unsigned long long* __restrict__ order, uint32_
     }
 }
 
-// One CTA: the rounds above on a status byte per position in shared memory
-// (dynamic: live bytes), then each position's family: its own (leader) or that
-// of its earliest leader neighbour. Families are numbered by their leaders'
-// positions, which is the greedy pass's order of formation. fam_size must be
-// zero on entry.
-__global__ void __launch_bounds__(1024) k_rep_lfmis(const unsigned long long* __restrict__ order, uint32_t live,
-                                                    const uint32_t* __restrict__ eoff,
-                                                    const uint32_t* __restrict__ nbr,
-                                                    const uint32_t* __restrict__ start,
-                                                    uint32_t* __restrict__ fidx, uint32_t* __restrict__ fam_of,
-                                                    uint32_t* __restrict__ fam_lead,
-                                                    unsigned long long* __restrict__ fam_size,
-                                                    uint32_t* __restrict__ nfam) {
+// One round over the undecided positions, by the whole grid. Statuses only ever go from
+// undecided to final, so a neighbour's status read before or after its own decision of
+// this round leads to a valid decision either way.
+EMB_DEV uint8_t fam_decide(uint32_t q, const uint32_t* __restrict__ eoff, const uint32_t* __restrict__ nbr,
+                           const volatile uint8_t* status) {
+    bool all_decided = true;
+    for (uint32_t e = eoff[q]; e < eoff[q + 1]; e++) {
+        const uint8_t st = status[nbr[e]];
+        if (st == kFamLeader) return kFamFollower;
+        if (st == kFamUndecided) all_decided = false;
+    }
+    return all_decided ? kFamLeader : kFamUndecided;
+}
+__global__ void __launch_bounds__(256) k_fam_round(uint32_t live, const uint32_t* __restrict__ eoff,
+                                                   const uint32_t* __restrict__ nbr, volatile uint8_t* status) {
+    const uint32_t q = (blockIdx.x * blockDim.x + threadIdx.x) >> 5;  // a warp per position
+    const int lane = threadIdx.x & 31;
+    if (q >= live || status[q] != kFamUndecided) return;
+    bool open = false;
+    const uint32_t end = eoff[q + 1];
+    for (uint32_t e0 = eoff[q]; e0 < end; e0 += 32) {
+        const uint8_t st = e0 + lane < end ? status[nbr[e0 + lane]] : (uint8_t)kFamFollower;
+        if (__any_sync(0xffffffffu, st == kFamLeader)) {
+            if (lane == 0) status[q] = kFamFollower;
+            return;
+        }
+        open |= __any_sync(0xffffffffu, st == kFamUndecided);
+    }
+    if (!open && lane == 0) status[q] = kFamLeader;
+}
+
+// The rounds that are left (usually none), in one CTA with the statuses in shared memory,
+// and the family number of each leader: leaders before it in position order.
+__global__ void __launch_bounds__(1024) k_fam_number(uint32_t live, const uint32_t* __restrict__ eoff,
+                                                     const uint32_t* __restrict__ nbr, uint8_t* __restrict__ status_g,
+                                                     uint32_t* __restrict__ fidx, uint32_t* __restrict__ nfam) {
     extern __shared__ uint8_t status[];
     __shared__ uint32_t ws[32];
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
-    for (uint32_t q = tid; q < live; q += 1024) status[q] = kFamUndecided;
+    for (uint32_t q = tid; q < live; q += 1024) status[q] = status_g[q];
     __syncthreads();
     for (uint32_t round = 0; round <= live; round++) {
         int open = 0;
         for (uint32_t q = tid; q < live; q += 1024) {
             if (status[q] != kFamUndecided) continue;
-            bool leader_seen = false, all_decided = true;
-            for (uint32_t e = eoff[q]; e < eoff[q + 1]; e++) {
-                const uint8_t st = status[nbr[e]];
-                if (st == kFamLeader) {
-                    leader_seen = true;
-                    break;
-                }
-                if (st == kFamUndecided) all_decided = false;
-            }
-            if (leader_seen) status[q] = kFamFollower;
-            else if (all_decided) status[q] = kFamLeader;
+            const uint8_t st = fam_decide(q, eoff, nbr, status);
+            if (st != kFamUndecided) status[q] = st;
             else open = 1;
         }
         if (!__syncthreads_or(open)) break;
     }
     // (every round decides the earliest undecided position, so none is left here)
-    for (uint32_t q = tid; q < live; q += 1024)
-        if (status[q] == kFamUndecided) status[q] = kFamLeader;
-    __syncthreads();
-    // family number of each leader: leaders before it in position order
     uint32_t carry = 0;
     for (uint32_t b0 = 0; b0 < live; b0 += 1024) {
         const uint32_t q = b0 + tid;
@@ -976,32 +1066,41 @@ __global__ void __launch_bounds__(1024) k_rep_lfmis(const unsigned long long* __
         const unsigned bal = __ballot_sync(0xffffffffu, isl);
         if (lane == 0) ws[warp] = __popc(bal);
         __syncthreads();
-        uint32_t before = carry;
-        for (int w = 0; w < warp; w++) before += ws[w];
-        before += __popc(bal & ((1u << lane) - 1u));
-        if (isl) fidx[q] = before;
-        uint32_t tot = 0;
-        for (int w = 0; w < 32; w++) tot += ws[w];
+        uint32_t before = carry, tot = 0;
+        for (int w = 0; w < 32; w++) {
+            before += w < warp ? ws[w] : 0u;
+            tot += ws[w];
+        }
+        if (isl) fidx[q] = before + __popc(bal & ((1u << lane) - 1u));
+        if (q < live) status_g[q] = status[q];
         carry += tot;
         __syncthreads();
     }
     if (tid == 0) *nfam = carry;
-    __syncthreads();
-    for (uint32_t q = tid; q < live; q += 1024) {
-        uint32_t lq = q;
-        if (status[q] != kFamLeader) {
-            lq = 0xffffffffu;
-            for (uint32_t e = eoff[q]; e < eoff[q + 1]; e++) {
-                const uint32_t u = nbr[e];
-                if (status[u] == kFamLeader && u < lq) lq = u;
-            }
+}
+
+// Every cluster into the family of its earliest leading neighbour (or its own).
+__global__ void __launch_bounds__(256) k_fam_join(const unsigned long long* __restrict__ order, uint32_t live,
+                                                  const uint32_t* __restrict__ eoff, const uint32_t* __restrict__ nbr,
+                                                  const uint8_t* __restrict__ status, const uint32_t* __restrict__ start,
+                                                  const uint32_t* __restrict__ fidx, uint32_t* __restrict__ fam_of,
+                                                  uint32_t* __restrict__ fam_lead,
+                                                  unsigned long long* __restrict__ fam_size) {
+    const uint32_t q = blockIdx.x * blockDim.x + threadIdx.x;
+    if (q >= live) return;
+    uint32_t lq = q;
+    if (status[q] != kFamLeader) {
+        lq = 0xffffffffu;
+        for (uint32_t e = eoff[q]; e < eoff[q + 1]; e++) {
+            const uint32_t u = nbr[e];
+            if (status[u] == kFamLeader && u < lq) lq = u;
         }
-        const uint32_t f = fidx[lq];
-        const uint32_t v = (uint32_t)order[q];
-        fam_of[v] = f;
-        atomicAdd(&fam_size[f], (unsigned long long)(start[v + 1] - start[v]));
-        if (lq == q) fam_lead[f] = v;
     }
+    const uint32_t f = fidx[lq];
+    const uint32_t v = (uint32_t)order[q];
+    fam_of[v] = f;
+    atomicAdd(&fam_size[f], (unsigned long long)(start[v + 1] - start[v]));
+    if (lq == q) fam_lead[f] = v;
 }
 
 // Families renumbered by size, largest first (formation order among equals).

@@ -76,6 +76,8 @@ struct TcParams {
     uint32_t* cand;           // COLLECT: [m][cand_cap] centroid indices
     uint32_t* cand_count;     // COLLECT: [m] candidates found (may exceed cand_cap)
     int cand_cap;
+    uint32_t* bits;           // COLLECT: instead of the lists, bit col of row's `words` words (every word of
+    int words;                // the searched columns is written), by the one thread that scores the column
     const uint32_t* m_dev;    // COLLECT: if set, the row count is min(m, *m_dev), read on the device
     // Grouped search (k_assign_grouped, centroid groups of a group-sorted matrix):
     // bucket tile t scores columns [tile_info[t].x, + 128 tile_info[t].y) of its
@@ -1121,6 +1123,7 @@ k_assign_tc(const T* __restrict__ x, const __grid_constant__ CUtensorMap map_hi,
         const int r = q * 32 + lane;
         float* pub = (float*)(smem + L.pub);
         uint32_t* mg = (uint32_t*)(smem + L.merge);
+        const int m_live = m;
         int tg = 0;
         bool ok = true;
         for (int i = 0; i < my_items; i++) {
@@ -1225,6 +1228,18 @@ k_assign_tc(const T* __restrict__ x, const __grid_constant__ CUtensorMap map_hi,
                             }
                         }
                     }
+                } else if (p.bits) {
+                    uint32_t m[2] = {0u, 0u};
+#pragma unroll
+                    for (int h = 0; h < 4; h++)
+                        if (mnh[h] <= theta) {
+#pragma unroll
+                            for (int j = 0; j < 16; j++)
+                                if (sc4[h][j] <= theta && cb + h * 16 + j < p.k) m[h >> 1] |= 1u << ((h & 1) * 16 + j);
+                        }
+#pragma unroll
+                    for (int u = 0; u < 2; u++)
+                        if (row < m_live && (cb >> 5) + u < p.words) p.bits[(size_t)row * p.words + (cb >> 5) + u] = m[u];
                 } else {
 #pragma unroll
                     for (int h = 0; h < 4; h++) {
