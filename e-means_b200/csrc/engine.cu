@@ -37,6 +37,10 @@
 #include "kernels_batched.cuh"
 
 constexpr int kRefineCap = 32;  // candidates kept per refined row
+// A host call of so few rows gets its results with the counters, in one copy: labels and
+// distances on their own were two more copies of 10 us each and a wait (100 x 96 rows,
+// k = 1024: 92 -> 76 us a call).
+constexpr size_t kSmallHostRows = 4096, kCounters = 8;
 constexpr size_t kBlindMin = 2048, kBlindMax = 65536;  // rows of a search without a host read in its middle
 constexpr size_t kMaxSearchRows = (size_t)1 << 26;  // rows per search pass (32-bit row indexing inside)
 
@@ -239,7 +243,9 @@ struct emb200_handle {
     DevBuf<uint32_t> redo_rows;
     DevBuf<float> redo_theta;
     DevBuf<uint32_t> cand, cand_count, redo2_rows;  // refine pass
-    DevBuf<uint32_t> counters;  // see assign_rows_dev
+    DevBuf<uint32_t> counters;  // see assign_rows_dev; a small host call's results follow them
+    size_t small_rows = 0;      // rows of a small host call in progress (assign_host)
+    std::vector<uint32_t> small_host;  // counters, labels and distances of that call
     DevBuf<unsigned long long> rkeys;  // exhaustive search: per listed row (score, index) keys
     DevBuf<uint32_t> rdone;            // and the slices of its centroids scored so far
 
@@ -792,9 +798,22 @@ int launch_tc(emb200_handle* h, const T* x, const uint32_t* gather, const uint32
 }
 
 // The device counters of one pipeline run, and the fast kernel's time (waits for the stream).
+// A small host call's labels and distances come with them (kSmallHostRows).
+int copy_counters(emb200_handle* h, cudaStream_t st, uint32_t (&c)[5]) {
+    if (h->small_rows) {
+        CK(cudaMemcpyAsync(h->small_host.data(), h->counters.p, (kCounters + 2 * h->small_rows) * sizeof(uint32_t),
+                           cudaMemcpyDeviceToHost, st));
+        CK(cudaStreamSynchronize(st));
+        std::memcpy(c, h->small_host.data(), sizeof c);
+    } else {
+        CK(cudaMemcpyAsync(c, h->counters.p, sizeof c, cudaMemcpyDeviceToHost, st));
+        CK(cudaStreamSynchronize(st));
+    }
+    return EMB200_OK;
+}
 int read_counters(emb200_handle* h, cudaStream_t st, uint32_t (&c)[5]) {
-    CK(cudaMemcpyAsync(c, h->counters.p, sizeof c, cudaMemcpyDeviceToHost, st));
-    CK(cudaStreamSynchronize(st));
+    const int rc = copy_counters(h, st, c);
+    if (rc) return rc;
     float kms = 0.0f;
     CK(cudaEventElapsedTime(&kms, h->evk0, h->evk1));
     h->stats.fast_ms += kms;
@@ -1078,8 +1097,8 @@ int settle_rows(emb200_handle* h, const T* x, const uint32_t* gather, size_t m, 
     const int rc = launch_research(h, x, gather, nredo, !refine, exhaustive, exhaustive_count, h->rkeys.p, h->rdone.p,
                                    labels, dist, st);
     if (rc) return rc;
-    CK(cudaMemcpyAsync(c0, ctr, sizeof c0, cudaMemcpyDeviceToHost, st));
-    CK(cudaStreamSynchronize(st));
+    const int rc2 = copy_counters(h, st, c0);
+    if (rc2) return rc2;
     fold_counters(h, c0, exhaustive_count == ctr + 3);
     return EMB200_OK;
 }
@@ -1141,8 +1160,12 @@ int assign_host(emb200_handle* h, int dtype, const void* x, size_t m, uint32_t* 
     for (size_t r0 = 0; r0 < m; r0 += chunk) starts.push_back(r0);
     starts.push_back(m);
     const size_t nch = starts.size() - 1;
-    if (h->stage.ensure(2 * chunk * row_bytes) || h->st_labels.ensure(chunk) || h->st_dist.ensure(chunk))
+    const bool small = m > 0 && m <= kSmallHostRows && nch == 1 && !use_i8_mode(h, dtype);
+    if (h->stage.ensure(2 * chunk * row_bytes) ||
+        (small ? (bool)h->counters.ensure(kCounters + 2 * kSmallHostRows)
+               : h->st_labels.ensure(chunk) || h->st_dist.ensure(chunk)))
         return fail(h, EMB200_ENOMEM, "staging allocation failed");
+    if (small) h->small_host.resize(kCounters + 2 * m);
     auto stage_of = [&](size_t i) { return h->stage.p + (i & 1) * chunk * row_bytes; };
     auto copy_in = [&](size_t i) -> int {
         const size_t r0 = starts[i], mc = starts[i + 1] - r0;
@@ -1164,6 +1187,17 @@ int assign_host(emb200_handle* h, int dtype, const void* x, size_t m, uint32_t* 
             if (rc) return rc;
         }
         CK(cudaStreamWaitEvent(st, h->ev_copied[i & 1], 0));
+        if (small) {  // the search ends with a read of its counters: the results come along
+            h->small_rows = m;
+            rc = assign_dispatch(h, dtype, stage_of(i), nullptr, m, h->counters.p + kCounters,
+                                 (float*)(h->counters.p + kCounters + m), st);
+            h->small_rows = 0;
+            if (rc) return rc;
+            CK(cudaEventRecord(h->ev_done[i & 1], st));
+            std::memcpy(labels, h->small_host.data() + kCounters, m * sizeof(uint32_t));
+            std::memcpy(dist, h->small_host.data() + kCounters + m, m * sizeof(float));
+            break;
+        }
         rc = assign_dispatch(h, dtype, stage_of(i), nullptr, mc, h->st_labels.p, h->st_dist.p, st);
         if (rc) return rc;
         CK(cudaEventRecord(h->ev_done[i & 1], st));

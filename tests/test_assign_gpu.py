@@ -526,3 +526,24 @@ def test_single_term_operand_scale(emb, orc, assigners, case, m, k, d):
     assert st["fast_aborted"] == 0 and st["fast_kernel"] == 1
     if case in ("plain", "tiny", "huge"):  # the scale keeps the bound: nearly every row certified at once
         assert st["rows_refined"] < 0.02 * m, st
+
+
+@pytest.mark.parametrize("precision", ["fp32", "bf16", "bf16x1"])
+@pytest.mark.parametrize("m", [1, 2048, 2049, 4096, 4097])
+def test_small_host_calls(emb, orc, assigners, precision, m):
+    # Calls of up to 4096 rows get their results with the counters: rows certified at
+    # once and rows (exact ties) that go through the refine pass, dtypes in turn, on one
+    # handle between calls of other sizes.
+    rng = np.random.default_rng(m)
+    d, k = 40, 90
+    c = rng.integers(-9, 10, (k, d)).astype(np.float32)
+    c[50:] = c[:40]  # duplicated centroids: no margin
+    a = assigners(precision)
+    a.set_centroids(c)
+    for x in (rng.standard_normal((m, d)).astype(np.float32) * 6, c[rng.integers(0, k, m)],
+              rng.integers(-9, 10, (m, d)).astype(np.int8), rng.integers(0, 10, (2 * m, d)).astype(np.uint8)):
+        lab, dist = a.assign(x)
+        rl, rd = orc.cpu_assign(x, c, emulate=not orc.has_kernel("avx512"))
+        assert np.array_equal(lab, rl) and same_f32(dist, rd)
+        st = a.stats()
+        assert st["rows"] == len(x) and st["rows_certified"] + st["rows_refined"] == len(x)
