@@ -118,7 +118,10 @@ struct Scratch {
                 props.location.type = cudaMemLocationTypeDevice;
                 props.location.id = device;
                 cudaError_t e = cudaMemPoolCreate(&pool, &props);
-                if (e != cudaSuccess) return e;
+                if (e != cudaSuccess) {
+                    cudaGetLastError();
+                    return e;
+                }
                 uint64_t keep = kScratchKeep;
                 cudaMemPoolSetAttribute(pool, cudaMemPoolAttrReleaseThreshold, &keep);
                 s.pool[device] = pool;
@@ -126,7 +129,12 @@ struct Scratch {
                 pool = it->second;
             }
         }
-        return cudaMallocFromPoolAsync((void**)&p, std::max(bytes, (size_t)16), pool, st);
+        const cudaError_t e = cudaMallocFromPoolAsync((void**)&p, std::max(bytes, (size_t)16), pool, st);
+        if (e != cudaSuccess) {  // a caller may go on without: leave no error behind
+            p = nullptr;
+            cudaGetLastError();
+        }
+        return e;
     }
 };
 
@@ -868,7 +876,7 @@ int assign_rows_dev(emb200_handle* h, const T* x, const uint32_t* gather, size_t
         return launch_i8_assign(h, (const int8_t*)x, gather, m, labels, dist, st, graph);
     }
     int prec = h->opts.precision;
-    // FP8 operands for f32 rows when prepared (d <= 256); otherwise the single-term BF16 search.
+    // FP8 operands for f32 rows when prepared (d <= 256); otherwise the single-term search.
     const bool fp8 = prec == EMB200_PREC_FP8 && dtype == EMB200_F32 && tc_supported(h, 1, true);
     if (prec == EMB200_PREC_FP8 && !fp8) prec = EMB200_PREC_BF16X1;
     const int fast_terms = tc_terms(prec, dtype);
@@ -1011,21 +1019,21 @@ int settle_rows(emb200_handle* h, const T* x, const uint32_t* gather, size_t m, 
     // Batches of some size: the host does not wait for the uncertified rows' count
     // either. The read costs 12 us, the launches whose rows it would have spared 2 us
     // each; a few rows are usually all certified, many rows need the exact grids.
-    const bool blind = !graph && m > kBlindMin && m <= kBlindMax;
+    // Without room for all of them the search asks for the count after all.
+    Scratch scratch(h->device, st);
+    const bool blind = !graph && m > kBlindMin && m <= kBlindMax &&
+                       !scratch.alloc(m * ((kRefineCap + 3) * sizeof(uint32_t) + sizeof(unsigned long long)));
     if (graph || blind) {
         // No host reads: every later launch takes its row count from the device
         // counters (grids sized for all m rows, surplus CTAs leave at once).
         const uint32_t* exhaustive = h->redo_rows.p;
         const uint32_t* exhaustive_count = ctr;
         const int ntiles = (int)((h->k + kTcBN - 1) / kTcBN);
-        Scratch scratch(h->device, st);
         const int cap = kRefineCap;
         uint32_t *cand = nullptr, *cand_count = nullptr, *redo2 = nullptr, *done = nullptr;
         unsigned long long* keys = nullptr;
         const bool refine = tc_supported(h, refine_terms);
         if (blind) {  // room for all m rows, most of it untouched: from the shared pool
-            if (scratch.alloc(m * ((cap + 3) * sizeof(uint32_t) + sizeof *keys)))
-                return fail(h, EMB200_ENOMEM, "refine allocation failed for %zu rows", m);
             keys = (unsigned long long*)scratch.p;
             cand = (uint32_t*)(keys + m);
             cand_count = cand + m * cap;

@@ -9,7 +9,7 @@ namespace emb {
 
 constexpr unsigned kFull = 0xffffffffu;
 
-// Device-side bounds used by the certification (filled by k_prep_centroids / k_bias).
+// Device-side bounds used by the certification (filled by k_prep_centroids and k_prep_f16).
 struct Bounds {
     float cmax;  // >= max_j |c_j| (upper-rounded)
     float nmax;  // >= max_j |norms_j| (norms include the bias)

@@ -848,7 +848,7 @@ template <typename T, bool COLLECT, bool FP8, bool NM = false>
 __global__ void __launch_bounds__(kTcPThreads, 1)
 k_assign_tc(const T* __restrict__ x, const __grid_constant__ CUtensorMap map_hi,
             const __grid_constant__ CUtensorMap map_lo, const TcParams p) {
-    static_assert(!NM || (!COLLECT && !FP8), "norms in the contraction: single-term BF16 fast search only");
+    static_assert(!NM || (!COLLECT && !FP8), "norms in the contraction: single-term fast search only");
     extern __shared__ __align__(1024) uint8_t smem_raw[];
     uint8_t* smem = smem_align1024(smem_raw);
     const TcLayout L = tc_layout(p.kpad, p.nterms, FP8, NM);
