@@ -36,7 +36,7 @@ sys.path.insert(0, ROOT)
 N_ROWS, DIM, K = 1_000_000, 128, 16384
 WORKLOAD = "assign 1,000,000 x 128 f32 embedding rows (32-d latent, L2-normalised) to k=16384 trained centroids"
 METRIC = "rows/s assigned (1M x 128-D, k=16384)"
-DTYPES = {"fp32": "f32", "bf16": "bf16x3 (hi/lo split) -> f32 accumulate", "bf16x1": "bf16 -> f32 accumulate",
+DTYPES = {"fp32": "f32", "bf16": "bf16x3 (hi/lo split) -> f32 accumulate", "bf16x1": "fp16 (one power-of-two scale) -> f32 accumulate",
           "fp8": "e4m3 (power-of-two scale per row and per centroid) -> f32 accumulate"}
 CPU_SAMPLE_ROWS = 262_144
 
@@ -434,11 +434,10 @@ def run_c1(args):
     upd_gbs = ust["update_bytes"] / (ust["update_ms"] / 1e3) / 1e9
     line_update = {"bound": "hbm", "achieved": upd_gbs, "peak": hbm["hbm_gbs"], "unit": "GB/s",
                    "frac": upd_gbs / hbm["hbm_gbs"], "peak_note": f"hbm {hbm['source']}",
-                   "kernels": "k_label_hist, k_exclusive_scan, k_label_scatter, k_segment_sums, k_store_labels, "
-                              "k_batch_objective, k_apply, k_revive, k_step_incr (per batch)",
+                   "kernels": "k_batch_tail, k_scan_scatter, k_update_small, k_update_big, k_revive (per batch)",
                    "algorithmic_bytes": ust["update_bytes"], "device_ms": ust["update_ms"],
                    "training_device_ms_eager": ust["ms_total"],
-                   "note": "latency-bound: one warp sums a cluster's rows in row order (the reference's f32 order)"}
+                   "note": "latency-bound: each cluster's rows are added in row order (the reference's f32 order)"}
     line = {"metric": "e-means train + exact assign, 200k x 96, k=1024, 5 epochs (rows/s)", "value": rows / t,
             "unit": "rows/s", "n_gpus": 1, "steps": args.steps, "warmup": args.warmup, "ms_per_step": t * 1e3,
             "higher_is_better": True, "dtype": "bf16x3->f32 search, f32 update",
@@ -527,6 +526,7 @@ def run_c3(args):
     a = emb.B200Assigner(0, precision="fp32", centroid_bits=8)
     # f32 rows resident, then Int8Quantizer::fit and encode on the device (faiss calibration)
     a.load_rows(x)
+    emb.Int8Quantizer.fit_resident(a, emb.Calibration.faiss())  # untimed: first use loads the kernels
     t0 = time.perf_counter()
     q = emb.Int8Quantizer.fit_resident(a, emb.Calibration.faiss())
     t1 = time.perf_counter()
@@ -634,10 +634,9 @@ def run_report(args):
                        "live_clusters": live, "families": len(r.families)},
             "clocks": clock.summary(),
             "pair_pass": {"element_ops": pairs, "note": "k^2 d (c_i - c_j)^2 terms per pass as the reference "
-                                                        "computes them; the device computes each unordered pair once "
-                                                        "(the rounding is symmetric), SIMT f32 in the reference's "
-                                                        "sqdist rounding (no tensor cores: the order of roundings is "
-                                                        "the result)"},
+                                                        "computes them; on the device a three-term BF16 search "
+                                                        "leaves the pairs that can matter, which are evaluated in "
+                                                        "the reference's sqdist rounding"},
             "e2e": {"value": n / te, "unit": "rows/s", "h2d_bytes_per_step": n * 8 + K * d * 4,
                     "d2h_bytes_per_step": n * 8 + K * 48 + live * 4}}
     if not args.no_cpu:
@@ -882,7 +881,7 @@ def run_c5(args):
     (top, conf, mass), t_mlp, st_mlp, lab_m, dist_m = runs[0]
     line = {"metric": "rows/s assigned (10M x 96 heavy-tailed, k=65536): learned proposer vs full search",
             "value": n / (t_mlp / 1e3), "unit": "rows/s", "n_gpus": 1, "steps": args.steps, "warmup": args.warmup,
-            "ms_per_step": t_mlp, "higher_is_better": True, "dtype": "bf16 -> f32 accumulate",
+            "ms_per_step": t_mlp, "higher_is_better": True, "dtype": "bf16 network, bf16x3 / fp16 search -> f32 accumulate",
             "config": {"workload": f"{n} x {d} heavy-tailed rows (Student-t nu=3, 8192 components), k={k}, "
                                    f"{groups} groups, network 96-512-512-256",
                        "top": top, "confidence": conf, "mass": mass, "proposer_steps": args.proposer_steps,

@@ -47,7 +47,8 @@ typedef struct emb200_handle emb200_handle;
  * certify are searched again exactly. */
 #define EMB200_PREC_FP32 0  /* FP32 SIMT contraction */
 #define EMB200_PREC_BF16 1  /* tcgen05 BF16, three-term split (hi*hi + hi*lo + lo*hi), FP32 accumulate */
-#define EMB200_PREC_BF16X1 2 /* tcgen05 BF16 single term, FP32 accumulate (wider bound, more re-search) */
+#define EMB200_PREC_BF16X1 2 /* tcgen05 single term, FP32 accumulate (wider bound, more refined rows): f32 rows as
+                                FP16 scaled by one power of two, integer rows in BF16 */
 #define EMB200_PREC_FP8 3    /* tcgen05 FP8 e4m3 operands (kind::f8f6f4), a power-of-two scale per row and per
                                 centroid, FP32 accumulate; f32 rows with d <= 256 (else as BF16X1). Its error
                                 bound (e4m3 unit roundoff 2^-4) is wide: most rows go on to the refine pass */
