@@ -995,7 +995,7 @@ int settle_rows(emb200_handle* h, const T* x, const uint32_t* gather, size_t m, 
     const int match = h->opts.match_kernel;
     bool vec4 = false;
     if constexpr (std::is_same<T, float>::value)
-        vec4 = d % 16 == 0 && ((uintptr_t)x & 15) == 0 && ((uintptr_t)h->c.p & 15) == 0;
+        vec4 = d % 4 == 0 && ((uintptr_t)x & 15) == 0 && ((uintptr_t)h->c.p & 15) == 0;
     if (certified) {
         // the fast kernel certified its rows itself (TcParams::fuse)
     } else if (match == kMatchAvx512 && vec4) {

@@ -547,3 +547,25 @@ def test_small_host_calls(emb, orc, assigners, precision, m):
         assert np.array_equal(lab, rl) and same_f32(dist, rd)
         st = a.stats()
         assert st["rows"] == len(x) and st["rows_certified"] + st["rows_refined"] == len(x)
+
+@pytest.mark.parametrize("precision", ["fp32", "bf16", "bf16x1"])
+@pytest.mark.parametrize("m,k,d", [(65, 40, 4), (3001, 257, 20), (2500, 300, 100), (1000, 64, 124), (700, 130, 252)])
+def test_certify_partial_chunks(emb, orc, precision, m, k, d):
+    # Rows of whole float4s but a partial last chunk of 16: the re-scores, the rows'
+    # norms and so every label and distance are the reference's bits; zero rows and
+    # negative zeros among them, a bias beside the norms.
+    rng = np.random.default_rng(7 * m + d)
+    c = rng.standard_normal((k, d), dtype=np.float32)
+    x = c[rng.integers(0, k, m)] + rng.standard_normal((m, d), dtype=np.float32) * np.float32(0.4)
+    x[::17] = 0.0
+    x[5::19] *= np.float32(-0.0)
+    c[k // 2] = 0.0
+    bias = rng.random(k).astype(np.float32)
+    a = emb.B200Assigner(0, precision=precision)
+    a.set_centroids(c)
+    a.set_bias(bias)
+    lab, dist = a.assign(x)
+    a.close()
+    ref_l, ref_d = orc.cpu_assign(x, c, bias=bias, kernel="avx512", emulate=not orc.has_kernel("avx512"))
+    assert np.array_equal(lab, ref_l)
+    assert np.array_equal(dist.view(np.uint32), ref_d.view(np.uint32))
