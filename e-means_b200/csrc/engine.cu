@@ -19,6 +19,7 @@
 #include "../../include/emb200.h"
 #include "common.cuh"
 #include "host_recipe.hpp"
+#include "search_plan.hpp"
 #include "kernels_exact.cuh"
 #include "kernels_i8.cuh"
 #include "kernels_simt.cuh"
@@ -46,6 +47,10 @@ constexpr size_t kMaxSearchRows = (size_t)1 << 26;  // rows per search pass (32-
 
 using namespace emb;
 
+static_assert(kPlanTcM == kTcBM && kPlanTcN == kTcBN && kPlanSimtLargeM == SimtLarge::BM && kPlanSimtLargeN == SimtLarge::BN &&
+                  kPlanSimtSmallM == SimtSmall::BM && kPlanSimtSmallN == SimtSmall::BN,
+              "search_plan.hpp plans the kernels' tiles");
+
 namespace {
 
 struct Proposer;
@@ -67,6 +72,7 @@ struct DevBuf {
         if (e == cudaSuccess) n = std::max(want, (size_t)1);
         return e;
     }
+    bool lacks(size_t want) const { return !p || n < want; }
     void release() {
         if (p) cudaFree(p);
         p = nullptr;
@@ -294,6 +300,12 @@ int fail(emb200_handle* h, int code, const char* fmt, ...) {
     va_end(ap);
     if (h) h->err = buf;
     return code;
+}
+
+// Within a training run's steps no scratch may move: captured graphs hold its address,
+// and the step before has zeroed what the next one adds to.
+int fail_steady(emb200_handle* h, size_t m) {
+    return fail(h, EMB200_ESTATE, "a training batch of %zu rows needs more scratch than its run reserved", m);
 }
 
 #define CK(call)                                                                                      \
@@ -569,6 +581,10 @@ int launch_i8_assign(emb200_handle* h, const int8_t* x, const uint32_t* gather, 
         }
     }
     // part_s holds int64 scores here: 2 floats per entry.
+    if (graph && h->steady &&
+        (h->part_s.lacks(part_rows * 2) || h->part_i.lacks(part_rows) || h->counters.lacks(8) ||
+         (tc && h->pkeys.lacks((h->k + kTcBN - 1) / kTcBN * kTcBN))))
+        return fail_steady(h, m);
     if (h->part_s.ensure(part_rows * 2) || h->part_i.ensure(part_rows) || h->counters.ensure(8))
         return fail(h, EMB200_ENOMEM, "scratch allocation failed for %zu rows", m);
     if (!graph) CK(cudaEventRecord(h->evk0, st));
@@ -660,67 +676,6 @@ bool tc_supported(const emb200_handle* h, int nterms, bool fp8 = false) {
     return L.stages >= 2 && L.total + 1024 <= (uint32_t)kTcSmemLimit;
 }
 
-// Column splits of the tensor-core search: the one with the fewest waves of items
-// times the tiles an item takes plus two tiles' time for its rows and the drain of
-// its accumulators, a larger split only when it saves 3%. 394 row tiles on 148 SMs:
-// 3 splits, 8 waves of 22 tiles, against 3 waves of 64 unsplit. Half a tile for an
-// item split too much: 20,011 x 100 rows against 1031 centroids 55 -> 38 us (three
-// terms) and 91 -> 38 us (single term), 19,000 x 4096 single term 81 -> 57 us; 3 or
-// 5 tiles measured the same as 2 or slower.
-//
-// Splits with the same tiles per CTA form runs of consecutive counts, and within
-// a run the waves never decrease with the count, so only the first count of each
-// run can be chosen: visiting those (O(sqrt(tiles)) of them) picks the same split
-// as trying every count from 1 to the number of tiles.
-int tc_nsplit(const emb200_handle* h, size_t m, size_t k) {
-    const long row_tiles = (long)((m + kTcBM - 1) / kTcBM);
-    const int ntiles = (int)((k + kTcBN - 1) / kTcBN);
-    const long sms = std::max(1, h->sm_count);
-    int best = 1;
-    double best_cost = 0.0;
-    for (int ns = 1; ns <= ntiles;) {
-        const int per_cta = (ntiles + ns - 1) / ns;
-        const double waves = (double)((row_tiles * ns + sms - 1) / sms);
-        const double cost = waves * ((double)per_cta + 2.0);
-        if (ns == 1 || cost < 0.97 * best_cost) {
-            best = ns;
-            best_cost = cost;
-        }
-        if (per_cta == 1) break;
-        ns = (ntiles + per_cta - 2) / (per_cta - 1);  // first count with fewer tiles per CTA
-    }
-    return best;
-}
-
-// Tile and column splits of the FP32 SIMT search: 128 x 256 tiles (one CTA per SM),
-// or 64 x 64 (two) while those would leave SMs without work; the split with the
-// fewest waves of CTAs times the tiles each takes plus half a tile for its start and
-// merge.
-struct SimtPlan {
-    bool small;
-    int row_tiles, nsplit;
-};
-SimtPlan simt_plan(int sms, size_t m, size_t k) {
-    SimtPlan p;
-    sms = std::max(1, sms);
-    p.small = (m + SimtLarge::BM - 1) / SimtLarge::BM * ((k + SimtLarge::BN - 1) / SimtLarge::BN) < (size_t)sms;
-    const size_t bm = p.small ? SimtSmall::BM : SimtLarge::BM, bn = p.small ? SimtSmall::BN : SimtLarge::BN;
-    const long slots = p.small ? 2L * sms : sms;
-    p.row_tiles = (int)((m + bm - 1) / bm);
-    const int ntiles = (int)((k + bn - 1) / bn);
-    p.nsplit = 1;
-    double best = 0.0;
-    for (int ns = 1; ns <= std::min(ntiles, 64); ns++) {
-        const int per = (ntiles + ns - 1) / ns;
-        const double cost = (double)(((long)p.row_tiles * ns + slots - 1) / slots) * (per + 0.5);
-        if (ns == 1 || cost < 0.97 * best) {
-            best = cost;
-            p.nsplit = ns;
-        }
-    }
-    return p;
-}
-
 template <typename T, bool COLLECT, bool FP8, bool NM = false>
 int launch_tc_kernel(emb200_handle* h, const T* x, const TcParams& p, int nsplit, cudaStream_t st,
                      const CUtensorMap* hi = nullptr, const CUtensorMap* lo = nullptr) {
@@ -765,7 +720,7 @@ int launch_tc(emb200_handle* h, const T* x, const uint32_t* gather, const uint32
         p.stall_tile = h->stall_tile;
         p.stall_ns = h->stall_ns;
     }
-    const int nsplit = nsplit_override > 0 ? nsplit_override : tc_nsplit(h, m, h->k);
+    const int nsplit = nsplit_override > 0 ? nsplit_override : tc_nsplit(h->sm_count, m, h->k);
     p.nsplit = nsplit;
     if constexpr (!COLLECT && std::is_same<T, float>::value) {
         if (fp8) return launch_tc_kernel<T, false, true>(h, x, p, nsplit, st);
@@ -882,7 +837,7 @@ int assign_rows_dev(emb200_handle* h, const T* x, const uint32_t* gather, size_t
     const int fast_terms = tc_terms(prec, dtype);
     const bool tc = prec != EMB200_PREC_FP32 && (fp8 || tc_supported(h, fast_terms));
     const SimtPlan plan = simt_plan(h->sm_count, m, h->k);
-    const int nsplit = tc ? tc_nsplit(h, m, h->k) : plan.nsplit;
+    const int nsplit = tc ? tc_nsplit(h->sm_count, m, h->k) : plan.nsplit;
     // Inside the training loop (graph = true) nothing may allocate while an epoch is
     // captured, and a smaller batch can need more split partials than a full one
     // (fewer row tiles, more splits): size them for every batch of up to m rows.
@@ -891,16 +846,16 @@ int assign_rows_dev(emb200_handle* h, const T* x, const uint32_t* gather, size_t
         // Sized before for every batch of up to part_size_m rows, which covers this one.
         part_rows = std::max(part_rows, h->part_size_rows);
     } else if (graph) {
-        for (size_t rt = 1; rt * kTcBM < m + kTcBM; rt++) {
-            const size_t mm = std::min(rt * kTcBM, m);
-            const int ns = tc ? tc_nsplit(h, mm, h->k) : simt_plan(h->sm_count, mm, h->k).nsplit;
-            part_rows = std::max(part_rows, (size_t)ns * mm);
-        }
+        part_rows = std::max(part_rows, search_part_rows(h->sm_count, m, h->k, tc));
         h->part_size_m = m;
         h->part_size_k = h->k;
         h->part_size_tc = tc;
         h->part_size_rows = part_rows;
     }
+    if (graph && h->steady &&
+        (h->part_s.lacks(part_rows * 2) || h->part_i.lacks(part_rows * 2) || h->redo_rows.lacks(m) ||
+         h->redo_theta.lacks(m) || h->counters.lacks(8)))
+        return fail_steady(h, m);
     if (h->part_s.ensure(part_rows * 2) || h->part_i.ensure(part_rows * 2) || h->redo_rows.ensure(m) ||
         h->redo_theta.ensure(m) || h->counters.ensure(8))
         return fail(h, EMB200_ENOMEM, "scratch allocation failed for %zu rows", m);
@@ -1040,6 +995,9 @@ int settle_rows(emb200_handle* h, const T* x, const uint32_t* gather, size_t m, 
             redo2 = cand_count + m;
             done = redo2 + m;
         } else {
+            if (h->steady && ((refine && (h->cand.lacks(m * cap) || h->cand_count.lacks(m) || h->redo2_rows.lacks(m))) ||
+                              h->rkeys.lacks(m) || h->rdone.lacks(m)))
+                return fail_steady(h, m);
             if ((refine && (h->cand.ensure(m * cap) || h->cand_count.ensure(m) || h->redo2_rows.ensure(m))) ||
                 h->rkeys.ensure(m) || h->rdone.ensure(m))
                 return fail(h, EMB200_ENOMEM, "refine allocation failed for %zu rows", m);

@@ -363,3 +363,21 @@ def test_lockstep_more_clusters_than_one_scan_block(emb):
         s = emb.train(p, 20, k, cfg, assigner=b)
         b.close()
         assert np.array_equal(o.labels, s.labels) and same_f32(o.centroids, s.centroids)
+
+
+@pytest.mark.parametrize("precision,n,k", [("fp32", 54853, 1573), ("fp32", 20011, 700), ("bf16", 20011, 700)])
+def test_graph_replay_after_an_epoch_of_another_length(emb, orc, precision, n, k):
+    # Whole epochs, a fractional one and a whole one: the whole epoch's graph, captured at
+    # its second use, is replayed after the fractional epoch ran kernel by kernel with its
+    # own last batch, which (1425 rows, k = 1573) takes more split partials than any batch
+    # of a multiple of 128 rows. The scratch must be where the graph has it.
+    x = emb.datasets.blobs(n, 20, n_blobs=300, seed=n % 89)
+    cfg = dict(nepochs=3.25, batch_size=4096)
+    out, ref, st = run_both(emb, orc, x, k, precision, **cfg)
+    assert out.recipe.epoch_rows == [n, n, round(n / 4), n]
+    check_same(out, ref)
+    assert st["fast_aborted"] == 0
+    a = emb.B200Assigner(0, precision=precision, train_eager=True)
+    eager = emb.train(x, 20, k, emb.Config(**cfg), assigner=a)
+    a.close()
+    assert np.array_equal(out.labels, eager.labels) and same_f32(out.centroids, eager.centroids)
