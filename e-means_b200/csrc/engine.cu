@@ -352,10 +352,11 @@ size_t elt_size(int dtype) { return dtype == EMB200_F32 ? 4 : 1; }
 // truncated terms, whose magnitudes add |norm| / 2 to the sum they are relative to,
 // so the score (twice the accumulator) gains gamma(d + 5, 2u) |norm|.
 //
-// kr (the same search, when the caller asks for it): the operands' rounding is bounded
-// per row instead, by kr (xr cmax + (|x| + xr) dmax) with xr = |x - x^| of the row and
-// dmax >= max_j |c_j - c^_j| (exact identity plus Cauchy-Schwarz, in score units), and
-// leaves ka.
+// kr (a single-term search, when the caller asks for it): the operands' rounding is
+// bounded per row instead, by kr (xr cmax + (|x| + xr) dmax) with xr = |x - x^| of the
+// row and dmax >= max_j |c_j - c^_j| (exact identity plus Cauchy-Schwarz, in score
+// units), and leaves ka. The residuals are those of the search's own operands: scaled
+// FP16 for f32 rows, BF16 for integer rows, whose xr is zero (single_term).
 void bound_coefficients(int precision, int dtype, size_t d, bool packed, float* ka, float* kb, bool norm_mma = false,
                         float* kr = nullptr) {
     if (kr) *kr = 0.0f;

@@ -3,6 +3,9 @@
 #pragma once
 #include <cuda_bf16.h>
 #include <cuda_fp16.h>
+
+#include <type_traits>
+
 #include "common.cuh"
 
 namespace emb {
@@ -14,7 +17,8 @@ struct Bounds {
     float cmax;  // >= max_j |c_j| (upper-rounded)
     float nmax;  // >= max_j |norms_j| (norms include the bias)
     float cmax_hi;  // >= max_j |bf16(c_j)| (three-term split bound)
-    float dmax;     // >= max_j |c_j - c^_j| of the single-term search's operands (k_prep_f16)
+    float dmax_bf;  // >= max_j |c_j - bf16(c_j)|: the single-term search of integer rows
+    float dmax;     // >= max_j |c_j - c^_j|: the same of f32 rows, scaled FP16 operands (k_prep_f16)
     float s16;      // their power-of-two scale
 };
 
@@ -136,7 +140,7 @@ __global__ void __launch_bounds__(256) k_prep_centroids(const float* __restrict_
     if (j < k) {
         const float* cj = c + (size_t)j * d;
         const float nrm = warp_sqnorm_ref(cj, d, lane);
-        float ss = 0.0f, ssh = 0.0f;
+        float ss = 0.0f, ssh = 0.0f, ssd = 0.0f;
         for (int i = lane; i < kpad; i += 32) {
             const float v = i < d ? cj[i] : 0.0f;
             ss = __fmaf_ru(v, v, ss);
@@ -144,23 +148,26 @@ __global__ void __launch_bounds__(256) k_prep_centroids(const float* __restrict_
                 const __nv_bfloat16 h = __float2bfloat16_rn(v);
                 const float hf = __bfloat162float(h);
                 hi[(size_t)j * kpad + i] = h;
-                lo[(size_t)j * kpad + i] = __float2bfloat16_rn(v - hf);
+                const float r = v - hf;  // exact
+                lo[(size_t)j * kpad + i] = __float2bfloat16_rn(r);
                 ssh = __fmaf_ru(hf, hf, ssh);
+                ssd = __fmaf_ru(r, r, ssd);
             }
         }
         for (int o = 16; o; o >>= 1) {
             ss = __fadd_ru(ss, __shfl_xor_sync(kFull, ss, o));
             ssh = __fadd_ru(ssh, __shfl_xor_sync(kFull, ssh, o));
+            ssd = __fadd_ru(ssd, __shfl_xor_sync(kFull, ssd, o));
         }
         if (lane == 0) norms[j] = nrm;
         mx = make_float4(__fmul_ru(__fsqrt_ru(ss), 1.0000005f), fabsf(nrm), __fmul_ru(__fsqrt_ru(ssh), 1.0000005f),
-                         0.0f);
+                         __fmul_ru(__fsqrt_ru(ssd), 1.0000005f));
     } else if (j < kp && lane == 0) {
         norms[j] = kPadNorm;
     }
     if (lane == 0) part[w] = mx;
     __syncthreads();
-    if (threadIdx.x < 3) {
+    if (threadIdx.x < 4) {
         // The maxima as bit patterns: the values are non-negative or NaN, and a NaN's
         // pattern is above every number's, as in atomic_max_pos.
         uint32_t m = 0;
@@ -241,6 +248,22 @@ __global__ void k_add_bias(float* __restrict__ norms, const float* __restrict__ 
     atomic_max_pos(&bounds->nmax, fabsf(v));
 }
 
+// What the scores of a single-term search leave out besides the accumulation's rounding.
+// T: the rows' type; f32 rows are searched as scaled FP16 (resid: the sum of the squared
+// residuals of S x), integer rows exactly, against the BF16 centroids.
+struct SingleTerm {
+    float xr;    // |x - x^| of the row
+    float dmax;  // max_j |c_j - c^_j|
+    float norm;  // error of the norms' FP16 parts
+};
+template <typename T>
+EMB_DEV SingleTerm single_term(const Bounds* __restrict__ b, float resid, float S) {
+    if constexpr (std::is_same<T, float>::value)
+        return SingleTerm{f16_resid(resid, S), b->dmax, __fmul_ru(0x1p-24f, __fmul_ru(b->cmax, b->cmax))};
+    else
+        return SingleTerm{0.0f, b->dmax_bf, 0.0f};
+}
+
 // The certify decision for one row, given the exact re-scores' dot products a1,
 // a2 (candidates j1, j2) and |x|^2: true when the row is certified (its label and
 // distance written), else false with the refine pass's threshold in *theta_out.
@@ -249,7 +272,7 @@ EMB_DEV bool certify_decide(int row, const Top2& t, uint32_t j1, uint32_t j2, fl
                             uint32_t* __restrict__ labels, float* __restrict__ dist,
                             const int* __restrict__ fast_err, float ka2, float kb2,
                             const float2* __restrict__ row_bounds, float* theta_out, float kr = 0.0f,
-                            float xr = 0.0f) {
+                            SingleTerm st = SingleTerm{}) {
     bool ok = t.i1 < (uint32_t)k && (k < 2 || t.i2 < (uint32_t)k);
     const float s1 = score_ref(norms[j1], a1);
     float sb = s1;
@@ -267,10 +290,10 @@ EMB_DEV bool certify_decide(int row, const Top2& t, uint32_t j1, uint32_t j2, fl
         float E = __fadd_ru(__fmul_ru(__fmul_ru(ka, xnorm), cm),
                             __fmul_ru(kb, row_bounds ? row_bounds[row].y : bounds->nmax));
         // Single-term search: x.c - x^.c^ = (x - x^).c + x^.(c - c^), at most xr cmax +
-        // (|x| + xr) dmax, with xr = |x - x^| of this row; and the norms' FP16 parts.
+        // (|x| + xr) dmax; and the norms' parts.
         if (kr > 0.0f) {
-            E = __fadd_ru(E, __fmul_ru(kr, __fadd_ru(__fmul_ru(xr, cm), __fmul_ru(__fadd_ru(xnorm, xr), bounds->dmax))));
-            E = __fadd_ru(E, __fmul_ru(0x1p-24f, __fmul_ru(cm, cm)));
+            E = __fadd_ru(E, __fmul_ru(kr, __fadd_ru(__fmul_ru(st.xr, cm), __fmul_ru(__fadd_ru(xnorm, st.xr), st.dmax))));
+            E = __fadd_ru(E, st.norm);
         }
         const float thr = __fsub_rd(t.s2, E);
         ok = isfinite(E) && sb < thr;  // NaN-safe: any NaN fails
@@ -335,18 +358,17 @@ __global__ void k_certify(const T* __restrict__ x, const uint32_t* __restrict__ 
     float dg = group_dot_ref(match, xr, c + (size_t)jg * d, d, lane);
     float d1 = __shfl_sync(kFull, dg, 0);
     float d2 = __shfl_sync(kFull, dg, gsz);
-    float xres = 0.0f;  // |x - x^|, upper-rounded (single-term bound)
-    if (kr > 0.0f) {
-        const float S = bounds->s16;
-        float acc = 0.0f;
-        for (int i = lane; i < d; i += 32) acc = f16_resid_sq(S * to_f32(xr[i]), acc);
-        for (int o = 16; o; o >>= 1) acc = __fadd_ru(acc, __shfl_xor_sync(kFull, acc, o));
-        xres = f16_resid(acc, S);
+    const bool f16 = std::is_same<T, float>::value && kr > 0.0f;
+    const float S = f16 ? bounds->s16 : 1.0f;
+    float rs = 0.0f;  // |S x - half(S x)|^2, upper-rounded (single-term bound)
+    if (f16) {
+        for (int i = lane; i < d; i += 32) rs = f16_resid_sq(S * to_f32(xr[i]), rs);
+        for (int o = 16; o; o >>= 1) rs = __fadd_ru(rs, __shfl_xor_sync(kFull, rs, o));
     }
     if (lane != 0) return;
     float theta = 0.0f;
     if (certify_decide(row, t, j1, j2, d1, d2, xn, k, norms, bounds, ka, kb, labels, dist, fast_err, ka2, kb2,
-                       row_bounds, &theta, kr, xres)) {
+                       row_bounds, &theta, kr, single_term<T>(bounds, rs, S))) {
         atomicAdd(cert_count, 1u);
     } else {
         const uint32_t slot = atomicAdd(redo_count, 1u);
@@ -411,12 +433,13 @@ __global__ void k_certify16(const T* __restrict__ x, const uint32_t* __restrict_
     const float* c2 = c + (size_t)j2 * d;
     const int body = d & ~15, dr = (d + 15) & ~15;
     float sq = 0.0f, a1 = 0.0f, a2 = 0.0f, rs = 0.0f;
-    const float S = kr > 0.0f ? bounds->s16 : 1.0f;
+    const bool f16 = std::is_same<T, float>::value && kr > 0.0f;
+    const float S = f16 ? bounds->s16 : 1.0f;
     for (int i = l; i < dr; i += 16) {
         const bool in = i < d;
         const float xv = in ? to_f32(xr[i]) : 0.0f;
         if (i < body) sq = __fadd_rn(sq, __fmul_rn(xv, xv));
-        if (kr > 0.0f) rs = f16_resid_sq(S * xv, rs);
+        if (f16) rs = f16_resid_sq(S * xv, rs);
         a1 = __fmaf_rn(xv, in ? c1[i] : 0.0f, a1);
         a2 = __fmaf_rn(xv, in ? c2[i] : 0.0f, a2);
     }
@@ -440,7 +463,7 @@ __global__ void k_certify16(const T* __restrict__ x, const uint32_t* __restrict_
     float theta = 0.0f;
     if (live && l == 0) {
         ok = certify_decide(row, t, j1, j2, a1, a2, xn, k, norms, bounds, ka, kb, labels, dist, fast_err, ka2, kb2,
-                              row_bounds, &theta, kr, f16_resid(rs, S));
+                              row_bounds, &theta, kr, single_term<T>(bounds, rs, S));
         redo = !ok;
     }
     certify_tally(ok, redo, row, theta, cert_count, redo_count, redo_rows, redo_theta);
@@ -533,7 +556,7 @@ __global__ void k_certify16v(const float* __restrict__ x, const uint32_t* __rest
     float theta = 0.0f;
     if (live && q == 0) {
         ok = certify_decide(row, t, j1, j2, a1, a2, xn, k, norms, bounds, ka, kb, labels, dist, fast_err, ka2, kb2,
-                              row_bounds, &theta, kr, f16_resid(rs, S));
+                              row_bounds, &theta, kr, single_term<float>(bounds, rs, S));
         redo = !ok;
     }
     certify_tally(ok, redo, row, theta, cert_count, redo_count, redo_rows, redo_theta);

@@ -834,7 +834,8 @@ EMB_DEV void tc_fused_certify(const TcParams& p, const float* __restrict__ x, co
                 // pair), so one exact dot product serves both.
                 const int no_abort = 0;
                 ok = certify_decide(row, t, j1, j1, a1, a1, xn, k, p.norms, p.bounds, p.ka, p.kb, p.labels, p.dist,
-                                    &no_abort, p.ka2, p.kb2, nullptr, &theta, p.kr, f16_resid(rs, S));
+                                    &no_abort, p.ka2, p.kb2, nullptr, &theta, p.kr,
+                                    single_term<float>(p.bounds, rs, S));
                 redo = !ok;
             }
         } else {

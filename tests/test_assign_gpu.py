@@ -569,3 +569,58 @@ def test_certify_partial_chunks(emb, orc, precision, m, k, d):
     ref_l, ref_d = orc.cpu_assign(x, c, bias=bias, kernel="avx512", emulate=not orc.has_kernel("avx512"))
     assert np.array_equal(lab, ref_l)
     assert np.array_equal(dist.view(np.uint32), ref_d.view(np.uint32))
+
+
+def _generic_codes(dtype, m, k, d, seed):
+    # integer rows around generic (not BF16-exact) centroids
+    rng = np.random.default_rng(seed)
+    info = np.iinfo(dtype)
+    c = rng.uniform(info.min, info.max, (k, d)).astype(np.float32)
+    x = np.clip(np.round(rng.uniform(info.min, info.max, (m, d))), info.min, info.max).astype(dtype)
+    return x, c
+
+
+@pytest.mark.parametrize("precision", ["bf16x1", "fp8"])
+@pytest.mark.parametrize("dtype", [np.int8, np.uint8])
+@pytest.mark.parametrize("d", [16, 40, 100])
+@pytest.mark.parametrize("with_bias", [False, True])
+def test_integer_rows_beside_f32_rows(orc, assigners, precision, dtype, d, with_bias):
+    # f32 rows, then integer rows, then f32 rows again on one set of centroids: each search
+    # has operands of its own (scaled FP16; BF16 with exact rows) and must be certified with
+    # their residuals, with and without a bias in between.
+    x, c = _generic_codes(dtype, 20000, 256, d, d)
+    a = assigners(precision)
+    a.set_centroids(c)
+    f = x[:3000].astype(np.float32) + np.float32(0.37)
+    bias = None
+    for step in range(3):
+        if step == 1 and with_bias:
+            bias = (np.random.default_rng(d).random(256) * d * 40).astype(np.float32)
+            a.set_bias(bias)
+        rows = x if step == 1 else f
+        lab, dist = a.assign(rows)
+        rl, rd = orc.cpu_assign(rows, c, bias=bias, emulate=not orc.has_kernel("avx512"))
+        assert np.array_equal(lab, rl) and same_f32(dist, rd), step
+
+
+@pytest.mark.parametrize("dtype", [np.int8, np.uint8])
+@pytest.mark.parametrize("after_f32", [False, True])
+def test_integer_rows_single_term_certifies(orc, emb, dtype, after_f32):
+    # Well separated integer blobs: the single-term search settles nearly every row at
+    # once, whatever was searched on the handle before.
+    rng = np.random.default_rng(3)
+    info = np.iinfo(dtype)
+    m, k, d = 30000, 400, 64
+    centre = rng.integers(info.min + 8, info.max - 8, (k, d))
+    x = (centre[rng.integers(0, k, m)] + rng.integers(-4, 5, (m, d))).astype(dtype)
+    c = (centre + rng.uniform(-0.5, 0.5, (k, d))).astype(np.float32)
+    a = emb.B200Assigner(0, precision="bf16x1")
+    a.set_centroids(c)
+    if after_f32:
+        a.assign(x[:100].astype(np.float32))
+    lab, dist = a.assign(x)
+    st = a.stats()
+    a.close()
+    rl, rd = orc.cpu_assign(x, c, emulate=not orc.has_kernel("avx512"))
+    assert np.array_equal(lab, rl) and same_f32(dist, rd)
+    assert st["rows_refined"] <= 0.03 * m, st
