@@ -33,10 +33,10 @@ struct Bounds {
 // narrow range costs values far below the largest one some of those bits, which only
 // enters through the residuals |x - x^| and |c - c^| that the bound is made of;
 // anything out of range (a row hundreds of times the centroids) has an infinite
-// residual and is refined.
+// residual and is refined. (Centroids that are all zero leave the scale to the biases.)
 EMB_DEV float f16_scale(const Bounds& b) {
-    if (!(b.cmax > 0.0f) || !isfinite(b.cmax) || !isfinite(b.nmax)) return 1.0f;
-    int e = 6 - ((int)(__float_as_uint(b.cmax) >> 23) - 127);
+    if (!isfinite(b.cmax) || !isfinite(b.nmax)) return 1.0f;
+    int e = b.cmax > 0.0f ? 6 - ((int)(__float_as_uint(b.cmax) >> 23) - 127) : 60;
     const int en = (int)(__float_as_uint(b.nmax) >> 23) - 127;
     if (b.nmax > 0.0f) e = min(e, (14 - en) >> 1);
     return __uint_as_float((uint32_t)(max(-60, min(60, e)) + 127) << 23);
@@ -176,16 +176,18 @@ __global__ void __launch_bounds__(256) k_prep_centroids(const float* __restrict_
     }
 }
 
+constexpr float kNrm16One = 1024.0f;    // the constant row operand against the norms' parts
+constexpr float kNrm16Err = 0x1p-14f;   // 2 kNrm16One 2^-25
+
 // The single-term search's centroid operands, from the norms (bias included) and bounds:
 // c16 [k][kpad] = half(S c), zeros past d, its residual into bounds->dmax, S into
 // bounds->s16; nrm16 [kp][16]: the norms inside the contraction. Row j holds the three
 // FP16 parts of h = S^2 norms[j] / 2 / kNrm16One (p1 = half(h), p2 = half(h - p1),
 // p3 = half(h - p1 - p2); the differences are exact in f32), then zeros: p1 + p2 + p3 is
-// within 2^-25 of h, so the score's norm within 2^-24 cmax^2 (a constant the bound
-// carries; S cmax >= 64, or the half-norms reach 2^12). A non-finite norm keeps its value in p1, so the
-// MMA sums the same inf or NaN the epilogue's norm - 2 acc would give. The padding up
-// to kp is the largest finite value: never a candidate. One warp per centroid.
-constexpr float kNrm16One = 1024.0f;  // the constant row operand against the parts
+// within 2^-25 of h, so the score's norm within kNrm16Err / S^2, which the bound adds. A
+// non-finite norm keeps its value in p1, so the MMA sums the same inf or NaN the
+// epilogue's norm - 2 acc would give. The padding up to kp is the largest finite value:
+// never a candidate. One warp per centroid.
 __global__ void __launch_bounds__(256) k_prep_f16(const float* __restrict__ c, int k, int kp, int d, int kpad,
                                                   const float* __restrict__ norms, Bounds* __restrict__ bounds,
                                                   __half* __restrict__ c16, __half* __restrict__ nrm16) {
@@ -259,7 +261,7 @@ struct SingleTerm {
 template <typename T>
 EMB_DEV SingleTerm single_term(const Bounds* __restrict__ b, float resid, float S) {
     if constexpr (std::is_same<T, float>::value)
-        return SingleTerm{f16_resid(resid, S), b->dmax, __fmul_ru(0x1p-24f, __fmul_ru(b->cmax, b->cmax))};
+        return SingleTerm{f16_resid(resid, S), b->dmax, __fmul_ru(kNrm16Err, (1.0f / S) * (1.0f / S))};
     else
         return SingleTerm{0.0f, b->dmax_bf, 0.0f};
 }

@@ -624,3 +624,37 @@ def test_integer_rows_single_term_certifies(orc, emb, dtype, after_f32):
     rl, rd = orc.cpu_assign(x, c, emulate=not orc.has_kernel("avx512"))
     assert np.array_equal(lab, rl) and same_f32(dist, rd)
     assert st["rows_refined"] <= 0.03 * m, st
+
+
+@pytest.mark.parametrize("e", [-50, -54, -56, -60, -62, -64, -66])
+@pytest.mark.parametrize("m,k,d", [(3000, 300, 33), (20003, 259, 64)])
+def test_single_term_tiny_centroids(orc, assigners, e, m, k, d):
+    # Centroid norms around 2^e, where the operands' scale reaches the end of its range:
+    # zero rows (the norms alone decide) and rows of ordinary magnitude.
+    rng = np.random.default_rng(m - e)
+    c = (rng.standard_normal((k, d)) * 2.0 ** e / np.sqrt(d)).astype(np.float32)
+    x = rng.standard_normal((m, d)).astype(np.float32)
+    x[::3] = 0.0
+    a = assigners("bf16x1")
+    a.set_centroids(c)
+    lab, dist = a.assign(x)
+    rl, rd = orc.cpu_assign(x, c, emulate=not orc.has_kernel("avx512"))
+    assert np.array_equal(lab, rl) and same_f32(dist, rd)
+
+
+@pytest.mark.parametrize("scale", [1e-5, 1.0, 1e-30, 3e6])
+@pytest.mark.parametrize("m,k", [(50, 40), (3000, 300), (20000, 700)])
+def test_single_term_zero_centroids_with_bias(orc, assigners, scale, m, k):
+    # All centroids zero: the biases alone decide, and give the operands their scale.
+    rng = np.random.default_rng(m + k)
+    d = 24
+    c = np.zeros((k, d), np.float32)
+    bias = (-np.arange(1, k + 1) * scale).astype(np.float32)[rng.permutation(k)]
+    x = rng.standard_normal((m, d)).astype(np.float32)
+    x[::3] = 0.0
+    a = assigners("bf16x1")
+    a.set_centroids(c)
+    a.set_bias(bias)
+    lab, dist = a.assign(x)
+    rl, rd = orc.cpu_assign(x, c, bias=bias, emulate=not orc.has_kernel("avx512"))
+    assert np.array_equal(lab, rl) and same_f32(dist, rd)
