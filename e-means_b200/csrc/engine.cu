@@ -344,13 +344,14 @@ int smem_attr_once(emb200_handle* h, std::atomic<uint64_t>& done, const void* fn
 size_t elt_size(int dtype) { return dtype == EMB200_F32 ? 4 : 1; }
 
 // Error-bound coefficients of the certification, E = ka |x| cmax + kb nmax
-// (see k_certify). u = 2^-24 (f32 rounding), ub = 2^-8 (bf16 rounding: 8
-// significant bits, round to nearest); the
-// tensor-core accumulation is allowed one f32 truncation (2u) per product term.
+// (see k_certify). u = 2^-24 (f32 rounding), ub = 2^-8 (bf16 rounding: 8 significant
+// bits, round to nearest); the tensor-core accumulation is allowed one f32 truncation (2u)
+// per product term.
 //
-// The single-term search of f32 rows (norm_mma) sums the half-norm's three parts in the same tensor-core accumulation as the d products: three more
-// truncated terms, whose magnitudes add |norm| / 2 to the sum they are relative to,
-// so the score (twice the accumulator) gains gamma(d + 5, 2u) |norm|.
+// The single-term search of f32 rows (norm_mma) sums the half-norm's five parts in the
+// same tensor-core accumulation as the d products: five more truncated terms, whose
+// magnitudes add |norm| / 2 to the sum they are relative to, so the score (twice the
+// accumulator) gains gamma(d + 7, 2u) |norm|. (What the parts leave out: SingleTerm.)
 //
 // kr (a single-term search, when the caller asks for it): the operands' rounding is
 // bounded per row instead, by kr (xr cmax + (|x| + xr) dmax) with xr = |x - x^| of the
@@ -386,10 +387,10 @@ void bound_coefficients(int precision, int dtype, size_t d, bool packed, float* 
             rep = 0.0;
             *kr = 2.0f * (1.0f + 0x1p-10f);
         }
-        a = 2.0 * (rep + 1.02 * gamma((double)d + (norm_mma ? 5 : 2), 2 * u) + g_ref) + 4.02 * u;
+        a = 2.0 * (rep + 1.02 * gamma((double)d + (norm_mma ? 7 : 2), 2 * u) + g_ref) + 4.02 * u;
     }
     double b = 2.0 * u;
-    if (norm_mma) b += 1.02 * gamma((double)d + 5, 2 * u);
+    if (norm_mma) b += 1.02 * gamma((double)d + 7, 2 * u);
     if (packed) {  // tensor-core top-2 keys carry the column in 5 mantissa bits: |key - s| <= 2^-18 |s|
         const double t = std::ldexp(1.0, -18);
         a += 2.01 * t;

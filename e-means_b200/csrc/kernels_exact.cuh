@@ -176,16 +176,19 @@ __global__ void __launch_bounds__(256) k_prep_centroids(const float* __restrict_
     }
 }
 
-constexpr float kNrm16One = 1024.0f;    // the constant row operand against the norms' parts
-constexpr float kNrm16Err = 0x1p-14f;   // 2 kNrm16One 2^-25
+constexpr float kNrm16One = 1024.0f;      // the constant row operand against the norms' first three parts
+constexpr float kNrm16Step = 0x1p24f;     // the last two are of kNrm16Step times what those leave (at 1024 2^-24)
+constexpr float kNrm16Err = 0x1p-38f;     // 2 kNrm16One 2^-25 / kNrm16Step
 
 // The single-term search's centroid operands, from the norms (bias included) and bounds:
 // c16 [k][kpad] = half(S c), zeros past d, its residual into bounds->dmax, S into
-// bounds->s16; nrm16 [kp][16]: the norms inside the contraction. Row j holds the three
-// FP16 parts of h = S^2 norms[j] / 2 / kNrm16One (p1 = half(h), p2 = half(h - p1),
-// p3 = half(h - p1 - p2); the differences are exact in f32), then zeros: p1 + p2 + p3 is
-// within 2^-25 of h, so the score's norm within kNrm16Err / S^2, which the bound adds. A
-// non-finite norm keeps its value in p1, so the MMA sums the same inf or NaN the
+// bounds->s16; nrm16 [kp][16]: the norms inside the contraction. Row j holds the FP16
+// parts of h = S^2 norms[j] / 2 / kNrm16One, then zeros: p1 = half(h), p2 = half(h - p1),
+// p3 = half(h - p1 - p2), which together are within 2^-25 of h (FP16's smallest step is
+// 2^-24), and p4, p5 the same of 2^24 times what is left. All differences are exact in
+// f32. h below 16 keeps all 24 bits down to 2^-25 (a norm 2^-29 of the largest) and is
+// within 2^-49 further down: the score's norm within kNrm16Err / S^2, which the bound
+// adds. A non-finite norm keeps its value in p1, so the MMA sums the same inf or NaN the
 // epilogue's norm - 2 acc would give. The padding up to kp is the largest finite value:
 // never a candidate. One warp per centroid.
 __global__ void __launch_bounds__(256) k_prep_f16(const float* __restrict__ c, int k, int kp, int d, int kpad,
@@ -208,22 +211,29 @@ __global__ void __launch_bounds__(256) k_prep_f16(const float* __restrict__ c, i
         dm = __fmul_ru(__fmul_ru(__fsqrt_ru(ssd), 1.0000005f), 1.0f / S);
     }
     if (lane == 0 && j < kp) {
-        __half p1 = __float2half_rn(65504.0f), p2 = p1, p3 = p1;
+        const __half zero = __float2half_rn(0.0f);
+        __half p1 = __float2half_rn(65504.0f), p2 = p1, p3 = p1, p4 = zero, p5 = zero;
         if (j < k) {
             const float h = norms[j] * (0.5f * S * S / kNrm16One);
             if (!(fabsf(h) > 65504.0f) || !isfinite(h)) {
                 p1 = __float2half_rn(h);
-                p2 = p3 = __float2half_rn(0.0f);
+                p2 = p3 = zero;
                 if (isfinite(h)) {
-                    const float r1 = h - __half2float(p1);
-                    p2 = __float2half_rn(r1);
-                    p3 = __float2half_rn(r1 - __half2float(p2));
+                    float r = h - __half2float(p1);
+                    p2 = __float2half_rn(r);
+                    r -= __half2float(p2);
+                    p3 = __float2half_rn(r);
+                    r = kNrm16Step * (r - __half2float(p3));
+                    p4 = __float2half_rn(r);
+                    p5 = __float2half_rn(r - __half2float(p4));
                 }
             }
         }
+        auto pair = [](__half a, __half b) {
+            return (uint32_t)__half_as_ushort(a) | ((uint32_t)__half_as_ushort(b) << 16);
+        };
         uint4* o = reinterpret_cast<uint4*>(nrm16 + (size_t)j * 16);
-        o[0] = make_uint4((uint32_t)__half_as_ushort(p1) | ((uint32_t)__half_as_ushort(p2) << 16),
-                          (uint32_t)__half_as_ushort(p3), 0u, 0u);
+        o[0] = make_uint4(pair(p1, p2), pair(p3, p4), pair(p5, zero), 0u);
         o[1] = make_uint4(0u, 0u, 0u, 0u);
     }
     if (lane == 0) part[w] = dm;

@@ -54,8 +54,8 @@ constexpr int kTcPThreads = 32 * (kTcEpi0 + kTcEpiWarps);
 constexpr int kTcRowScaleSlots = 4;  // FP8 per-row scales, a ring over work items
 // Norms inside the contraction (single-term search of f32 rows, NM, FP16 operands
 // scaled by S: k_prep_f16): each tile starts with one K = 16 MMA of a constant row
-// operand [1024, 1024, 1024, 0, ...] against the tile's half-norms split into three
-// parts, so the accumulator holds S^2 (norm / 2 - x . c) (the rows enter negated), the
+// operand [1024, 1024, 1024, 2^-14, 2^-14, 0, ...] against the tile's half-norms split into
+// five parts, so the accumulator holds S^2 (norm / 2 - x . c) (the rows enter negated), the
 // score times S^2 / 2, and the epilogue scores without loading norms or multiplying. A
 // ring of two 8 KB slices.
 constexpr int kTcNmSlots = 2;
@@ -930,12 +930,13 @@ k_assign_tc(const T* __restrict__ x, const __grid_constant__ CUtensorMap map_hi,
         for (int i = threadIdx.x; i < 4 * kTcBM; i += blockDim.x) pub[i] = INFINITY;
     }
     if (NM) {
-        // The constant row operand of the norm MMA: every row [1024, 1024, 1024, 0, 0, 0,
-        // 0, 0] (kNrm16One, FP16 0x6400) in both 16-byte halves, so whichever half the 32-byte
-        // swizzle pairs with the norm slice's parts, the product is 1024 (p1 + p2 + p3).
+        // The constant row operand of the norm MMA: every row [1024, 1024, 1024, 2^-14,
+        // 2^-14, 0, 0, 0] (kNrm16One, FP16 0x6400; kNrm16One / kNrm16Step, 0x0400) in both
+        // 16-byte halves, so whichever half the 32-byte swizzle pairs with the norm slice's
+        // parts, the product is 1024 (p1 + p2 + p3 + 2^-24 (p4 + p5)).
         uint4* nc = reinterpret_cast<uint4*>(smem + L.nconst);
         for (int i = threadIdx.x; i < (int)(kTcNmConstBytes / 16); i += blockDim.x)
-            nc[i] = make_uint4(0x64006400u, 0x00006400u, 0u, 0u);
+            nc[i] = make_uint4(0x64006400u, 0x04006400u, 0x00000400u, 0u);
         asm volatile("fence.proxy.async.shared::cta;" ::: "memory");  // visible to the tensor cores
     }
     tc_fence_before();
