@@ -55,9 +55,13 @@ __device__ __forceinline__ void qs_cp_wait() { asm volatile("cp.async.wait_group
 //   k_quant_colpart  per block of kQsubRows rows and dimension: the sum, the
 //                    range of its prefix sums and its smallest non-zero magnitude
 //                    (which bounds q). One pass over the rows: HBM bounds it.
+//                    A block is added as four parts that start at zero: a part's sums
+//                    lie within the range's width, hi - lo, so they are exact where
+//                    that is at most 2^(53 + q).
 //   k_quant_colscan  one warp per dimension walks the blocks 32 at a time: a lane's
 //                    block is accepted as a whole when the range above shows that
-//                    no partial sum inside it rounds; the first block that is not
+//                    no partial sum inside it (nor inside its parts) rounds; the first
+//                    block that is not
 //                    is replayed from its rows (quant_replay64), which finds the
 //                    adds that do round by their exact error and redoes the rest
 //                    from there.
@@ -351,8 +355,8 @@ __global__ void __launch_bounds__(32 * kQscanWarps) k_quant_colscan(const float*
             bool ok = tn == 0xffffffffu || isnan(p) || (isinf(p) && fin);
             if (!ok) {
                 const double top = quant_pow2(53 + min(qx, quant_lsb(p)));
-                ok = fin && (double)mag < quant_pow2(53 + qx) && __dadd_ru(p, (double)e.hi) <= top &&
-                     __dadd_rd(p, (double)e.lo) >= -top;
+                ok = fin && __dsub_ru((double)e.hi, (double)e.lo) <= quant_pow2(53 + qx) &&
+                     __dadd_ru(p, (double)e.hi) <= top && __dadd_rd(p, (double)e.lo) >= -top;
             }
             const unsigned bad = __ballot_sync(0xffffffffu, lane >= s0 && lane < lim && !ok);
             if (!bad) {

@@ -205,3 +205,31 @@ def test_row_order_sums_over_several_slabs(emb, orc, qa):
     q = emb.Int8Quantizer.fit(x, d, emb.Calibration.faiss(), assigner=qa)
     shift, scale = orc.quantizer_fit(x)
     assert np.array_equal(q.shift.view(np.uint32), shift.view(np.uint32)) and q.scale == np.float32(scale)
+
+
+@pytest.mark.parametrize("d", [1, 4, 33])
+@pytest.mark.parametrize("part", [0, 1, 2])
+def test_row_order_sums_part_beyond_the_blocks_range(emb, orc, qa, d, part):
+    # 64 rows down, then (within one quarter of a 256-row block) up by twice as much, then
+    # back: the sums from the block's start stay within 2^53 of their lowest bit, a
+    # quarter's own sum does not, and the low bit of one row must not be lost there.
+    n = 2304
+    col = np.zeros(n, np.float64)
+    s = 64 * part
+    col[s:s + 64] = -15_000_000.0
+    col[s + 64] = 1.0 + 2.0 ** -23
+    col[s + 65:s + 128] = 30_000_000.0
+    rest = 30_000_000.0 * 63 - 15_000_000.0 * 64
+    left = max(1, min(62, 256 - (s + 128)))
+    if s + 128 < 256:
+        col[s + 128:s + 128 + left] = -15_000_000.0
+        rest -= 15_000_000.0 * left
+    while rest > 0:  # the rest comes off after the block
+        j = 256 + int(np.count_nonzero(col[256:]))
+        col[j] = -min(rest, 15_000_000.0)
+        rest += col[j]
+    x = np.repeat(col.astype(np.float32)[:, None], d, axis=1)
+    assert np.array_equal(x[:, 0].astype(np.float64), col)
+    q = emb.Int8Quantizer.fit(x, d, emb.Calibration.faiss(), assigner=qa)
+    shift, _ = orc.quantizer_fit(x)
+    assert np.array_equal(q.shift.view(np.uint32), shift.view(np.uint32))
