@@ -61,10 +61,9 @@ __device__ __forceinline__ void qs_cp_wait() { asm volatile("cp.async.wait_group
 //   k_quant_colscan  one warp per dimension walks the blocks 32 at a time: a lane's
 //                    block is accepted as a whole when the range above shows that
 //                    no partial sum inside it (nor inside its parts) rounds; the first
-//                    block that is not
-//                    is replayed from its rows (quant_replay64), which finds the
-//                    adds that do round by their exact error and redoes the rest
-//                    from there.
+//                    block that is not is replayed from its rows (quant_replay64), which
+//                    finds the adds that do round by their exact error and redoes the
+//                    rest from there.
 // On 500,000 x 512 unit-norm rows: 0.175 ms (5.9 TB/s of rows, 0.90 of the copy
 // bandwidth) and 0.068 ms, against 4.25 ms for the chain itself (16.7 cycles an
 // add). Blocks of 256 rows: with 64 the scan of four times the entries took
@@ -214,29 +213,26 @@ __device__ __forceinline__ double quant_two_sum_err(double a, double b, double s
 // first add that rounds, and its two-sum error shows which that is). The rest is
 // then added one by one, from the warp's shared memory. The look needs the prefix
 // sums to be exact: 64 times the largest value within 53 bits of the lowest bit.
-// chain: straight to the adds. rough counts the groups that needed most of them.
-__device__ __forceinline__ double quant_replay64(double acc, float x0, float x1, int lane, bool chain, double* buf,
-                                                 int& rough) {
+// rough counts the groups that needed most of the adds.
+__device__ __forceinline__ double quant_replay64(double acc, float x0, float x1, int lane, double* buf, int& rough) {
     int s0 = 0;
-    if (!chain) {
-        const uint32_t tn = __reduce_min_sync(0xffffffffu, min(quant_tiny(x0), quant_tiny(x1)));
-        if (tn == 0xffffffffu) return acc;  // zeros change nothing
-        const uint32_t mx = __reduce_max_sync(
-            0xffffffffu, max(__float_as_uint(x0) & 0x7fffffffu, __float_as_uint(x1) & 0x7fffffffu));
-        if (mx < 0x7f800000u && isfinite(acc) &&
-            64.0 * (double)__uint_as_float(mx) <= quant_pow2(53 + quant_tiny_lsb(tn))) {
-            const double i0 = quant_scan32((double)x0, lane), i1r = quant_scan32((double)x1, lane);
-            const double i1 = __dadd_rn(__shfl_sync(0xffffffffu, i0, 31), i1r);
-            const double p0 = __dadd_rn(acc, i0), p1 = __dadd_rn(acc, i1);
-            const unsigned b0 = __ballot_sync(0xffffffffu, quant_two_sum_err(acc, i0, p0) != 0.0);
-            const unsigned b1 = __ballot_sync(0xffffffffu, quant_two_sum_err(acc, i1, p1) != 0.0);
-            if (!(b0 | b1)) return __shfl_sync(0xffffffffu, p1, 31);
-            const int f = b0 ? __ffs((int)b0) - 1 : __ffs((int)b1) - 1;
-            acc = __shfl_sync(0xffffffffu, b0 ? p0 : p1, f);
-            s0 = f + (b0 ? 1 : 33);
-        }
-        rough += s0 == 0 || s0 < 33;
+    const uint32_t tn = __reduce_min_sync(0xffffffffu, min(quant_tiny(x0), quant_tiny(x1)));
+    if (tn == 0xffffffffu) return acc;  // zeros change nothing
+    const uint32_t mx =
+        __reduce_max_sync(0xffffffffu, max(__float_as_uint(x0) & 0x7fffffffu, __float_as_uint(x1) & 0x7fffffffu));
+    if (mx < 0x7f800000u && isfinite(acc) &&
+        64.0 * (double)__uint_as_float(mx) <= quant_pow2(53 + quant_tiny_lsb(tn))) {
+        const double i0 = quant_scan32((double)x0, lane), i1r = quant_scan32((double)x1, lane);
+        const double i1 = __dadd_rn(__shfl_sync(0xffffffffu, i0, 31), i1r);
+        const double p0 = __dadd_rn(acc, i0), p1 = __dadd_rn(acc, i1);
+        const unsigned b0 = __ballot_sync(0xffffffffu, quant_two_sum_err(acc, i0, p0) != 0.0);
+        const unsigned b1 = __ballot_sync(0xffffffffu, quant_two_sum_err(acc, i1, p1) != 0.0);
+        if (!(b0 | b1)) return __shfl_sync(0xffffffffu, p1, 31);
+        const int f = b0 ? __ffs((int)b0) - 1 : __ffs((int)b1) - 1;
+        acc = __shfl_sync(0xffffffffu, b0 ? p0 : p1, f);
+        s0 = f + (b0 ? 1 : 33);
     }
+    rough += s0 < 33;
     buf[lane] = (double)x0;
     buf[32 + lane] = (double)x1;
     __syncwarp();
@@ -255,44 +251,85 @@ __device__ __forceinline__ double quant_replay64(double acc, float x0, float x1,
     return acc;
 }
 
+// acc after 256 rows (doubles in shared memory), added one by one, 16 at a time with the
+// next 16 on their way.
+__device__ __forceinline__ double quant_chain256(double acc, const double* rows) {
+    double a[16], b[16];
+#pragma unroll
+    for (int j = 0; j < 16; j++) a[j] = rows[j];
+#pragma unroll 1
+    for (int r = 0; r < kQsubRows; r += 32) {
+#pragma unroll
+        for (int j = 0; j < 16; j++) b[j] = rows[r + 16 + j];
+#pragma unroll
+        for (int j = 0; j < 16; j++) acc = __dadd_rn(acc, a[j]);
+        const double* next = rows + (r + 32) % kQsubRows;  // (the first again at the end: not used)
+#pragma unroll
+        for (int j = 0; j < 16; j++) a[j] = next[j];
+#pragma unroll
+        for (int j = 0; j < 16; j++) acc = __dadd_rn(acc, b[j]);
+    }
+    return acc;
+}
+
 // One warp per dimension; first / last: the sample's first / last slab of rows
 // (carry holds the sums in between). sub = nullptr: no entries, every block is
 // replayed (short samples: n <= kQscanShort, where the entries' launch costs more
 // than they save).
 // Where the adds round often (magnitudes spread over many binades), looking first is
-// slower than the chain: a block with two or more groups of 64 rows that needed
-// most of it sends the next kQscanChain blocks straight there, the rows of each on
-// their way while the one before is added. Magnitudes over 60 binades, 200,000 x 64:
-// 2.1 ms (1.77 ms for the bare chain); squares of normals 1.9 ms; normals 0.11 ms.
+// slower than the chain: a warp that has met two groups of 64 rows that needed most of
+// their adds, in one block after another, leaves the next blocks to its whole CTA:
+// kQscanJoint of them, and twice as many, up to kQscanJointMost, each time that this
+// happens again within as many as the last time. There one warp adds, a lane a
+// dimension, and the others bring the rows: each row's 32 bytes are read once, where a
+// warp alone touches 32 lines for 32 values of its column, which bounds it (9.6 ns a row,
+// 17 with two CTAs on an SM), and no FP64 cycles go into 32 equal results. Whole fits,
+// each dimension's warp replaying by itself / so / every dimension as one chain from the
+// start: magnitudes over 60 binades, 200,000 x 64 1985 / 1251 / 1780 us, 50,000 x 2048
+// 1094 / 624 / 574; squares of normals 200,000 x 64 1871 / 1347 / 1778, 50,000 x 2048 963
+// / 728 / 577; normals, 200,000 x 64, 126 / 126 / 1780. First joint runs of 8 and 16
+// blocks: 1264 and 1260, 842 and 770 us where 32 takes 1251 and 728.
 constexpr size_t kQscanShort = 2048;
-constexpr int kQscanChain = 32;
+constexpr int kQscanJoint = 32, kQscanJointMost = 256;
+constexpr int kQscanPitch = kQsubRows + 4;  // of a dimension's converted rows: no bank conflicts across dimensions
+struct QuantRing {
+    QuantSub sub[kQscanWarps][kQscanDepth][32];
+    uint32_t tiny[kQscanWarps][kQscanDepth][32];
+};
+union QuantScanSmem {
+    QuantRing ring;                                // a warp's entries
+    double joint[2][kQscanWarps][kQscanPitch];     // two blocks of all its dimensions' rows
+};
 __global__ void __launch_bounds__(32 * kQscanWarps) k_quant_colscan(const float* __restrict__ x, size_t n, size_t d,
                                                                     size_t nsub, const QuantSub* __restrict__ sub,
                                                                     const uint32_t* __restrict__ tiny,
                                                                     double* __restrict__ carry, bool first, bool last,
                                                                     size_t n_all, float* __restrict__ shift) {
-    __shared__ QuantSub ring_s[kQscanWarps][kQscanDepth][32];
-    __shared__ uint32_t ring_t[kQscanWarps][kQscanDepth][32];
+    __shared__ __align__(16) uint8_t smem_raw[sizeof(QuantScanSmem)];
     __shared__ __align__(16) double chain_s[kQscanWarps][64];
+    __shared__ size_t pos_s[kQscanWarps];
+    __shared__ double acc_s[kQscanWarps];
+    QuantScanSmem& sm = *reinterpret_cast<QuantScanSmem*>(smem_raw);
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
     const size_t t = (size_t)blockIdx.x * kQscanWarps + warp;
-    if (t >= d) return;
     const size_t nb = (nsub + 31) / 32;
     auto issue = [&](size_t b) {  // each lane copies, and later reads, its own entries only
         const size_t s = b * 32 + lane;
         if (s < nsub) {
-            qs_cp_async16(reinterpret_cast<float*>(&ring_s[warp][b % kQscanDepth][lane]),
+            qs_cp_async16(reinterpret_cast<float*>(&sm.ring.sub[warp][b % kQscanDepth][lane]),
                           reinterpret_cast<const float*>(sub + s * d + t));
-            qs_cp_async4(reinterpret_cast<float*>(&ring_t[warp][b % kQscanDepth][lane]),
+            qs_cp_async4(reinterpret_cast<float*>(&sm.ring.tiny[warp][b % kQscanDepth][lane]),
                          reinterpret_cast<const float*>(tiny + s * d + t));
         }
         qs_cp_commit();
     };
-    double acc = first ? 0.0 : carry[t];
+    double acc = first || t >= d ? 0.0 : carry[t];
+    size_t pos = t < d ? 0 : nsub;  // blocks before it are in acc
     constexpr int kPer = kQsubRows / 32;
     float ahead[kPer];  // rows of block ahead_s, loaded before they are needed
     size_t ahead_s = ~(size_t)0;
-    int chain = 0;
+    int rough = 0;  // groups of the latest replayed blocks that needed most of their adds
+    bool leave = false;
     auto rows_of = [&](size_t s, float (&v)[kPer]) {
 #pragma unroll
         for (int u = 0; u < kPer; u++) {
@@ -308,70 +345,129 @@ __global__ void __launch_bounds__(32 * kQscanWarps) k_quant_colscan(const float*
         } else {
             rows_of(s, v);
         }
-        if (chain > 0 || !sub) {
+        if (!sub) {
             ahead_s = s + 1;
             rows_of(ahead_s, ahead);
         }
-        int rough = 0;
 #pragma unroll
-        for (int u = 0; u < kPer; u += 2) acc = quant_replay64(acc, v[u], v[u + 1], lane, chain > 0, chain_s[warp], rough);
-        chain = rough >= 2 ? kQscanChain : max(chain - 1, 0);
+        for (int u = 0; u < kPer; u += 2) acc = quant_replay64(acc, v[u], v[u + 1], lane, chain_s[warp], rough);
+        leave = rough >= 2;
+        pos = s + 1;
     };
-    if (!sub) {
-        for (size_t s = 0; s < nsub; s++) replay(s);
-    } else {
-        for (int b = 0; b < kQscanDepth - 1; b++) issue(b);
-    }
-    for (size_t b = 0; sub && b < nb; b++) {
-        issue(b + kQscanDepth - 1);
-        qs_cp_wait<kQscanDepth - 1>();
-        QuantSub e{0.0, 0.0f, 0.0f};
-        uint32_t tn = 0xffffffffu;
-        if (b * 32 + lane < nsub) {
-            e = ring_s[warp][b % kQscanDepth][lane];
-            tn = ring_t[warp][b % kQscanDepth][lane];
+    // The blocks from pos on, until the end or until the warp leaves some to all of them.
+    auto scan = [&]() {
+        leave = false;
+        rough = 0;
+        if (!sub) {
+            while (pos < nsub && !leave) replay(pos);
+            return;
         }
-        const int qx = quant_tiny_lsb(tn);
-        const int qmin = __reduce_min_sync(0xffffffffu, qx);
-        if (qmin == 900) continue;  // nothing but zeros
-        const float mag = fmaxf(fabsf(e.lo), fabsf(e.hi));
-        const float magmax = __uint_as_float(__reduce_max_sync(0xffffffffu, __float_as_uint(mag)));
-        // Sums of any of these blocks are exact; otherwise one block at a time.
-        const bool wide = 32.0 * (double)magmax < quant_pow2(53 + qmin);
-        const bool fin = isfinite(e.sum);
-        for (int s0 = 0; s0 < 32;) {
-            if (chain > 0) {
-                if (b * 32 + s0 < nsub) replay(b * 32 + s0);
-                s0++;
+        const size_t b0 = pos / 32;
+        for (size_t b = b0; b < b0 + kQscanDepth - 1; b++) issue(b);
+        for (size_t b = b0; b < nb && !leave; b++) {
+            issue(b + kQscanDepth - 1);
+            qs_cp_wait<kQscanDepth - 1>();
+            QuantSub e{0.0, 0.0f, 0.0f};
+            uint32_t tn = 0xffffffffu;
+            if (b * 32 + lane < nsub) {
+                e = sm.ring.sub[warp][b % kQscanDepth][lane];
+                tn = sm.ring.tiny[warp][b % kQscanDepth][lane];
+            }
+            const size_t end = min(nsub, b * 32 + 32);
+            const int qx = quant_tiny_lsb(tn);
+            const int qmin = __reduce_min_sync(0xffffffffu, qx);
+            if (qmin == 900) {  // nothing but zeros
+                pos = end;
                 continue;
             }
-            const int lim = wide ? 32 : s0 + 1;
-            double before = 0.0;  // of the blocks s0 .. lane - 1
-            if (wide) {
-                before = __shfl_up_sync(0xffffffffu, quant_scan32(lane >= s0 ? e.sum : 0.0, lane), 1);
-                if (lane == 0) before = 0.0;
+            const float mag = fmaxf(fabsf(e.lo), fabsf(e.hi));
+            const float magmax = __uint_as_float(__reduce_max_sync(0xffffffffu, __float_as_uint(mag)));
+            // Sums of any of these blocks are exact; otherwise one block at a time.
+            const bool wide = 32.0 * (double)magmax < quant_pow2(53 + qmin);
+            const bool fin = isfinite(e.sum);
+            while (pos < end && !leave) {
+                const int s0 = (int)(pos - b * 32), lim = wide ? 32 : s0 + 1;
+                double before = 0.0;  // of the blocks s0 .. lane - 1
+                if (wide) {
+                    before = __shfl_up_sync(0xffffffffu, quant_scan32(lane >= s0 ? e.sum : 0.0, lane), 1);
+                    if (lane == 0) before = 0.0;
+                }
+                const double p = __dadd_rn(acc, before);
+                bool ok = tn == 0xffffffffu || isnan(p) || (isinf(p) && fin);
+                if (!ok) {
+                    const double top = quant_pow2(53 + min(qx, quant_lsb(p)));
+                    ok = fin && __dsub_ru((double)e.hi, (double)e.lo) <= quant_pow2(53 + qx) &&
+                         __dadd_ru(p, (double)e.hi) <= top && __dadd_rd(p, (double)e.lo) >= -top;
+                }
+                const unsigned bad = __ballot_sync(0xffffffffu, lane >= s0 && lane < lim && !ok);
+                const int f = bad ? __ffs((int)bad) - 1 : lim;  // the blocks before it are taken whole
+                acc = __shfl_sync(0xffffffffu, bad ? p : __dadd_rn(p, e.sum), bad ? f : lim - 1);
+                if (f > s0) rough = 0;
+                pos = min(end, b * 32 + f);
+                if (bad) replay(pos);
             }
-            const double p = __dadd_rn(acc, before);
-            bool ok = tn == 0xffffffffu || isnan(p) || (isinf(p) && fin);
-            if (!ok) {
-                const double top = quant_pow2(53 + min(qx, quant_lsb(p)));
-                ok = fin && __dsub_ru((double)e.hi, (double)e.lo) <= quant_pow2(53 + qx) &&
-                     __dadd_ru(p, (double)e.hi) <= top && __dadd_rd(p, (double)e.lo) >= -top;
-            }
-            const unsigned bad = __ballot_sync(0xffffffffu, lane >= s0 && lane < lim && !ok);
-            if (!bad) {
-                acc = __shfl_sync(0xffffffffu, __dadd_rn(p, e.sum), lim - 1);
-                s0 = lim;
-                continue;
-            }
-            const int f = __ffs((int)bad) - 1;
-            acc = __shfl_sync(0xffffffffu, p, f);
-            replay(b * 32 + f);
-            s0 = f + 1;
         }
+        qs_cp_wait<0>();
+    };
+    size_t joint = kQscanJoint, joint_end = 0;
+    for (;;) {
+        if (pos < nsub) scan();
+        if (lane == 0) {
+            pos_s[warp] = pos;
+            acc_s[warp] = acc;
+        }
+        __syncthreads();  // the ring is free as well
+        size_t s = nsub;
+        for (int w = 0; w < kQscanWarps; w++) s = min(s, pos_s[w]);
+        if (s == nsub) break;  // the same for all
+        joint = joint_end && s <= joint_end + joint ? min(2 * joint, (size_t)kQscanJointMost) : kQscanJoint;
+        const size_t end = min(nsub, s + joint);
+        joint_end = end;
+        // Warp 0 adds, lane l dimension l % 8 (a warp for each would take the FP64 pipe's
+        // time for 32 equal results); the others bring the next block.
+        constexpr int kLoaders = 32 * (kQscanWarps - 1), kValues = kQsubRows * kQscanWarps;
+        auto bring = [&](size_t blk, int buf) {
+            float v[(kValues + kLoaders - 1) / kLoaders];
+            const int e0 = (int)threadIdx.x - 32;
+#pragma unroll
+            for (int i = 0; e0 + i * kLoaders < kValues && i < (kValues + kLoaders - 1) / kLoaders; i++) {
+                const int e = e0 + i * kLoaders;
+                const size_t r = blk * kQsubRows + e / kQscanWarps, c = (size_t)blockIdx.x * kQscanWarps + e % kQscanWarps;
+                v[i] = r < n && c < d ? __ldg(x + r * d + c) : 0.0f;
+            }
+#pragma unroll
+            for (int i = 0; e0 + i * kLoaders < kValues && i < (kValues + kLoaders - 1) / kLoaders; i++) {
+                const int e = e0 + i * kLoaders;
+                sm.joint[buf][e % kQscanWarps][e / kQscanWarps] = (double)v[i];
+            }
+        };
+        const int mine = lane % kQscanWarps;
+        acc = acc_s[mine];
+        pos = pos_s[mine];
+        if (warp > 0) bring(s, 0);
+        __syncthreads();
+        for (int buf = 0; s < end; s++, buf ^= 1) {
+            if (warp == 0) {
+                const double sum = quant_chain256(acc, sm.joint[buf][mine]);
+                if (pos == s) {  // (a dimension further on joins in when the blocks get there)
+                    acc = sum;
+                    pos = s + 1;
+                }
+            } else if (s + 1 < end) {
+                bring(s + 1, buf ^ 1);
+            }
+            __syncthreads();
+        }
+        if (threadIdx.x < kQscanWarps) {
+            acc_s[threadIdx.x] = acc;
+            pos_s[threadIdx.x] = pos;
+        }
+        __syncthreads();
+        acc = acc_s[warp];
+        pos = pos_s[warp];
+        __syncwarp();
     }
-    qs_cp_wait<0>();
-    if (lane == 0) {
+    if (lane == 0 && t < d) {
         if (last) shift[t] = __double2float_rn(__ddiv_rn(acc, (double)n_all));
         else carry[t] = acc;
     }

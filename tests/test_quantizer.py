@@ -233,3 +233,22 @@ def test_row_order_sums_part_beyond_the_blocks_range(emb, orc, qa, d, part):
     q = emb.Int8Quantizer.fit(x, d, emb.Calibration.faiss(), assigner=qa)
     shift, _ = orc.quantizer_fit(x)
     assert np.array_equal(q.shift.view(np.uint32), shift.view(np.uint32))
+
+
+@pytest.mark.parametrize("n,d", [(256 * 34, 8), (90_003, 11), (150_000, 36)])
+def test_row_order_sums_rough_dimensions_beside_smooth_ones(emb, orc, qa, n, d):
+    # Neighbouring dimensions whose adds round from the start, from some row on, in spells,
+    # in a single spell or never: each takes its own way through the blocks, alone and
+    # together with the others.
+    rng = np.random.default_rng(n)
+    x = rng.standard_normal((n, d))
+    wide = np.exp2(rng.integers(-40, 20, (n, d)).astype(np.float64))
+    row = np.arange(n)[:, None]
+    kind = np.arange(d)[None, :] % 6
+    rough = ((kind == 0) | ((kind == 1) & (row > n // 3)) | ((kind == 2) & (row // 9000 % 2 == 0))
+             | ((kind == 3) & (row > 20_000) & (row < 24_000)) | ((kind == 4) & (row < n // 2)))
+    x = np.where(rough, x * wide, x).astype(np.float32)
+    x[:, kind[0] == 5] = np.round(x[:, kind[0] == 5] * 16) / 16
+    q = emb.Int8Quantizer.fit(x, d, emb.Calibration.faiss(), assigner=qa)
+    shift, scale = orc.quantizer_fit(x)
+    assert np.array_equal(q.shift.view(np.uint32), shift.view(np.uint32)) and q.scale == np.float32(scale)
