@@ -619,7 +619,9 @@ __global__ void __launch_bounds__(kPairThreads, 2) k_rep_pairs(const float* __re
 // of norm_j - 2 dot (bound_coefficients), norm_j within (d / 16 + 20) u |c_j|^2 of
 // |c_j|^2, and s(j) within (d / 16 + 36) u S(j), S(j) <= 4 cmax^2 (u = 2^-24). For
 // d <= 256 the last two are below 2^-16 cmax^2 together: E = E1 + 2^-15 cmax^2 bounds
-// |a(j) + |c_i|^2 - s(j)|.
+// |a(j) + |c_i|^2 - s(j)|. Those are relative errors; below f32's normal range an operation
+// is off by up to 2^-126 whatever its result, and kPairFloor, added to E, covers the
+// 3 d + 2 d of them (centroids of 2^-60 and less end up in the exact pass).
 //  * nearest: with v the second smallest a of the row (its own column is one of the two
 //    smallest or the smallest is a partner nearer than it), the nearest partner has
 //    a <= v + 2 E.
@@ -636,10 +638,11 @@ __global__ void k_pair_mask(const float* __restrict__ norms, const uint32_t* __r
     if (j < kp) masked[j] = j < k && start[j + 1] > start[j] ? norms[j] : kPadNorm;
 }
 
+constexpr float kPairFloor = 0x1p-115f;
 EMB_DEV float pair_bound(float norm, const Bounds& b, float ka, float kb) {
     const float xn = __fmul_ru(__fsqrt_ru(fmaxf(norm, 0.0f)), 1.00001f);
     const float e = __fadd_ru(__fmul_ru(__fmul_ru(ka, xn), b.cmax), __fmul_ru(kb, b.nmax));
-    return __fadd_ru(e, __fmul_ru(0x1p-15f, __fmul_ru(b.cmax, b.cmax)));
+    return __fadd_ru(__fadd_ru(e, __fmul_ru(0x1p-15f, __fmul_ru(b.cmax, b.cmax))), kPairFloor);
 }
 
 // Collection thresholds (NaN: none) from the rows' two smallest scores.

@@ -195,3 +195,15 @@ def test_report_pair_search_matches_oracle(emb, orc, case, k, d):
         live = np.unique(labels)[:3]
         labels = live[labels % 3].astype(np.uint32)
     _assert_same(emb.report(labels, sq, c, d, cfg), _oracle_report(emb, orc, labels, sq, c, cfg))
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("e", [-60, -63, -66, -67, -68, -69, -70, -71, -72, -73, -75])
+def test_report_pair_search_tiny_centroids(emb, orc, e):
+    # Squares and products at the bottom of the f32 range, where rounding errors are
+    # absolute: the pairs' values and the families are still the reference's.
+    k, d = 2100, 64
+    labels, sq, c = _synthetic(6 * k, k, d, seed=k + d, empty=0.1)
+    c = (c * np.float32(2.0 ** e)).astype(np.float32)
+    cfg = emb.ReportConfig(family_pass=2)
+    _assert_same(emb.report(labels, sq, c, d, cfg), _oracle_report(emb, orc, labels, sq, c, cfg))
