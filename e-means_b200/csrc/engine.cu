@@ -1275,7 +1275,7 @@ int emb200_name(emb200_handle* h, char* buf, size_t len) {
     const char* prec = h->opts.precision == EMB200_PREC_FP32   ? "FP32 SIMT"
                        : h->opts.precision == EMB200_PREC_BF16 ? "BF16x3 tcgen05"
                        : h->opts.precision == EMB200_PREC_FP8  ? "FP8 e4m3 tcgen05"
-                                                               : "BF16 tcgen05";
+                                                               : "FP16 tcgen05 (integer rows: BF16)";
     const char* match = h->opts.match_kernel == 0 ? "AVX-512" : h->opts.match_kernel == 1 ? "AVX2" : "portable";
     char ib[64] = "";
     if (h->opts.centroid_bits == 8) snprintf(ib, sizeof ib, ", int8 centroids for i8 rows");

@@ -658,3 +658,8 @@ def test_single_term_zero_centroids_with_bias(orc, assigners, scale, m, k):
     lab, dist = a.assign(x)
     rl, rd = orc.cpu_assign(x, c, bias=bias, emulate=not orc.has_kernel("avx512"))
     assert np.array_equal(lab, rl) and same_f32(dist, rd)
+
+
+@pytest.mark.parametrize("precision,search", [("fp32", "FP32"), ("bf16", "BF16x3"), ("bf16x1", "FP16"), ("fp8", "FP8")])
+def test_name_says_what_the_search_multiplies(assigners, precision, search):
+    assert search in assigners(precision).name()
