@@ -47,8 +47,9 @@ constexpr size_t kMaxSearchRows = (size_t)1 << 26;  // rows per search pass (32-
 
 using namespace emb;
 
-static_assert(kPlanTcM == kTcBM && kPlanTcN == kTcBN && kPlanSimtLargeM == SimtLarge::BM && kPlanSimtLargeN == SimtLarge::BN &&
-                  kPlanSimtSmallM == SimtSmall::BM && kPlanSimtSmallN == SimtSmall::BN,
+static_assert(kPlanTcM == kTcBM && kPlanTcN == kTcBN && kPlanSimtLargeM == SimtLarge::BM &&
+                  kPlanSimtLargeN == SimtLarge::BN && kPlanSimtSmallM == SimtSmall::BM &&
+                  kPlanSimtSmallN == SimtSmall::BN,
               "search_plan.hpp plans the kernels' tiles");
 
 namespace {
@@ -461,7 +462,8 @@ int prepare_centroids(emb200_handle* h) {
         rc = encode_bf16_map(h, &h->map_lo, lo, h->k, h->kpad);
         if (rc) return rc;
         if (h->opts.precision == EMB200_PREC_BF16X1 || h->opts.precision == EMB200_PREC_FP8) {
-            // (FP8 takes this search where its own operands do not fit.) Allocated here, outside any captured epoch; filled before the first search.
+            // (FP8 takes this search where its own operands do not fit.) Allocated here, outside
+            // any captured epoch; filled before the first search.
             if (h->nrm16.ensure(kp * 16) || h->c_f16.ensure((size_t)k * h->kpad))
                 return fail(h, EMB200_ENOMEM, "FP16 centroid allocation failed");
             rc = encode_bf16_map(h, &h->map_f16, h->c_f16.p, h->k, h->kpad);

@@ -29,10 +29,9 @@ struct Bounds {
 // significant bits where BF16 has eight, at the same MMA rate: the operands' rounding,
 // nearly all of the certification bound, is eight times smaller, so rows that need the
 // three-term refine pass are rare (1M x 128 embeddings, k = 16384: the refine pass
-// 675 -> 106 us; k = 65536, heavy-tailed: 4.4 -> 0.7 ms). FP16's
-// narrow range costs values far below the largest one some of those bits, which only
-// enters through the residuals |x - x^| and |c - c^| that the bound is made of;
-// anything out of range (a row hundreds of times the centroids) has an infinite
+// 675 -> 106 us; k = 65536, heavy-tailed: 4.4 -> 0.7 ms). FP16's narrow range costs values
+// far below the largest one some of those bits, which only enters through the residuals
+// |x - x^| and |c - c^| that the bound is made of; anything out of range (a row hundreds of times the centroids) has an infinite
 // residual and is refined. (Centroids that are all zero leave the scale to the biases.)
 EMB_DEV float f16_scale(const Bounds& b) {
     if (!isfinite(b.cmax) || !isfinite(b.nmax)) return 1.0f;
@@ -485,9 +484,10 @@ __global__ void k_certify16(const T* __restrict__ x, const uint32_t* __restrict_
 // d % 4 == 0: thread q keeps AVX-512 lanes 4q .. 4q+3 and loads them as float4; of a
 // last partial chunk the threads beyond d add products of zeros, as masked lanes do.
 // Bound by the latency of a row's dependent loads, hence the fewer, wider ones: 20,011
-// rows of d = 100: 7.6 us, against 15.6 us for k_certify16. The lane sums combine in the reference's tree order (lane l with l^8, l^4,
-// l^2, l^1: threads q^2 and q^1, then in registers), and |x|^2 adds the 16 lane
-// partials in lane order, so every value equals k_certify16's.
+// rows of d = 100: 7.6 us, against 15.6 us for k_certify16. The lane sums combine in the
+// reference's tree order (lane l with l^8, l^4, l^2, l^1: threads q^2 and q^1, then in
+// registers), and |x|^2 adds the 16 lane partials in lane order, so every value equals
+// k_certify16's.
 __global__ void k_certify16v(const float* __restrict__ x, const uint32_t* __restrict__ gather, int m, int d,
                              const float* __restrict__ c, const float* __restrict__ norms, int k,
                              const float* __restrict__ part_s, const uint32_t* __restrict__ part_i, int nsplit,

@@ -432,7 +432,8 @@ __global__ void __launch_bounds__(32 * kQscanWarps) k_quant_colscan(const float*
 #pragma unroll
             for (int i = 0; e0 + i * kLoaders < kValues && i < (kValues + kLoaders - 1) / kLoaders; i++) {
                 const int e = e0 + i * kLoaders;
-                const size_t r = blk * kQsubRows + e / kQscanWarps, c = (size_t)blockIdx.x * kQscanWarps + e % kQscanWarps;
+                const size_t r = blk * kQsubRows + e / kQscanWarps;
+                const size_t c = (size_t)blockIdx.x * kQscanWarps + e % kQscanWarps;
                 v[i] = r < n && c < d ? __ldg(x + r * d + c) : 0.0f;
             }
 #pragma unroll
