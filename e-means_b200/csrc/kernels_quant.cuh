@@ -277,20 +277,23 @@ __device__ __forceinline__ double quant_chain256(double acc, const double* rows)
 // replayed (short samples: n <= kQscanShort, where the entries' launch costs more
 // than they save).
 // Where the adds round often (magnitudes spread over many binades), looking first is
-// slower than the chain: a warp that has met two groups of 64 rows that needed most of
-// their adds, in one block after another, leaves the next blocks to its whole CTA:
+// slower than the chain: a warp that has met kRoughFirst groups of 64 rows that needed
+// most of their adds, in one block after another, leaves the next blocks to its whole CTA:
 // kQscanJoint of them, and twice as many, up to kQscanJointMost, each time that this
-// happens again within as many as the last time. There one warp adds, a lane a
-// dimension, and the others bring the rows: each row's 32 bytes are read once, where a
-// warp alone touches 32 lines for 32 values of its column, which bounds it (9.6 ns a row,
-// 17 with two CTAs on an SM), and no FP64 cycles go into 32 equal results. Whole fits,
-// each dimension's warp replaying by itself / so / every dimension as one chain from the
-// start: magnitudes over 60 binades, 200,000 x 64 1985 / 1251 / 1780 us, 50,000 x 2048
-// 1094 / 624 / 574; squares of normals 200,000 x 64 1871 / 1347 / 1778, 50,000 x 2048 963
-// / 728 / 577; normals, 200,000 x 64, 126 / 126 / 1780. First joint runs of 8 and 16
-// blocks: 1264 and 1260, 842 and 770 us where 32 takes 1251 and 728.
+// happens again (then at the first such group) within as many as the last time. There one
+// warp adds, a lane a dimension, and the others bring the rows: each row's 32 bytes are
+// read once, where a warp alone touches 32 lines for 32 values of its column, which bounds
+// it (9.6 ns a row, 17 with two CTAs on an SM), and no FP64 cycles go into 32 equal
+// results. Whole fits, each dimension's warp replaying by itself / so / every dimension as
+// one chain from the start: magnitudes over 60 binades, 200,000 x 64 1986 / 1250 / 1784 us,
+// 50,000 x 2048 1097 / 618 / 575; squares of normals 200,000 x 64 1873 / 1359 / 1781,
+// 50,000 x 2048 967 / 790 / 576, 50,000 x 64 508 / 499 / 497; normals, 200,000 x 64, 126 /
+// 129 / 1781; unit-norm embeddings, 500,000 x 512, six samples, 472 .. 520 / 474 .. 492 /
+// 4515 .. 4520. Two groups to begin with: such samples up to 548; two of them afterwards as
+// well, or joint runs of 16 blocks at first: the squares, 50,000 x 64, 1.05 and 1.33 times
+// as long.
 constexpr size_t kQscanShort = 2048;
-constexpr int kQscanJoint = 32, kQscanJointMost = 256;
+constexpr int kRoughFirst = 3, kQscanJoint = 32, kQscanJointMost = 256;
 constexpr int kQscanPitch = kQsubRows + 4;  // of a dimension's converted rows: no bank conflicts across dimensions
 struct QuantRing {
     QuantSub sub[kQscanWarps][kQscanDepth][32];
@@ -329,6 +332,7 @@ __global__ void __launch_bounds__(32 * kQscanWarps) k_quant_colscan(const float*
     float ahead[kPer];  // rows of block ahead_s, loaded before they are needed
     size_t ahead_s = ~(size_t)0;
     int rough = 0;  // groups of the latest replayed blocks that needed most of their adds
+    size_t joint = kQscanJoint, joint_end = 0;  // blocks of the CTA's last joint run, and its end
     bool leave = false;
     auto rows_of = [&](size_t s, float (&v)[kPer]) {
 #pragma unroll
@@ -351,7 +355,7 @@ __global__ void __launch_bounds__(32 * kQscanWarps) k_quant_colscan(const float*
         }
 #pragma unroll
         for (int u = 0; u < kPer; u += 2) acc = quant_replay64(acc, v[u], v[u + 1], lane, chain_s[warp], rough);
-        leave = rough >= 2;
+        leave = rough >= (joint_end && s <= joint_end + joint ? 1 : kRoughFirst);
         pos = s + 1;
     };
     // The blocks from pos on, until the end or until the warp leaves some to all of them.
@@ -409,7 +413,6 @@ __global__ void __launch_bounds__(32 * kQscanWarps) k_quant_colscan(const float*
         }
         qs_cp_wait<0>();
     };
-    size_t joint = kQscanJoint, joint_end = 0;
     for (;;) {
         if (pos < nsub) scan();
         if (lane == 0) {
