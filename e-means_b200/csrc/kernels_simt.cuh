@@ -15,7 +15,7 @@ namespace emb {
 // FMAs, half the issue slots) over neighbouring columns and 8 x 16 values per thread
 // (six loads per 128 FMAs); the running top-2 of a thread's rows lives in shared
 // memory, touched once per tile. 200,000 x 96 rows, k = 1024: 1488 -> 951 us (26 ->
-// 41 TF/s; FMA pipe 57% busy, the rest mostly shared-load latency that two warps per
+// 41 TF/s; FMA pipe 59% busy, the rest mostly shared-load latency that two warps per
 // scheduler do not cover). Storing each row value twice, so that its pair is one
 // load, or 8 x 8 values with two CTAs per SM measured 32 TF/s.
 // Few rows (100 x 96, k = 1024: 30 -> 13 us) take 64 x 64 tiles, 4 x 4 values per
