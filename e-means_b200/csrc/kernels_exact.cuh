@@ -31,8 +31,9 @@ struct Bounds {
 // three-term refine pass are rare (1M x 128 embeddings, k = 16384: the refine pass
 // 675 -> 106 us; k = 65536, heavy-tailed: 4.4 -> 0.7 ms). FP16's narrow range costs values
 // far below the largest one some of those bits, which only enters through the residuals
-// |x - x^| and |c - c^| that the bound is made of; anything out of range (a row hundreds of times the centroids) has an infinite
-// residual and is refined. (Centroids that are all zero leave the scale to the biases.)
+// |x - x^| and |c - c^| that the bound is made of; anything out of range (a row hundreds
+// of times the centroids) has an infinite residual and is refined. (Centroids that are
+// all zero leave the scale to the biases.)
 EMB_DEV float f16_scale(const Bounds& b) {
     if (!isfinite(b.cmax) || !isfinite(b.nmax)) return 1.0f;
     int e = b.cmax > 0.0f ? 6 - ((int)(__float_as_uint(b.cmax) >> 23) - 127) : 60;
